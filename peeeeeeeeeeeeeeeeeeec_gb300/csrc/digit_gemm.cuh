@@ -1,0 +1,38 @@
+// C -= A B in FP64 accuracy on the tcgen05 tensor cores, real and complex:
+// the trailing updates of the FP64 LU factorisations and of the transient
+// system's inverse (digit_gemm.cu has the method and its error).
+#pragma once
+
+#include <stddef.h>
+
+namespace peec {
+
+// K of one update at most: every sum of digit products stays an integer
+// below 2^24 (see digit_gemm.cu).
+static const int kDigitMaxKReal = 256;
+static const int kDigitMaxKCplx = 192;
+
+// Scratch of the updates of one factorisation: the digits of A (m rows) and
+// B (n columns) and the exponents of their rows, columns and inner scaling.
+struct DigitScratch {
+    void *a = nullptr, *b = nullptr;
+    int *ea = nullptr, *eb = nullptr, *ef = nullptr;
+    int m = 0, n = 0, k = 0;
+    bool cplx = false;
+    DigitScratch() = default;
+    bool alloc(bool cplx_, int m_, int n_, int k_);
+    ~DigitScratch();
+    DigitScratch(const DigitScratch &) = delete;
+    DigitScratch &operator=(const DigitScratch &) = delete;
+};
+size_t digit_scratch_bytes(bool cplx, size_t m, size_t n, size_t k);
+
+// C (m x n, row-major, leading dimension ldc) -= A (m x k, lda) B (k x n,
+// ldb); complex entries are interleaved {re, im} and the leading dimensions
+// count entries.  C must not overlap A or B.  m, n, k within the scratch's
+// sizes.  *code (device): nothing is done when it is not 0; it is set to 6
+// when a bounded wait inside the kernel runs out.
+bool digit_gemm_sub(bool cplx, const void *A, size_t lda, const void *B, size_t ldb, void *C, size_t ldc, int m, int n,
+                    int k, DigitScratch &s, int *code);
+
+}  // namespace peec

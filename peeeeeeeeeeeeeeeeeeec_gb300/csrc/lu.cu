@@ -17,8 +17,9 @@
 //   k_laswp     replays the panel's row swaps on the columns left and right
 //               of the panel;
 //   k_trsm      U12 = L11^-1 A12 (one thread per column, L11 in shared memory);
-//   k_gemm_*    A22 -= L21 U12, register-tiled FP64 (complex: 4 real FMAs
-//               per complex multiply-add).
+//   A22 -= L21 U12: k_gemm_rect, register-tiled FP64 (complex: 4 real FMAs per
+//               complex multiply-add), or from about a thousand unknowns on
+//               the digit GEMM on the tensor cores (digit_gemm.cu).
 // A device status word stops every later kernel after a singular pivot, so
 // the host synchronises once per factorisation.
 #include <math.h>
@@ -29,6 +30,7 @@
 #include <atomic>
 #include <chrono>
 #include <complex>
+#include <functional>
 #include <list>
 #include <mutex>
 #include <type_traits>
@@ -42,6 +44,7 @@
 #include <cuda_bf16.h>
 
 #include "common.cuh"
+#include "digit_gemm.cuh"
 
 namespace peec {
 
@@ -113,7 +116,7 @@ __device__ __forceinline__ cplx addv(cplx a, cplx b) { return cplx{a.re + b.re, 
 __device__ __forceinline__ cplxf addv(cplxf a, cplxf b) { return cplxf{a.re + b.re, a.im + b.im}; }
 
 struct Status {
-    int code;    // 0 ok, 2 singular / invalid pivot
+    int code;    // 0 ok, 2 singular / invalid pivot, 7 near tie of two pivot candidates (checked runs)
     int column;  // failing column
     double value;
 };
@@ -132,10 +135,27 @@ __global__ void k_max_mag(const T *a, size_t count, unsigned long long *out) {
     if ((threadIdx.x & 31) == 0) atomicMax(out, (unsigned long long)__double_as_longlong(best));
 }
 
+// Near ties.  A checked factorisation (tie > 0) stops with status 7 when another
+// candidate's magnitude is within `tie` ulps of the pivot's: there the pivot
+// would depend on how its column's earlier updates were rounded.
+static const long long kTieUlps = 1LL << 18;  // 2^-34 relative
+__device__ __forceinline__ bool near_tie(double m, double best, long long tie) {
+    return __double_as_longlong(m) >= __double_as_longlong(best) - tie;  // both finite, best > 0; m = -1: none
+}
+// the same of an entry whose magnitude is not at hand, behind a cheap bound
+__device__ __forceinline__ bool near_tie_of(double v, double best, long long tie) {
+    return near_tie(fabs(v), best, tie);
+}
+__device__ __forceinline__ bool near_tie_of(cplx v, double best, long long tie) {
+    const int b = (int)(__double_as_longlong(best) >> 52) - 1;
+    const int e = max((int)(__double_as_longlong(v.re) >> 52 & 0x7ff), (int)(__double_as_longlong(v.im) >> 52 & 0x7ff));
+    return e >= b && near_tie(mag(v), best, tie);
+}
+
 // ---- panel ----------------------------------------------------------
 template <class T>
 __global__ void __launch_bounds__(1024) k_panel(T *a, int n, int k0, int kb, double limit, long long *piv,
-                                                Status *st) {
+                                                Status *st, long long tie) {
     __shared__ double s_val[32];
     __shared__ int s_idx[32];
     __shared__ int s_pivot;
@@ -196,11 +216,13 @@ __global__ void __launch_bounds__(1024) k_panel(T *a, int n, int k0, int kb, dou
                     piv[k] = bi;
                 }
                 s_pivot = bi;
+                s_val[0] = best;
             }
         }
         __syncthreads();
         if (s_fail) return;
         const int p = s_pivot;
+        const double pivot_mag = s_val[0];
         if (p != k) {
             for (int j = k0 + tid; j < k0 + kb; j += nthr) {
                 T t = a[(size_t)k * n + j];
@@ -215,6 +237,8 @@ __global__ void __launch_bounds__(1024) k_panel(T *a, int n, int k0, int kb, dou
         const T pivot = s_row[kk];
         for (int i = k + 1 + tid; i < n; i += nthr) {
             T *row = a + (size_t)i * n + k0;
+            if constexpr (!std::is_same<T, cplxf>::value)
+                if (tie > 0 && near_tie_of(row[kk], pivot_mag, tie)) atomicCAS(&st->code, 0, 7);
             T m = divide(row[kk], pivot);
             row[kk] = m;
             for (int j = kk + 1; j < kb; ++j) row[j] = msub(row[j], m, s_row[j]);
@@ -307,7 +331,7 @@ __device__ __forceinline__ bool grid_barrier(PanelSlots *ps, unsigned int nblock
 template <class T>
 __global__ void __launch_bounds__(256) k_panel_coop(T *a, int n, int k0, int kb, int rows_per_cta, double limit,
                                                     long long *piv, Status *st, PanelSlots *ps, double *cand_val,
-                                                    int *cand_idx, T *cand_row, T *krow) {
+                                                    int *cand_idx, T *cand_row, T *krow, long long tie) {
     extern __shared__ unsigned char smem_raw[];
     T *tile = reinterpret_cast<T *>(smem_raw);  // [rows_per_cta][kPS] (padded rows: no bank conflicts)
     using M = typename MagType<T>::type;  // FP32 magnitudes for the FP32 factorisation
@@ -435,10 +459,12 @@ __global__ void __launch_bounds__(256) k_panel_coop(T *a, int n, int k0, int kb,
             }
             s_p = gi;
             s_pc = gc;
+            s_val[0] = gb;
         }
         __syncthreads();
         if (s_fail) return;
         const int p = s_p, pc = s_pc;
+        const double pivot_mag = (double)s_val[0];
         // the new row k is the published row p (full panel width: columns
         // < kk hold earlier multipliers and move with the row)
         const T *prow_g = cand_row + ((size_t)par * G + pc) * NB;
@@ -456,6 +482,8 @@ __global__ void __launch_bounds__(256) k_panel_coop(T *a, int n, int k0, int kb,
         const T pivot = s_prow[kk];
         for (int i = max(r0, k + 1) + tid; i < r1; i += blockDim.x) {
             T *row = tile + (i - r0) * kPS;
+            if constexpr (!std::is_same<T, cplxf>::value)
+                if (tie > 0 && near_tie_of(row[kk], pivot_mag, tie)) atomicCAS(&st->code, 0, 7);
             T m = divide(row[kk], pivot);
             row[kk] = m;
             for (int j = kk + 1; j < kb; ++j) row[j] = msub(row[j], m, s_prow[j]);
@@ -749,7 +777,7 @@ __global__ void __launch_bounds__(kLeanThreads) k_panel_lean64(T *a, int n, int 
                                                                long long *piv, Status *st, PanelSlots *ps,
                                                                unsigned long long *flag, int flag_stride,
                                                                int *cand_idx, double *cand_val, T *cand_row,
-                                                               T *krow) {
+                                                               T *krow, long long tie) {
     __shared__ T tile[kLeanThreads][kPS];
     __shared__ T s_prow[2][NB];
     __shared__ double s_wv[2], s_gb;
@@ -906,6 +934,9 @@ __global__ void __launch_bounds__(kLeanThreads) k_panel_lean64(T *a, int n, int 
         }
         __syncthreads();
         const int p = s_p;
+        // (mv still is this row's candidate; every CTA has passed the status
+        // check at the top: the flags of this column were all published)
+        if (tie > 0 && mine && i >= k && i != p && near_tie(mv, gb, tie)) atomicCAS(&st->code, 0, 7);
         if (p != k) {
             if (warp == 0 && k >= r0 && k < r1 && lane < kb) tile[k - r0][lane] = pcur[lane];
             if (warp == 1 && gc == c && lane < kb) tile[p - r0][lane] = kval;
@@ -1319,168 +1350,57 @@ __global__ void __launch_bounds__(256) k_trsm(T *a, int n, int k0, int kb, int c
         if (i < kb) a[(size_t)(k0 + i) * n + j] = x[i];
 }
 
-// ---- A22 -= L21 U12 --------------------------------------------------
-// Real: 64x64 C tile per 256-thread CTA, 4x4 per thread.
-__global__ void __launch_bounds__(256) k_gemm_real(double *a, int n, int k0, int kb, const Status *st) {
-    __shared__ double As[NB][64 + 1];
-    __shared__ double Bs[NB][64];
+// ---- C -= L U on a rectangle, FP64 pipe -------------------------------
+// rows r0 .. r1-1, columns c0 .. c1-1, the kb columns k0 .. of L and rows k0 ..
+// of U.  RB x CB tile per 256-thread CTA, (RB / 16) x (CB / 16) entries per
+// thread.  The updates inside a 64-column block (32 columns or 32 rows wide);
+// the trailing update is the digit GEMM's.
+template <class T, int RB, int CB>
+__global__ void __launch_bounds__(256) k_gemm_rect(T *a, int n, int k0, int kb, int r_first, int r1, int c_first,
+                                                   int c1, const Status *st) {
+    __shared__ T As[NB][RB + 1];
+    __shared__ T Bs[NB][CB];
     if (st->code != 0) return;
-    const int r0 = k0 + kb + blockIdx.y * 64, c0 = k0 + kb + blockIdx.x * 64;
+    const int r0 = r_first + blockIdx.y * RB, c0 = c_first + blockIdx.x * CB;
     const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-    for (int t = threadIdx.x; t < 64 * NB; t += 256) {
-        int r = t / NB, m = t % NB;  // A tile: rows r0.., cols k0..
-        As[m][r] = (r0 + r < n && m < kb) ? a[(size_t)(r0 + r) * n + k0 + m] : 0.0;
-        int mm = t / 64, c = t % 64;  // B tile: rows k0.., cols c0..
-        Bs[mm][c] = (c0 + c < n && mm < kb) ? a[(size_t)(k0 + mm) * n + c0 + c] : 0.0;
+    constexpr int TR = RB / 16, TC = CB / 16;
+    for (int t = threadIdx.x; t < RB * NB; t += 256) {
+        const int r = t / NB, m = t % NB;
+        As[m][r] = (r0 + r < r1 && m < kb) ? a[(size_t)(r0 + r) * n + k0 + m] : T{};
+    }
+    for (int t = threadIdx.x; t < CB * NB; t += 256) {
+        const int m = t / CB, c = t % CB;
+        Bs[m][c] = (c0 + c < c1 && m < kb) ? a[(size_t)(k0 + m) * n + c0 + c] : T{};
     }
     __syncthreads();
-    double acc[4][4];
+    T acc[TR][TC];
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
+    for (int i = 0; i < TR; ++i)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            int r = r0 + ty + 16 * i, c = c0 + tx + 16 * j;
-            acc[i][j] = (r < n && c < n) ? a[(size_t)r * n + c] : 0.0;
+        for (int j = 0; j < TC; ++j) {
+            const int r = r0 + ty + 16 * i, c = c0 + tx + 16 * j;
+            acc[i][j] = (r < r1 && c < c1) ? a[(size_t)r * n + c] : T{};
         }
-#pragma unroll 8
+#pragma unroll(sizeof(T) == 8 ? 8 : 4)
     for (int m = 0; m < NB; ++m) {
-        double av[4], bv[4];
+        T av[TR], bv[TC];
 #pragma unroll
-        for (int i = 0; i < 4; ++i) av[i] = As[m][ty + 16 * i];
+        for (int i = 0; i < TR; ++i) av[i] = As[m][ty + 16 * i];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) bv[j] = Bs[m][tx + 16 * j];
+        for (int j = 0; j < TC; ++j) bv[j] = Bs[m][tx + 16 * j];
 #pragma unroll
-        for (int i = 0; i < 4; ++i)
+        for (int i = 0; i < TR; ++i)
 #pragma unroll
-            for (int j = 0; j < 4; ++j) acc[i][j] = fma(-av[i], bv[j], acc[i][j]);
+            for (int j = 0; j < TC; ++j) acc[i][j] = msub(acc[i][j], av[i], bv[j]);
     }
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
+    for (int i = 0; i < TR; ++i)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            int r = r0 + ty + 16 * i, c = c0 + tx + 16 * j;
-            if (r < n && c < n) a[(size_t)r * n + c] = acc[i][j];
+        for (int j = 0; j < TC; ++j) {
+            const int r = r0 + ty + 16 * i, c = c0 + tx + 16 * j;
+            if (r < r1 && c < c1) a[(size_t)r * n + c] = acc[i][j];
         }
 }
-
-// Complex: 32x64 C tile per 256-thread CTA, 2x4 per thread.
-__global__ void __launch_bounds__(256) k_gemm_cplx(cplx *a, int n, int k0, int kb, const Status *st) {
-    __shared__ cplx As[NB][32 + 1];
-    __shared__ cplx Bs[NB][64];
-    if (st->code != 0) return;
-    const int r0 = k0 + kb + blockIdx.y * 32, c0 = k0 + kb + blockIdx.x * 64;
-    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-    const cplx z = {0.0, 0.0};
-    for (int t = threadIdx.x; t < 32 * NB; t += 256) {
-        int r = t / NB, m = t % NB;
-        As[m][r] = (r0 + r < n && m < kb) ? a[(size_t)(r0 + r) * n + k0 + m] : z;
-    }
-    for (int t = threadIdx.x; t < 64 * NB; t += 256) {
-        int mm = t / 64, c = t % 64;
-        Bs[mm][c] = (c0 + c < n && mm < kb) ? a[(size_t)(k0 + mm) * n + c0 + c] : z;
-    }
-    __syncthreads();
-    cplx acc[2][4];
-#pragma unroll
-    for (int i = 0; i < 2; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            int r = r0 + ty + 16 * i, c = c0 + tx + 16 * j;
-            acc[i][j] = (r < n && c < n) ? a[(size_t)r * n + c] : z;
-        }
-#pragma unroll 4
-    for (int m = 0; m < NB; ++m) {
-        cplx av[2], bv[4];
-#pragma unroll
-        for (int i = 0; i < 2; ++i) av[i] = As[m][ty + 16 * i];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) bv[j] = Bs[m][tx + 16 * j];
-#pragma unroll
-        for (int i = 0; i < 2; ++i)
-#pragma unroll
-            for (int j = 0; j < 4; ++j) acc[i][j] = msub(acc[i][j], av[i], bv[j]);
-    }
-#pragma unroll
-    for (int i = 0; i < 2; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            int r = r0 + ty + 16 * i, c = c0 + tx + 16 * j;
-            if (r < n && c < n) a[(size_t)r * n + c] = acc[i][j];
-        }
-}
-
-// Complex, 3 real products per complex multiply-add (Gauss / 3M):
-//   T1 = Ar Br, T2 = Ai Bi, T3 = (Ar + Ai)(Br + Bi),
-//   C -= (T1 - T2) + j (T3 - T1 - T2),
-// 25% fewer FP64 operations than the 4-product form; the sums Ar + Ai and
-// Br + Bi are formed once per tile in shared memory.  32x64 C tile per
-// 256-thread CTA, 2x4 per thread.
-__global__ void __launch_bounds__(256) k_gemm_cplx3m(cplx *a, int n, int k0, int kb, const Status *st) {
-    extern __shared__ double sm3[];
-    double *Ar = sm3, *Ai = Ar + NB * 33, *As = Ai + NB * 33;  // [NB][33]
-    double *Br = As + NB * 33, *Bi = Br + NB * 64, *Bs = Bi + NB * 64;  // [NB][64]
-    if (st->code != 0) return;
-    const int r0 = k0 + kb + blockIdx.y * 32, c0 = k0 + kb + blockIdx.x * 64;
-    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-    for (int t = threadIdx.x; t < 32 * NB; t += 256) {
-        int r = t / NB, m = t % NB;
-        cplx v = (r0 + r < n && m < kb) ? a[(size_t)(r0 + r) * n + k0 + m] : cplx{0.0, 0.0};
-        Ar[m * 33 + r] = v.re;
-        Ai[m * 33 + r] = v.im;
-        As[m * 33 + r] = v.re + v.im;
-    }
-    for (int t = threadIdx.x; t < 64 * NB; t += 256) {
-        int mm = t / 64, c = t % 64;
-        cplx v = (c0 + c < n && mm < kb) ? a[(size_t)(k0 + mm) * n + c0 + c] : cplx{0.0, 0.0};
-        Br[mm * 64 + c] = v.re;
-        Bi[mm * 64 + c] = v.im;
-        Bs[mm * 64 + c] = v.re + v.im;
-    }
-    __syncthreads();
-    double t1[2][4], t2[2][4], t3[2][4];
-#pragma unroll
-    for (int i = 0; i < 2; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) t1[i][j] = t2[i][j] = t3[i][j] = 0.0;
-#pragma unroll 4
-    for (int m = 0; m < NB; ++m) {
-        double ar[2], ai[2], as[2], br[4], bi[4], bs[4];
-#pragma unroll
-        for (int i = 0; i < 2; ++i) {
-            ar[i] = Ar[m * 33 + ty + 16 * i];
-            ai[i] = Ai[m * 33 + ty + 16 * i];
-            as[i] = As[m * 33 + ty + 16 * i];
-        }
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            br[j] = Br[m * 64 + tx + 16 * j];
-            bi[j] = Bi[m * 64 + tx + 16 * j];
-            bs[j] = Bs[m * 64 + tx + 16 * j];
-        }
-#pragma unroll
-        for (int i = 0; i < 2; ++i)
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                t1[i][j] = fma(ar[i], br[j], t1[i][j]);
-                t2[i][j] = fma(ai[i], bi[j], t2[i][j]);
-                t3[i][j] = fma(as[i], bs[j], t3[i][j]);
-            }
-    }
-#pragma unroll
-    for (int i = 0; i < 2; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            int r = r0 + ty + 16 * i, c = c0 + tx + 16 * j;
-            if (r < n && c < n) {
-                cplx v = a[(size_t)r * n + c];
-                v.re -= t1[i][j] - t2[i][j];
-                v.im -= (t3[i][j] - t1[i][j]) - t2[i][j];
-                a[(size_t)r * n + c] = v;
-            }
-        }
-}
-
-static const size_t kGemm3mSmem = (size_t)NB * 33 * 3 * 8 + (size_t)NB * 64 * 3 * 8;
 
 // ---- final diagonal check (lu.c:455-476) -----------------------------
 template <class T>
@@ -2391,18 +2311,6 @@ static int lean64_panel_ctas(int m) {
     return g <= cap && g <= 32 * kLeanPoll ? g : 0;
 }
 
-// Complex trailing update form: the direct 4-product form (default; it keeps
-// the reference's backward error, 1.5e-11 on the 8402-unknown box) or 3 real
-// products when PEEC_GB300_CGEMM=3m (17% faster, backward error 3.4e-11).
-static bool complex_gemm_3m() {
-    static int mode = -1;
-    if (mode < 0) {
-        const char *e = getenv("PEEC_GB300_CGEMM");
-        mode = (e && strcmp(e, "3m") == 0) ? 1 : 0;
-    }
-    return mode == 1;
-}
-
 struct PanelScratch {
     PanelSlots *ps = nullptr;
     double *cand_val = nullptr;
@@ -2447,8 +2355,24 @@ struct LuTiming {
 };
 static thread_local LuTiming g_lu_timing;  // per host thread, like the stream
 
+// How a factorisation does its trailing updates.
+enum class LuMode {
+    chain,    // chains of FP64 FMAs in pivot order: the reference's arithmetic up to FMA rounding
+    digits,   // digit GEMMs
+    checked,  // digit GEMMs, stopping with status 7 at a near tie of two pivot candidates
+};
+// Unknowns from which digit GEMMs are the faster form (LU of random matrices on
+// GB300, chains / digits in ms: complex 1000: 19.2 / 20.1, 1200: 24.1 / 24.3, 2102:
+// 58.7 / 43.0, 4000: 212 / 97, 8402: 1436 / 285; real 2102: 21.7 / 19.9, 4000: 65.9 / 48,
+// 8402: 386 / 126).  A checked run may have to be done again by chains (real
+// systems of regular meshes nearly always tie), so real ones start later.
+static const int kDigitsFromCplx = 1300;
+static const int kDigitsFromReal = 2000;
+static const int kCheckedFromReal = 5000;
+static const int kLuWideFrom = 3000;  // unknowns from which wide outer blocks pay (2102 complex: 45 ms with, 43 without)
+
 template <class T>
-static bool factor_device(T *d_a, int n, double limit, long long *d_piv, Status *d_st) {
+static bool factor_device(T *d_a, int n, double limit, long long *d_piv, Status *d_st, LuMode mode) {
     LuTiming &tm = g_lu_timing;
     if (tm.enabled) tm.reset();
     DBuf<unsigned char> scratch;
@@ -2479,9 +2403,15 @@ static bool factor_device(T *d_a, int n, double limit, long long *d_piv, Status 
         sc.cand_row = b + off;
         sc.krow = b + off + 2 * G * NB * sizeof(T);
     }
-    for (int k0 = 0; k0 < n; k0 += NB) {
-        int kb = std::min(NB, n - k0);
-        tm.mark(2);
+    constexpr bool cx = sizeof(T) == sizeof(cplx);
+    auto swaps = [&](int k0, int kb) {
+        PEEC_LAUNCH(k_laswp<T>, (n + kLaswpCols - 1) / kLaswpCols, 256, 2 * NB * kLaswpCols * sizeof(T), d_a, n, k0, kb,
+                    d_piv, d_st);
+    };
+    auto rows_of_u = [&](int k0, int kb, int c0, int c1) {
+        PEEC_LAUNCH(k_trsm<T>, (c1 - c0 + 63) / 64, 64, 0, d_a, n, k0, kb, c0, c1, d_st);
+    };
+    auto panel = [&](int k0, int kb, long long tie) -> bool {
         CoopPlan<T> pl = coop_plan<T>(n - k0);
         const int lean_g = lean64_panel_ctas<T>(n - k0);
         if (lean_g > 0) {
@@ -2490,7 +2420,7 @@ static bool factor_device(T *d_a, int n, double limit, long long *d_piv, Status 
             int *li = lean_idx.p;
             double *lv = lean_val.p;
             T *lr = lean_rows.p, *lk = lean_rows.p + 2 * GL * NB;
-            void *args[] = {&d_a, &n, (void *)&k0, &kb, &limit, &d_piv, &d_st, &sc.ps, &fl, &fls, &li, &lv, &lr, &lk};
+            void *args[] = {&d_a, &n, &k0, &kb, &limit, &d_piv, &d_st, &sc.ps, &fl, &fls, &li, &lv, &lr, &lk, &tie};
             if (!cuda_ok(cudaLaunchCooperativeKernel((const void *)k_panel_lean64<T>, dim3(lean_g), dim3(kLeanThreads),
                                                      args, 0, stream()),
                          "lean FP64 panel launch"))
@@ -2499,40 +2429,94 @@ static bool factor_device(T *d_a, int n, double limit, long long *d_piv, Status 
         } else if (pl.G > 0) {
             int rows = pl.rows;
             T *cr = (T *)sc.cand_row, *kr = (T *)sc.krow;
-            void *args[] = {&d_a, &n, (void *)&k0, &kb, &rows, &limit, &d_piv, &d_st, &sc.ps, &sc.cand_val,
-                            &sc.cand_idx, &cr, &kr};
+            void *args[] = {&d_a,         &n,           &k0, &kb, &rows, &limit, &d_piv, &d_st, &sc.ps,
+                            &sc.cand_val, &sc.cand_idx, &cr, &kr, &tie};
             if (!cuda_ok(cudaLaunchCooperativeKernel((const void *)k_panel_coop<T>, dim3(pl.G), dim3(256), args,
                                                      pl.smem, stream()),
                          "cooperative panel launch"))
                 return false;
             note_launch();
         } else {
-            PEEC_LAUNCH(k_panel<T>, 1, 1024, 0, d_a, n, k0, kb, limit, d_piv, d_st);
+            PEEC_LAUNCH(k_panel<T>, 1, 1024, 0, d_a, n, k0, kb, limit, d_piv, d_st, tie);
         }
-        tm.mark(0);
-        PEEC_LAUNCH(k_laswp<T>, (n + kLaswpCols - 1) / kLaswpCols, 256, 2 * NB * kLaswpCols * sizeof(T), d_a, n, k0, kb,
-                    d_piv, d_st);
-        int rest = n - (k0 + kb);
-        if (rest > 0) {
-            PEEC_LAUNCH(k_trsm<T>, (rest + 255) / 256, 256, 0, d_a, n, k0, kb, k0 + kb, n, d_st);
-        }
-        tm.mark(1);
-        if (tm.enabled) tm.flops_update += (sizeof(T) == sizeof(double) ? 2.0 : 8.0) * (double)rest * rest * kb;
-        if (rest > 0) {
-            if constexpr (sizeof(T) == sizeof(double)) {
-                dim3 g((rest + 63) / 64, (rest + 63) / 64);
-                PEEC_LAUNCH(k_gemm_real, g, 256, 0, (double *)d_a, n, k0, kb, d_st);
-            } else {
-                dim3 g((rest + 63) / 64, (rest + 31) / 32);
-                if (complex_gemm_3m()) {
-                    static const cudaError_t attr = cudaFuncSetAttribute(
-                        k_gemm_cplx3m, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGemm3mSmem);
-                    (void)attr;
-                    PEEC_LAUNCH(k_gemm_cplx3m, g, 256, kGemm3mSmem, (cplx *)d_a, n, k0, kb, d_st);
-                } else {
-                    PEEC_LAUNCH(k_gemm_cplx, g, 256, 0, (cplx *)d_a, n, k0, kb, d_st);
-                }
+        return true;
+    };
+    if (mode == LuMode::chain) {
+        for (int k0 = 0; k0 < n; k0 += NB) {
+            const int kb = std::min(NB, n - k0), r1 = k0 + kb, rest = n - r1;
+            tm.mark(2);
+            if (!panel(k0, kb, 0)) return false;
+            tm.mark(0);
+            swaps(k0, kb);
+            if (rest > 0) rows_of_u(k0, kb, r1, n);
+            tm.mark(1);
+            if (tm.enabled) tm.flops_update += (cx ? 8.0 : 2.0) * (double)rest * rest * kb;
+            if (rest > 0) {
+                constexpr int RB = cx ? 32 : 64;
+                PEEC_LAUNCH((k_gemm_rect<T, RB, 64>), dim3((rest + 63) / 64, (rest + RB - 1) / RB), 256, 0, d_a, n, k0,
+                            kb, r1, n, r1, n, d_st);
             }
+        }
+    } else {
+        // Outer blocks of W columns, inner blocks of two panels.  Everything
+        // wider than a panel is a digit GEMM: per inner block, the block's
+        // columns below its first row get what the outer block's earlier
+        // columns did (before the panels), then its rows to the right (after
+        // them: the panels' swaps bring rows from below that lack it too); per
+        // outer block, the trailing update with K = W.  A digit GEMM's tile
+        // costs an integer epilogue per entry whatever K is (m = n = 4000
+        // complex: 702 us with K = 64, 1350 us with 192), so W is its largest K;
+        // small systems, where launches count, take one inner block.
+        const int W = n < kLuWideFrom ? 2 * NB : cx ? kDigitMaxKCplx : kDigitMaxKReal;
+        DigitScratch digits;
+        if (n > 2 * NB && !digits.alloc(cx, n - 2 * NB, n - 2 * NB, W)) return false;
+        // C -= L U on rows r0 .. r1-1, columns c0 .. c1-1 with the columns / rows k0 .. k1-1
+        auto update = [&](int k0, int k1, int r0, int r1, int c0, int c1) {
+            if (tm.enabled) tm.flops_update += (cx ? 8.0 : 2.0) * (double)(r1 - r0) * (c1 - c0) * (k1 - k0);
+            return digit_gemm_sub(cx, d_a + (size_t)r0 * n + k0, n, d_a + (size_t)k0 * n + c0, n,
+                                  d_a + (size_t)r0 * n + c0, n, r1 - r0, c1 - c0, k1 - k0, digits, &d_st->code);
+        };
+        bool looked = mode != LuMode::checked;
+        for (int K0 = 0; K0 < n; K0 += W) {
+            const int K1 = std::min(n, K0 + W);
+            if (!looked && K0 >= 192) {
+                // matrices that tie do so early: look once before the bulk of the work
+                looked = true;
+                int code = 0;
+                cudaMemcpyAsync(&code, &d_st->code, sizeof(int), cudaMemcpyDeviceToHost, stream());
+                if (!sync("LU status")) return false;
+                if (code != 0) return true;
+            }
+            for (int b0 = K0; b0 < K1; b0 += 2 * NB) {
+                const int b1 = std::min(K1, b0 + 2 * NB);
+                // the first block's entries have seen chains only: the same in every mode
+                const long long tie = mode == LuMode::checked && b0 > 0 ? kTieUlps : 0;
+                tm.mark(2);
+                if (b0 > K0 && !update(K0, b0, b0, n, b0, b1)) return false;
+                for (int k0 = b0; k0 < b1; k0 += NB) {
+                    const int kb = std::min(NB, n - k0), r1 = k0 + kb;
+                    tm.mark(2);
+                    if (!panel(k0, kb, tie)) return false;
+                    tm.mark(0);
+                    swaps(k0, kb);
+                    if (r1 < b1) {  // the block's second panel
+                        rows_of_u(k0, kb, r1, b1);
+                        PEEC_LAUNCH((k_gemm_rect<T, 64, 32>), dim3((b1 - r1 + 31) / 32, (n - r1 + 63) / 64), 256, 0,
+                                    d_a, n, k0, kb, r1, n, r1, b1, d_st);
+                    }
+                    tm.mark(1);
+                }
+                if (b1 == n) continue;
+                // the block's rows to the right of it
+                if (b0 > K0 && !update(K0, b0, b0, b1, b1, n)) return false;
+                tm.mark(2);
+                rows_of_u(b0, NB, b1, n);
+                PEEC_LAUNCH((k_gemm_rect<T, 32, 64>), dim3((n - b1 + 63) / 64, 1), 256, 0, d_a, n, b0, NB, b0 + NB, b1,
+                            b1, n, d_st);
+                rows_of_u(b0 + NB, b1 - b0 - NB, b1, n);
+                tm.mark(1);
+            }
+            if (K1 < n && !update(K0, K1, K1, n, K1, n)) return false;
         }
     }
     tm.mark(2);
@@ -2615,41 +2599,50 @@ namespace peec {
 // with *hs holding the device status (code 0 ok) and *scale max|A| (NaN
 // ignored).  A zero / non-finite complex row or column gives hs->code 4/5
 // before any factorisation.
-template <class T>
+//
+// again(): puts the original matrix back into d_a; with it, large systems are
+// factored by digit GEMMs in a checked run, and by chains of FP64 FMAs from the
+// start again if that met a near tie of two pivot candidates or a singular
+// pivot: pivots and status are those of the chains in every case.
+template <class T, class Again>
 static int factor_inplace(T *d_a, int n, double pivot_tolerance, bool cx, long long *d_piv, int *d_perm,
-                          double *d_row, double *d_col, double *scale, Status *hs) {
+                          double *d_row, double *d_col, double *scale, Status *hs, LuMode mode, Again again) {
     size_t nn = (size_t)n * n;
     DBuf<Status> st(1);
     DBuf<unsigned long long> mx(1);
     if (!st.p || !mx.p) return -1;
-    cudaMemsetAsync(st.p, 0, sizeof(Status), stream());
-    cudaMemsetAsync(mx.p, 0, sizeof(unsigned long long), stream());
-    if (cx) {
-        // complex_lu.c:275-302: row scales, then column scales of the row-scaled matrix
-        PEEC_LAUNCH(k_row_scale, (unsigned)(((size_t)n * 32 + 255) / 256), 256, 0, (const cplx *)d_a, (cplx *)d_a, n,
-                    d_row, st.p);
-        PEEC_LAUNCH(k_col_max, (n + 31) / 32, 256, 0, (const cplx *)d_a, n, d_col, st.p);
-        PEEC_LAUNCH(k_col_divide, 152 * 16, 256, 0, (cplx *)d_a, n, d_col, st.p);
+    for (;; mode = LuMode::chain) {
+        cudaMemsetAsync(st.p, 0, sizeof(Status), stream());
+        cudaMemsetAsync(mx.p, 0, sizeof(unsigned long long), stream());
+        if (cx) {
+            // complex_lu.c:275-302: row scales, then column scales of the row-scaled matrix
+            PEEC_LAUNCH(k_row_scale, (unsigned)(((size_t)n * 32 + 255) / 256), 256, 0, (const cplx *)d_a, (cplx *)d_a, n,
+                        d_row, st.p);
+            PEEC_LAUNCH(k_col_max, (n + 31) / 32, 256, 0, (const cplx *)d_a, n, d_col, st.p);
+            PEEC_LAUNCH(k_col_divide, 152 * 16, 256, 0, (cplx *)d_a, n, d_col, st.p);
+        }
+        PEEC_LAUNCH(k_max_mag<T>, 152 * 8, 256, 0, d_a, nn, mx.p);
+        unsigned long long bits = 0;
+        cudaMemcpyAsync(&bits, mx.p, sizeof(bits), cudaMemcpyDeviceToHost, stream());
+        cudaMemcpyAsync(hs, st.p, sizeof(Status), cudaMemcpyDeviceToHost, stream());
+        if (!sync("LU scale")) return -1;
+        memcpy(scale, &bits, sizeof(double));
+        if (hs->code != 0 || !isfinite(*scale) || *scale <= 0.0) return 0;
+        double limit = pivot_tolerance * *scale;
+        if (!factor_device<T>(d_a, n, limit, d_piv, st.p, mode)) return -1;
+        size_t perm_smem = (size_t)n * sizeof(int);
+        if (perm_smem > 48 * 1024)
+            cudaFuncSetAttribute(k_perm, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)perm_smem);
+        PEEC_LAUNCH(k_perm, 1, 1024, perm_smem, d_piv, n, d_perm, st.p);
+        cudaMemcpyAsync(hs, st.p, sizeof(Status), cudaMemcpyDeviceToHost, stream());
+        if (!launch_ok("LU permutation") || !sync("LU factorisation")) return -1;
+        if (hs->code == 6) {
+            set_error("LU panel synchronisation timed out");
+            return -1;
+        }
+        if (hs->code == 0 || mode == LuMode::chain) return 0;
+        if (!again()) return -1;
     }
-    PEEC_LAUNCH(k_max_mag<T>, 152 * 8, 256, 0, d_a, nn, mx.p);
-    unsigned long long bits = 0;
-    cudaMemcpyAsync(&bits, mx.p, sizeof(bits), cudaMemcpyDeviceToHost, stream());
-    cudaMemcpyAsync(hs, st.p, sizeof(Status), cudaMemcpyDeviceToHost, stream());
-    if (!sync("LU scale")) return -1;
-    memcpy(scale, &bits, sizeof(double));
-    if (hs->code != 0 || !isfinite(*scale) || *scale <= 0.0) return 0;
-    double limit = pivot_tolerance * *scale;
-    if (!factor_device<T>(d_a, n, limit, d_piv, st.p)) return -1;
-    size_t perm_smem = (size_t)n * sizeof(int);
-    if (perm_smem > 48 * 1024) cudaFuncSetAttribute(k_perm, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)perm_smem);
-    PEEC_LAUNCH(k_perm, 1, 1024, perm_smem, d_piv, n, d_perm, st.p);
-    cudaMemcpyAsync(hs, st.p, sizeof(Status), cudaMemcpyDeviceToHost, stream());
-    if (!launch_ok("LU permutation") || !sync("LU factorisation")) return -1;
-    if (hs->code == 6) {
-        set_error("LU panel synchronisation timed out");
-        return -1;
-    }
-    return 0;
 }
 
 static void report_status(const Status &hs, bool cx) {
@@ -2662,6 +2655,57 @@ static void report_status(const Status &hs, bool cx) {
                            : "ERROR: invalid diagonal U[%d,%d] = %.9e.\n",
                 hs.column, hs.column, hs.value);
 }
+
+// For callers inside the library that can make the matrix again.  Real: the
+// pivots stay inside (the transient system), so near ties need no second run.
+int lu_factor_again(double *d_a, int n, double pivot_tolerance, long long *d_piv, int *d_perm, double *scale,
+                    int *failed_column, const std::function<bool()> &again) {
+    Status hs;
+    if (factor_inplace<double>(d_a, n, pivot_tolerance, false, d_piv, d_perm, nullptr, nullptr, scale, &hs,
+                               n >= kDigitsFromReal ? LuMode::digits : LuMode::chain, again) != 0)
+        return -1;
+    *failed_column = hs.code ? hs.column : -1;
+    if (!isfinite(*scale) || *scale <= 0.0) return -2;
+    if (hs.code) report_status(hs, false);
+    return hs.code ? -2 : 0;
+}
+int complex_lu_factor_again(Complex *d_a, int n, double pivot_tolerance, long long *d_piv, int *d_perm, double *d_row,
+                            double *d_col, const std::function<bool()> &again) {
+    Status hs;
+    double scale = 0.0;
+    if (factor_inplace<cplx>((cplx *)d_a, n, pivot_tolerance, true, d_piv, d_perm, d_row, d_col, &scale, &hs,
+                             n >= kDigitsFromCplx ? LuMode::checked : LuMode::chain, again) != 0)
+        return -1;
+    if (hs.code == 4 || hs.code == 5 || !isfinite(scale) || scale <= 0.0) return -2;
+    if (hs.code) report_status(hs, true);
+    return hs.code ? -2 : 0;
+}
+
+// The device-resident forms keep a copy of the matrix for a second run; where
+// there is no memory for it, chains it is.
+template <class T>
+static int factor_inplace_copy(T *d_a, int n, double pivot_tolerance, bool cx, long long *d_piv, int *d_perm,
+                               double *d_row, double *d_col, double *scale, Status *hs) {
+    const size_t bytes = (size_t)n * n * sizeof(T);
+    void *copy = nullptr;
+    if (n >= (cx ? kDigitsFromCplx : kCheckedFromReal) && cudaMallocAsync(&copy, bytes, stream()) != cudaSuccess) {
+        (void)cudaGetLastError();
+        copy = nullptr;
+    }
+    if (copy && !cuda_ok(cudaMemcpyAsync(copy, d_a, bytes, cudaMemcpyDeviceToDevice, stream()), "LU copy")) {
+        dfree(copy);
+        return -1;
+    }
+    const int s = factor_inplace<T>(d_a, n, pivot_tolerance, cx, d_piv, d_perm, d_row, d_col, scale, hs,
+                                    copy ? LuMode::checked : LuMode::chain, [&] {
+                                        return cuda_ok(cudaMemcpyAsync(d_a, copy, bytes, cudaMemcpyDeviceToDevice,
+                                                                       stream()),
+                                                       "LU copy");
+                                    });
+    dfree(copy);
+    return s;
+}
+
 
 // Shared host driver for both factorisations.  On success the factor stays
 // resident on the device (registry) for the solves.
@@ -2692,7 +2736,10 @@ static int factorize_common(const T *input, size_t n, double pivot_tolerance, bo
     }
     Status hs;
     double scale = 0.0;
-    if (factor_inplace<T>(d_a, ni, pivot_tolerance, cx, r.d_piv, r.d_perm, r.d_row, r.d_col, &scale, &hs) != 0) {
+    const LuMode mode = ni >= (cx ? kDigitsFromCplx : kCheckedFromReal) ? LuMode::checked : LuMode::chain;
+    if (factor_inplace<T>(d_a, ni, pivot_tolerance, cx, r.d_piv, r.d_perm, r.d_row, r.d_col, &scale, &hs, mode, [&] {
+            return cuda_ok(cudaMemcpyAsync(d_a, input, nn * sizeof(T), cudaMemcpyHostToDevice, stream()), "LU upload");
+        }) != 0) {
         release(r);
         return -1;
     }
@@ -2980,7 +3027,7 @@ int peec_gb300_lu_factor_device(double *d_a, size_t n, double pivot_tolerance, l
     if (!d_a || !d_piv || !d_perm || n == 0 || n > (size_t)0x7fffffff) return -1;
     Status hs;
     double scale = 0.0;
-    if (factor_inplace<double>(d_a, (int)n, pivot_tolerance, false, d_piv, d_perm, nullptr, nullptr, &scale, &hs) != 0)
+    if (factor_inplace_copy<double>(d_a, (int)n, pivot_tolerance, false, d_piv, d_perm, nullptr, nullptr, &scale, &hs) != 0)
         return -1;
     if (matrix_scale) *matrix_scale = scale;
     if (failed_column) *failed_column = hs.code ? hs.column : -1;
@@ -2998,7 +3045,7 @@ int peec_gb300_complex_lu_factor_device(Complex *d_a, size_t n, double pivot_tol
     if (!d_a || !d_piv || !d_perm || !d_row_scale || !d_column_scale || n == 0 || n > (size_t)0x7fffffff) return -1;
     Status hs;
     double scale = 0.0;
-    if (factor_inplace<cplx>((cplx *)d_a, (int)n, pivot_tolerance, true, d_piv, d_perm, d_row_scale, d_column_scale,
+    if (factor_inplace_copy<cplx>((cplx *)d_a, (int)n, pivot_tolerance, true, d_piv, d_perm, d_row_scale, d_column_scale,
                              &scale, &hs) != 0)
         return -1;
     if (matrix_scale) *matrix_scale = scale;
@@ -3114,25 +3161,26 @@ extern "C" int peec_gb300_lu_factor_device_noalloc(double *d_a, size_t n, double
         int kb = std::min(NB, ni - k0);
         CoopPlan<double> pl = coop_plan<double>(ni - k0);
         if (pl.G > 0) {
+            long long no_tie = 0;
             int rows = pl.rows;
             double *cr = (double *)sc.cand_row, *kr = (double *)sc.krow;
             void *args[] = {&d_a, (void *)&ni, (void *)&k0, &kb, &rows, &limit, &d_piv, &st, &sc.ps, &sc.cand_val,
-                            &sc.cand_idx, &cr, &kr};
+                            &sc.cand_idx, &cr, &kr, &no_tie};
             if (!cuda_ok(cudaLaunchCooperativeKernel((const void *)k_panel_coop<double>, dim3(pl.G), dim3(256), args,
                                                      pl.smem, stream()),
                          "cooperative panel launch"))
                 return -1;
             note_launch();
         } else {
-            PEEC_LAUNCH(k_panel<double>, 1, 1024, 0, d_a, ni, k0, kb, limit, d_piv, st);
+            PEEC_LAUNCH(k_panel<double>, 1, 1024, 0, d_a, ni, k0, kb, limit, d_piv, st, 0LL);
         }
         PEEC_LAUNCH(k_laswp<double>, (ni + kLaswpCols - 1) / kLaswpCols, 256, 2 * NB * kLaswpCols * sizeof(double), d_a,
                     ni, k0, kb, d_piv, st);
         int rest = ni - (k0 + kb);
         if (rest > 0) {
             PEEC_LAUNCH(k_trsm<double>, (rest + 255) / 256, 256, 0, d_a, ni, k0, kb, k0 + kb, ni, st);
-            dim3 g((rest + 63) / 64, (rest + 63) / 64);
-            PEEC_LAUNCH(k_gemm_real, g, 256, 0, d_a, ni, k0, kb, st);
+            PEEC_LAUNCH((k_gemm_rect<double, 64, 64>), dim3((rest + 63) / 64, (rest + 63) / 64), 256, 0, d_a, ni, k0, kb,
+                        k0 + kb, ni, k0 + kb, ni, st);
         }
     }
     PEEC_LAUNCH(k_check_diag<double>, (ni + 255) / 256, 256, 0, d_a, ni, limit, st);
@@ -3958,20 +4006,21 @@ int mixed_solve_impl(const Complex *d_Z, size_t n_, const Complex *d_b, Complex 
                         return -1;
                     note_launch();
                 } else if (pl.G > 0) {
+                    long long no_tie = 0;
                     int rows = pl.rows;
                     cplxf *cr = (cplxf *)sc.cand_row, *kr = (cplxf *)sc.krow;
                     Status *stp = st.p;
                     long long *pivp = piv.p;
                     int kbv = kb;
                     void *args[] = {&a, (void *)&n, (void *)&k0, &kbv, &rows, (void *)&limit, &pivp, &stp, &sc.ps,
-                                    &sc.cand_val, &sc.cand_idx, &cr, &kr};
+                                    &sc.cand_val, &sc.cand_idx, &cr, &kr, &no_tie};
                     if (!cuda_ok(cudaLaunchCooperativeKernel((const void *)k_panel_coop<cplxf>, dim3(pl.G), dim3(256),
                                                              args, pl.smem, stream()),
                                  "cooperative panel launch"))
                         return -1;
                     note_launch();
                 } else {
-                    PEEC_LAUNCH(k_panel<cplxf>, 1, 1024, 0, a, n, k0, kb, limit, piv.p, st.p);
+                    PEEC_LAUNCH(k_panel<cplxf>, 1, 1024, 0, a, n, k0, kb, limit, piv.p, st.p, 0LL);
                 }
                 tm.mark(0);
                 pdl_launch(k_laswp<cplxf>, dim3((n + kLaswpCols - 1) / kLaswpCols), dim3(256),

@@ -17,6 +17,7 @@
 #include <math.h>
 
 #include "common.cuh"
+#include "digit_gemm.cuh"
 
 namespace peec {
 namespace mrhs {
@@ -29,6 +30,7 @@ struct c32 {
 };
 
 static const int kDB = 64;  // rows of a diagonal block
+static const int kDigitsFrom = 1000;  // unknowns from which the inverse uses digit GEMMs
 
 // Y[i][q] = r[q][perm[i]] / rs[perm[i]] in FP32, through a 32 x 32 tile of
 // shared memory (coalesced on both sides).
@@ -227,8 +229,14 @@ __global__ void __launch_bounds__(256) k_trsm_diag_d(const double *lu, int n, in
             if (lane + 32 > j) v1 = fma(-B[lane + 32][j], xj, v1);
         }
     } else {
+        // reciprocals of the diagonal once; a quotient is then y r corrected by its
+        // remainder (three FP64 operations a step where a division takes about ten)
+        const double r0d = 1.0 / B[lane][lane], r1d = 1.0 / B[lane + 32][lane + 32];
         for (int j = kDB - 1; j >= 0; --j) {
-            const double xj = __shfl_sync(0xffffffffu, j < 32 ? v0 : v1, j & 31) / B[j][j];
+            const double y = __shfl_sync(0xffffffffu, j < 32 ? v0 : v1, j & 31);
+            const double r = __shfl_sync(0xffffffffu, j < 32 ? r0d : r1d, j & 31);
+            const double q = y * r;
+            const double xj = fma(fma(-q, B[j][j], y), r, q);
             if (lane < j) v0 = fma(-B[lane][j], xj, v0);
             if (lane + 32 < j) v1 = fma(-B[lane + 32][j], xj, v1);
             if (lane == (j & 31)) {
@@ -477,25 +485,71 @@ __global__ void k_mark_done(const unsigned long long *be_q, int *done, int nrhs,
 // The inverse of a matrix from its packed FP64 LU factor (unit L, U, row
 // permutation perm as the solves use it): X = U^-1 L^-1 P, i.e. the blocked
 // forward and backward substitution of the permuted identity, all n columns
-// at once, into Minv (n x n row-major).  About 2 n^3 FP64 flops.
+// at once, into Minv (n x n row-major).  About 2 n^3 flops.
 bool inverse_from_lu_real(const double *lu, const int *perm, int n, double *Minv) {
     using namespace mrhs;
     PEEC_LAUNCH(k_permuted_identity, (unsigned)(((size_t)n * n + 255) / 256), 256, 0, perm, n, Minv);
-    const int nb = (n + kDB - 1) / kDB;
     const unsigned dgrid = (unsigned)((n + 7) / 8);
-    for (int blk = 0; blk < nb; ++blk) {
-        const int r0 = blk * kDB, nrow = min(kDB, n - r0), r1 = r0 + nrow;
-        PEEC_LAUNCH(k_trsm_diag_d<true>, dgrid, 256, 0, lu, n, r0, nrow, Minv, n);
-        if (r1 < n)
-            PEEC_LAUNCH(k_dgemm_sub, dim3((n + 63) / 64, (n - r1 + 63) / 64), 256, 0, lu + (size_t)r1 * n + r0, n,
-                        Minv + (size_t)r0 * n, Minv + (size_t)r1 * n, n, n - r1, n, nrow);
+    auto block = [&](bool lower, int r0, int nrow) {
+        if (lower)
+            PEEC_LAUNCH(k_trsm_diag_d<true>, dgrid, 256, 0, lu, n, r0, nrow, Minv, n);
+        else
+            PEEC_LAUNCH(k_trsm_diag_d<false>, dgrid, 256, 0, lu, n, r0, nrow, Minv, n);
+    };
+    if (n < kDigitsFrom) {
+        const int nb = (n + kDB - 1) / kDB;
+        for (int blk = 0; blk < nb; ++blk) {
+            const int r0 = blk * kDB, nrow = min(kDB, n - r0), r1 = r0 + nrow;
+            block(true, r0, nrow);
+            if (r1 < n)
+                PEEC_LAUNCH(k_dgemm_sub, dim3((n + 63) / 64, (n - r1 + 63) / 64), 256, 0, lu + (size_t)r1 * n + r0, n,
+                            Minv + (size_t)r0 * n, Minv + (size_t)r1 * n, n, n - r1, n, nrow);
+        }
+        for (int blk = nb - 1; blk >= 0; --blk) {
+            const int r0 = blk * kDB, nrow = min(kDB, n - r0);
+            block(false, r0, nrow);
+            if (r0 > 0)
+                PEEC_LAUNCH(k_dgemm_sub, dim3((n + 63) / 64, (r0 + 63) / 64), 256, 0, lu + r0, n,
+                            Minv + (size_t)r0 * n, Minv, n, r0, n, nrow);
+        }
+        return launch_ok("inverse from the LU factor");
     }
-    for (int blk = nb - 1; blk >= 0; --blk) {
-        const int r0 = blk * kDB, nrow = min(kDB, n - r0);
-        PEEC_LAUNCH(k_trsm_diag_d<false>, dgrid, 256, 0, lu, n, r0, nrow, Minv, n);
-        if (r0 > 0)
-            PEEC_LAUNCH(k_dgemm_sub, dim3((n + 63) / 64, (r0 + 63) / 64), 256, 0, lu + r0, n, Minv + (size_t)r0 * n,
-                        Minv, n, r0, n, nrow);
+    // Digit GEMMs: outer blocks of their largest K, inside them each diagonal
+    // block's rows first get what the block's solved rows contribute.
+    const int W = kDigitMaxKReal;
+    DigitScratch digits;
+    DBuf<int> code(1);
+    if (!digits.alloc(false, n, n, W) || !code.p) return false;
+    cudaMemsetAsync(code.p, 0, sizeof(int), stream());
+    // rows r0 .. r1-1 of Minv -= (rows r0 .., columns k0 .. k1-1 of the factor) rows k0 .. k1-1 of Minv
+    auto update = [&](int r0, int r1, int k0, int k1) {
+        return digit_gemm_sub(false, lu + (size_t)r0 * n + k0, n, Minv + (size_t)k0 * n, n, Minv + (size_t)r0 * n, n,
+                              r1 - r0, n, k1 - k0, digits, code.p);
+    };
+    for (int K0 = 0; K0 < n; K0 += W) {  // forward: unit lower
+        const int K1 = min(n, K0 + W);
+        for (int r0 = K0; r0 < K1; r0 += kDB) {
+            const int r1 = min(K1, r0 + kDB);
+            if (r0 > K0 && !update(r0, r1, K0, r0)) return false;
+            block(true, r0, r1 - r0);
+        }
+        if (K1 < n && !update(K1, n, K0, K1)) return false;
+    }
+    for (int K0 = (n - 1) / W * W; K0 >= 0; K0 -= W) {  // backward: upper
+        const int K1 = min(n, K0 + W);
+        for (int r0 = K0 + (K1 - 1 - K0) / kDB * kDB; r0 >= K0; r0 -= kDB) {
+            const int r1 = min(K1, r0 + kDB);
+            if (r1 < K1 && !update(r0, r1, r1, K1)) return false;
+            block(false, r0, r1 - r0);
+        }
+        if (K0 > 0 && !update(0, K0, K0, K1)) return false;
+    }
+    int hcode = 0;
+    cudaMemcpyAsync(&hcode, code.p, sizeof(int), cudaMemcpyDeviceToHost, stream());
+    if (!sync("inverse from the LU factor")) return false;
+    if (hcode != 0) {
+        set_error("inverse from the LU factor: a wait inside a digit GEMM ran out");
+        return false;
     }
     return launch_ok("inverse from the LU factor");
 }

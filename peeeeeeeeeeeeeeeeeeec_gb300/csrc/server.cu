@@ -16,6 +16,7 @@
 #include <chrono>
 #include <condition_variable>
 #include <deque>
+#include <functional>
 #include <map>
 #include <memory>
 #include <mutex>
@@ -24,8 +25,12 @@
 
 #include "../../include/peec_gb300.h"
 #include "common.cuh"
+#include "digit_gemm.cuh"
 
 namespace peec {
+
+int complex_lu_factor_again(Complex *d_a, int n, double pivot_tolerance, long long *d_piv, int *d_perm, double *d_row,
+                            double *d_col, const std::function<bool()> &again);
 
 int transient_lightning_runs(void *system, int nrun, const double *K, const double *alpha, const double *beta,
                              const double *delay, const size_t *strike_node, const size_t *return_node,
@@ -122,6 +127,10 @@ class Server {
         // also keeps Z as float pairs for its residual
         j->bytes = 32 * n * n + (r->mixed ? 9216 * n : 0) + (r->mixed && r->nrhs >= 32 ? 16 * n * n : 0) +
                    112 * n * r->nrhs + (64 << 20);
+        // the FP64 factorisation's digits, beyond those 64 MiB (counted where the
+        // budget holds them: it can do without)
+        const size_t digits = digit_scratch_bytes(true, n, n, kDigitMaxKCplx);
+        if (digits > (64 << 20) && j->bytes + j->mesh_bytes + digits <= budget_) j->bytes += digits;
         return enqueue(j);
     }
 
@@ -392,9 +401,9 @@ class Server {
             DBuf<double> rs(n), cs(n);
             if (!W.alloc(n * n) || !piv.p || !perm.p || !rs.p || !cs.p) return -1;
             if (peec_gb300_copy_device(W.p, Z.p, n * n * sizeof(Complex)) != 0) return -1;
-            double scale;
-            int col;
-            status = peec_gb300_complex_lu_factor_device(W.p, n, 1e-14, piv.p, perm.p, rs.p, cs.p, &scale, &col);
+            status = complex_lu_factor_again(W.p, (int)n, 1e-14, piv.p, perm.p, rs.p, cs.p, [&] {
+                return peec_gb300_copy_device(W.p, Z.p, n * n * sizeof(Complex)) == 0;
+            });
             if (status == 0)
                 status = peec_gb300_complex_lu_solve_device(W.p, perm.p, rs.p, cs.p, n, B.p, X.p, nrhs);
             if (status == 0) {

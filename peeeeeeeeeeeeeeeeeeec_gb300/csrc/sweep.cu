@@ -29,6 +29,7 @@
 #include <string.h>
 
 #include <algorithm>
+#include <functional>
 #include <vector>
 
 #include "../../include/peec_gb300.h"
@@ -37,6 +38,8 @@
 
 namespace peec {
 
+int complex_lu_factor_again(Complex *d_a, int n, double pivot_tolerance, long long *d_piv, int *d_perm, double *d_row,
+                            double *d_col, const std::function<bool()> &again);
 bool launch_harmonic_fill_dev(const double *L, const double *P, const int *edges, const double *R, int ne, int nv,
                               const double *omega_dev, void *Z);
 bool launch_plane_waves_dev(const double *centers, const double *vectors, int ne, int nv, int nrhs,
@@ -176,9 +179,10 @@ static int solve_fallback(SweepPlan &p, double freq, double tol, Complex *d_X, d
     if (!lu.p || !piv.p || !perm.p || !rs.p || !cs.p) return -1;
     if (!cuda_ok(cudaMemcpyAsync(lu.p, p.d_Z, nn * sizeof(Complex), cudaMemcpyDeviceToDevice, stream()), "sweep: Z"))
         return -1;
-    double scale = 0.0;
-    int col = -1;
-    if (peec_gb300_complex_lu_factor_device(lu.p, (size_t)p.n, 1e-14, piv.p, perm.p, rs.p, cs.p, &scale, &col) != 0)
+    if (complex_lu_factor_again(lu.p, p.n, 1e-14, piv.p, perm.p, rs.p, cs.p, [&] {
+            return cuda_ok(cudaMemcpyAsync(lu.p, p.d_Z, nn * sizeof(Complex), cudaMemcpyDeviceToDevice, stream()),
+                           "sweep: Z");
+        }) != 0)
         return -1;
     if (s != 1 &&
         peec_gb300_complex_lu_solve_device(lu.p, perm.p, rs.p, cs.p, (size_t)p.n, p.d_b, d_X, (size_t)p.nrhs) != 0)

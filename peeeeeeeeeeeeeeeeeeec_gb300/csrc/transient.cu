@@ -20,6 +20,7 @@
 #include <math.h>
 #include <string.h>
 
+#include <functional>
 #include <vector>
 
 #include "../../include/peec_gb300.h"
@@ -28,6 +29,8 @@
 namespace peec {
 
 bool inverse_from_lu_real(const double *lu, const int *perm, int n, double *Minv);
+int lu_factor_again(double *d_a, int n, double pivot_tolerance, long long *d_piv, int *d_perm, double *scale,
+                    int *failed_column, const std::function<bool()> &again);
 
 struct TransientSystem {
     int ne = 0, nv = 0, nt = 0, scheme = 0;
@@ -547,7 +550,11 @@ static int create(const double *d_L, const double *d_P, const int *d_edges, cons
     PEEC_LAUNCH(k_self_capacitance, (nv + 255) / 256, 256, 0, d_P, nv, S.F, bad.p);
     size_t nas = (size_t)ne * nv;
     PEEC_LAUNCH(k_as_build, (unsigned)((nas + 255) / 256), 256, 0, d_P, S.edges, ne, nv, S.AS);
-    PEEC_LAUNCH(k_transient_fill, 152 * 16, 256, 0, d_L, S.R, S.AS, S.F, S.edges, ne, nv, S.theta, dt, S.lu);
+    auto fill_matrix = [&] {
+        PEEC_LAUNCH(k_transient_fill, 152 * 16, 256, 0, d_L, S.R, S.AS, S.F, S.edges, ne, nv, S.theta, dt, S.lu);
+        return launch_ok("transient matrix");
+    };
+    if (!fill_matrix()) return -1;
     int hbad = 0;
     cudaMemcpyAsync(&hbad, bad.p, sizeof(int), cudaMemcpyDeviceToHost, st);
     if (!launch_ok("transient system") || !sync("transient system")) return -1;
@@ -566,13 +573,13 @@ static int create(const double *d_L, const double *d_P, const int *d_edges, cons
                 (float *)nullptr);
     PEEC_LAUNCH(k_split_rows, (unsigned)(((size_t)ne * S.ldn + 255) / 256), 256, 0, S.AS, ne, nv, S.ldn, S.ASf,
                 (float *)nullptr);
-    if (!launch_ok("transient split") || !sync("transient split")) return -1;
-    dfree(S.AS);
-    S.AS = nullptr;
+    if (!launch_ok("transient split")) return -1;
     double scale;
     int col;
-    int s = peec_gb300_lu_factor_device(S.lu, nt, 1.0e-14, S.piv, S.perm, &scale, &col);
+    int s = lu_factor_again(S.lu, nt, 1.0e-14, S.piv, S.perm, &scale, &col, fill_matrix);
     if (s != 0) return s == -2 ? -2 : -1;
+    dfree(S.AS);  // (the factorisation may fill the matrix again)
+    S.AS = nullptr;
     // M^-1 from the factor, once (the factor is not needed afterwards), kept
     // as float pairs for the double-float applies
     const size_t nn = (size_t)nt * nt;
