@@ -94,9 +94,9 @@ int peec_gb300_set_near_reuse(int on);
  * column of a singular pivot, or -1.  Large systems (complex from 1300, real
  * from 5000 unknowns) are updated on the tensor cores from integer digits; for
  * that the call holds a copy of the matrix while it runs (without the memory
- * for it, FP64 FMAs do the updates): where two pivot candidates come within
- * 2^-34 of each other it starts again with FP64 FMAs, so pivots and status do
- * not depend on the form of the updates. */
+ * for it, FP64 FMAs do the updates): where two pivot candidates are so close
+ * that rounding could decide between them it starts again with FP64 FMAs, so
+ * pivots and status do not depend on the form of the updates. */
 int peec_gb300_lu_factor_device(double *d_a, size_t n, double pivot_tolerance,
                                 long long *d_piv, int *d_perm, double *matrix_scale,
                                 int *failed_column);

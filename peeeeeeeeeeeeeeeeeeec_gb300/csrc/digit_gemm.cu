@@ -12,15 +12,18 @@
 // digits i and j has weight 2^(2 - 7 (i + j)): the pairs with the same sum i + j
 // up to kDigits + 1 are added up in one TMEM accumulator each.  Such a sum of at
 // most ten pairs is an integer below 2^24 (10 x 2 K x 2^12 at K = 192 complex, 10 x
-// K x 2^12 at K = 256 real), so FP32 accumulation is exact.
+// K x 2^12 at K = 256 real), so FP32 accumulation is exact (the last two sums could
+// round by a unit of 2^-82 at worst).
 //
-// The sums are combined in 84-bit integers of unit 2^-82 and leave them once,
+// The sums are combined in 90-bit integers of unit 2^-89 and leave them once,
 // rounded to FP64, for the subtraction from C: the only FP64 operation of an
-// update.  Its error is about 2^-71 |row of A| |column of B| (what is dropped).
+// update.  Its error is about 2^-78 |row of A| |column of B| (what is dropped).
 // A chain of K FP64 FMAs rounds at 2^-53 of its running sum, so entries whose C
 // and update are both below 2^-kExactBelow |row| |column| are left out and done
-// by that chain (matrices of weakly coupled parts, systems at kHz): no entry is
-// less accurate than on the FP64 pipe.
+// in FP64 (matrices of weakly coupled parts, systems at kHz): no entry is
+// less accurate than on the FP64 pipe.  (Eleven digits, 66 pairs, with the line
+// at 2^-18: 5% faster on random matrices, but 341 against 294 ms for the solve of
+// the 8402-unknown box, where more entries take the FP64 way.)
 //
 // Operands.  Two kernels write the digits in the layout that the MMA reads
 // from shared memory (K-major rows of 16 BF16 = 32 bytes, 32-byte swizzle),
@@ -52,7 +55,9 @@ using tc::mma_bf16;
 using tc::mma_commit;
 using tc::smem_u32;
 
-static const int kDigits = 11;  // 66 digit pairs
+static const int kDigits = 12;              // 78 digit pairs
+static const int kLowBits = 7 * (kDigits - 9);  // of the digits kept apart while they are cut (63 bits hold nine)
+static const int kUnit = 7 * (kDigits + 1) - 2;  // sums are in units of 2^-kUnit
 static const int kBM = 128;  // rows of a tile
 static const int kKC = 16;   // K of a block: one MMA
 static const int kNotFinite = 1 << 28;  // exponent of a row or column with an infinity or NaN
@@ -102,8 +107,8 @@ __device__ __forceinline__ int norm_shift(float sq) {
 }
 
 // The scaled x 2^(shift + 1022 - emax) (emax: at least the biased exponent of x
-// 2^shift, so that it is below 1) in units of 2^(1 - 7 kDigits) = 2^-76, as hi 2^14 +
-// lo, 0 <= lo < 2^14: two digits in lo, the others in hi.
+// 2^shift, so that it is below 1) in units of 2^(1 - 7 kDigits), as hi 2^kLowBits + lo,
+// 0 <= lo < 2^kLowBits: the lowest digits in lo, nine in hi.
 struct Fixed {
     long long hi;
     unsigned lo;
@@ -114,24 +119,25 @@ __device__ __forceinline__ Fixed fixed_point(double x, int shift, int emax) {
     Fixed r = {0, 0u};
     if (ex == 0) return r;
     const unsigned long long m = (b & 0xFFFFFFFFFFFFFull) | 0x10000000000000ull;
-    const int sh = ex + shift - emax + 23;  // at most 23
+    constexpr unsigned mask = (1u << kLowBits) - 1u;
+    const int sh = ex + shift - emax + 9 + kLowBits;  // at most 9 + kLowBits
     unsigned long long hi;
-    if (sh >= 14) {
-        hi = m << (sh - 14);
+    if (sh >= kLowBits) {
+        hi = m << (sh - kLowBits);
     } else if (sh >= 0) {
-        hi = m >> (14 - sh);
-        r.lo = (unsigned)(m << sh) & 0x3fffu;
+        hi = m >> (kLowBits - sh);
+        r.lo = (unsigned)(m << sh) & mask;
     } else if (sh > -56) {
         const unsigned long long v = (m + (1ull << (-sh - 1))) >> -sh;
-        hi = v >> 14;
-        r.lo = (unsigned)v & 0x3fffu;
+        hi = v >> kLowBits;
+        r.lo = (unsigned)v & mask;
     } else {
         hi = 0;
     }
     r.hi = (long long)hi;
     if (b >> 63) {
         r.hi = (long long)(~hi + (r.lo == 0 ? 1u : 0u));
-        r.lo = (0u - r.lo) & 0x3fffu;
+        r.lo = (0u - r.lo) & mask;
     }
     return r;
 }
@@ -161,10 +167,10 @@ __global__ void __launch_bounds__(256) k_row_exponents(const double *B, size_t l
 // number, counted from 0; the last one left is the leading digit (-64 .. 64).
 __device__ __forceinline__ float next_digit(Fixed &X, int s) {
     int d;
-    if (s >= kDigits - 2) {  // the two lowest, in lo, then a carry into hi
+    if (s >= 9) {  // the lowest, in lo, then a carry into hi
         d = (int)(X.lo << 25) >> 25;
         X.lo = (unsigned)((int)X.lo - d) >> 7;
-        if (s == kDigits - 2) X.hi += X.lo;
+        if (s == 9) X.hi += X.lo;
     } else if (s > 0) {
         d = (int)((unsigned)X.hi << 25) >> 25;
         X.hi = (X.hi - d) >> 7;
@@ -386,16 +392,17 @@ __device__ __forceinline__ int integer(float x) {
     return (__float_as_int(t) - 0x4B400000) * 2048 + (__float_as_int(r + M) - 0x4B400000);
 }
 
-// (v 2^20 + low) 2^(E - 20) as FP64 bits, low: the low 20 bits of its argument:
-// rounded once to 53 bits by integer operations (an FP64 conversion takes one
-// of GB300's two FP64 slots per clock and SM).  No branches: eight of these
-// run interleaved.  Results below 2^-1022 are zero.
+// v 2^E and the kUnit - 62 low bits of `low` below it, as FP64 bits: rounded once
+// to 53 bits by integer operations (an FP64 conversion takes one of GB300's two
+// FP64 slots per clock and SM).  No branches: eight of these run interleaved.
+// Results below 2^-1022 are zero.
 __device__ __forceinline__ long long compose(long long v, unsigned low, int E) {
     const unsigned sign = (unsigned)((int)(v >> 32) >> 31);
-    low = ((low ^ sign) & 0xfffffu) - sign;  // negated below: ~x + 1 over both words
-    const unsigned long long a = ((unsigned long long)v ^ ((unsigned long long)sign << 32 | sign)) + (low >> 20);
+    constexpr int bits = kUnit - 62;
+    low = ((low ^ sign) & ((1u << bits) - 1u)) - sign;  // negated: ~x + 1 over both words
+    const unsigned long long a = ((unsigned long long)v ^ ((unsigned long long)sign << 32 | sign)) + (low >> bits);
     unsigned hi = (unsigned)(a >> 32), lo = (unsigned)a;
-    low <<= 12;
+    low <<= 32 - bits;
 #pragma unroll
     for (int t = 0; t < 2; ++t) {  // leading zero words
         const bool z = hi == 0;
@@ -447,7 +454,7 @@ struct Args {
     int *code;
 };
 
-static const int kExactBelow = 18;  // entries below 2^-18 of |row| |column| take the FP64 chain
+static const int kExactBelow = 25;  // entries below 2^-25 of |row| |column| take the FP64 way
 // |v| 2^-62 below 2^-kExactBelow
 __device__ __forceinline__ bool below(long long v) {
     return (unsigned)((int)(v >> 32) + (1 << (30 - kExactBelow))) < (2u << (30 - kExactBelow));
@@ -457,29 +464,63 @@ __device__ __forceinline__ bool below(double z, int E) {
     return (int)((__double_as_longlong(z) >> 52) & 0x7ff) < E + 1023 - kExactBelow;
 }
 
-// One entry of C -= A B as a chain of FP64 FMAs.
+// One entry of C -= A B in FP64: K products from k0 on, `step` apart.
 template <bool CX>
-__device__ __noinline__ void exact_entry(const Args &A, int i, int j) {
+__device__ __forceinline__ double2 exact_sum(const Args &A, int i, int j, int k0, int step) {
+    double2 z = make_double2(0.0, 0.0);
     if constexpr (CX) {
         const double2 *a = reinterpret_cast<const double2 *>(A.a64) + (size_t)i * A.lda;
         const double2 *b = reinterpret_cast<const double2 *>(A.b64) + j;
-        double2 *c = reinterpret_cast<double2 *>(A.c) + (size_t)i * A.ldc + j;
-        double2 z = *c;
-#pragma unroll 4
-        for (int k = 0; k < A.k; ++k) {
+#pragma unroll 2
+        for (int k = k0; k < A.k; k += step) {
             const double2 x = a[k], y = b[(size_t)k * A.ldb];
-            if (y.x == 0.0 && y.y == 0.0 && isfinite(x.x) && isfinite(x.y)) continue;  // sparse columns
-            z.x = fma(x.y, y.y, fma(-x.x, y.x, z.x));
-            z.y = fma(-x.y, y.x, fma(-x.x, y.y, z.y));
+            z.x = fma(-x.y, y.y, fma(x.x, y.x, z.x));
+            z.y = fma(x.y, y.x, fma(x.x, y.y, z.y));
         }
-        *c = z;
     } else {
         const double *a = A.a64 + (size_t)i * A.lda, *b = A.b64 + j;
-        double *c = A.c + (size_t)i * A.ldc + j;
-        double z = *c;
-#pragma unroll 8
-        for (int k = 0; k < A.k; ++k) z = fma(-a[k], b[(size_t)k * A.ldb], z);
-        *c = z;
+#pragma unroll 4
+        for (int k = k0; k < A.k; k += step) z.x = fma(a[k], b[(size_t)k * A.ldb], z.x);
+    }
+    return z;
+}
+template <bool CX>
+__device__ __forceinline__ void exact_update(const Args &A, int i, int j, double2 z) {
+    if constexpr (CX) {
+        double2 *c = reinterpret_cast<double2 *>(A.c) + (size_t)i * A.ldc + j;
+        const double2 y = *c;
+        *c = make_double2(y.x - z.x, y.y - z.y);
+    } else {
+        A.c[(size_t)i * A.ldc + j] -= z.x;
+    }
+}
+// The entries of rows row0 + lane whose column (from col0) has a bit in the lane's
+// mask.  An FP64 instruction of a warp takes 64 cycles whatever its lanes do:
+// with many lanes at work each takes an entry of its own, else the lanes share
+// the products of one entry at a time (K = 192 complex: 768 instructions a round
+// against 34 an entry).
+template <bool CX>
+__device__ __noinline__ void exact_entries(const Args &A, int row0, int col0, unsigned mask) {
+    const int lane = threadIdx.x & 31;
+    for (;;) {
+        const unsigned busy = __ballot_sync(0xffffffffu, mask != 0);
+        if (busy == 0) return;
+        if (__popc(busy) >= 20) {
+            if (mask != 0) {
+                const int j = col0 + __ffs((int)mask) - 1;
+                mask &= mask - 1;
+                exact_update<CX>(A, row0 + lane, j, exact_sum<CX>(A, row0 + lane, j, 0, 1));
+            }
+            __syncwarp();
+            continue;
+        }
+        const int from = __ffs((int)busy) - 1;
+        const int i = row0 + from, j = col0 + __ffs(__shfl_sync(0xffffffffu, (int)mask, from)) - 1;
+        if (lane == from) mask &= mask - 1;
+        double2 z = exact_sum<CX>(A, i, j, lane, 32);
+        z.x = warp_sum(z.x);
+        if constexpr (CX) z.y = warp_sum(z.y);
+        if (lane == from) exact_update<CX>(A, i, j, z);
     }
 }
 
@@ -741,9 +782,9 @@ __global__ void __launch_bounds__(32 * (2 + kEpiWarps), 1) k_digit_gemm(Args A) 
             fetch(1);
             const int er = A.ea[row0 + lane];
             const int ec = A.eb[col0 + lane % S::kWarpCols];
-            // Sums of i + j <= 9 in units of 2^-61; then bits 52 and up of the sum in
-            // units of 2^-82 go to TMEM and its low 64 bits (modulo 2^64) stay: what is
-            // still added is below 2^-30, one unit of bit 52.
+            // Sums of i + j <= 9 in units of 2^-61; then the sum in units of 2^-30 goes to
+            // TMEM and its low 64 bits (modulo 2^64) in units of 2^-kUnit stay: what is
+            // still added is below 2^-30.
             long long run[32];
 #pragma unroll
             for (int c = 0; c < 32; ++c) run[c] = 0;
@@ -774,7 +815,7 @@ __global__ void __launch_bounds__(32 * (2 + kEpiWarps), 1) k_digit_gemm(Args A) 
 #pragma unroll
                         for (int c = 0; c < 16; ++c) {
                             top[c] = (int)(run[16 * p + c] >> 31);
-                            run[16 * p + c] <<= 21;
+                            run[16 * p + c] <<= kUnit - 61;
                         }
                         tmem_st16(ts + 16 * p, top);
                     }
@@ -788,7 +829,7 @@ __global__ void __launch_bounds__(32 * (2 + kEpiWarps), 1) k_digit_gemm(Args A) 
             }
             tmem_wait_st();
             // C -= sums 2^(row exponent + column exponent), a chunk at a time
-            unsigned exact = 0;  // columns of this lane's row left to the FP64 chain
+            unsigned exact = 0;  // columns of this lane's row left to FP64
 #pragma unroll
             for (int ch = 0; ch < S::kChunks; ++ch) {
                 unsigned char *buf = mine + (ch & 1) * S::kChunkBytes;
@@ -798,10 +839,11 @@ __global__ void __launch_bounds__(32 * (2 + kEpiWarps), 1) k_digit_gemm(Args A) 
                 tmem_ld4(ts + (CX ? ch * 4 : ch * 8), top);
                 tmem_ld4(ts + (CX ? 16 + ch * 4 : ch * 8 + 4), top + 4);
                 tmem_wait_ld(top, top + 4);
-                // the whole sum's bits 20 and up (units of 2^-62)
+                // the whole sum in units of 2^-62; the bits below stay in r
                 auto upper = [&](long long r, int t) {
-                    const int d = (int)((unsigned)(r >> 32) - ((unsigned)t << 20)) >> 20;  // the carry from below
-                    return (long long)(t + d) * (1ll << 32) | (long long)((unsigned long long)r << 12 >> 32);
+                    constexpr int top = 94 - kUnit;  // bits of r above 2^-30: t modulo 2^top and a carry from below
+                    const int d = (int)((unsigned)(r >> 32) - ((unsigned)t << (32 - top))) >> (32 - top);
+                    return (long long)(t + d) * (1ll << 32) | (long long)((unsigned long long)r << top >> 32);
                 };
                 Scalar *p = reinterpret_cast<Scalar *>(buf + lane * S::kRowStride);
                 double w[8];            // re, im of four columns, or eight columns
@@ -850,13 +892,8 @@ __global__ void __launch_bounds__(32 * (2 + kEpiWarps), 1) k_digit_gemm(Args A) 
                     copy_commit();
             }
             if (row0 + lane >= A.m) exact = 0;
-            while (__any_sync(0xffffffffu, exact != 0)) {
-                if (exact == 0) continue;
-                const int col = __ffs((int)exact) - 1;
-                exact &= exact - 1;
-                if (col0 + col < A.n)
-                    exact_entry<CX>(A, row0 + lane, col0 + col);
-            }
+            exact &= col0 + S::kWarpCols <= A.n ? 0xffffffffu : A.n > col0 ? (1u << (A.n - col0)) - 1u : 0u;
+            if (__any_sync(0xffffffffu, exact != 0)) exact_entries<CX>(A, row0, col0, exact);
         }
     leave:
         if (!ok) s_abort = 1;

@@ -136,26 +136,25 @@ __global__ void k_max_mag(const T *a, size_t count, unsigned long long *out) {
 }
 
 // Near ties.  A checked factorisation (tie > 0) stops with status 7 when another
-// candidate's magnitude is within `tie` ulps of the pivot's: there the pivot
-// would depend on how its column's earlier updates were rounded.
-static const long long kTieUlps = 1LL << 18;  // 2^-34 relative
-__device__ __forceinline__ bool near_tie(double m, double best, long long tie) {
-    return __double_as_longlong(m) >= __double_as_longlong(best) - tie;  // both finite, best > 0; m = -1: none
+// candidate's magnitude comes within the fraction `tie` of the pivot's: there
+// the pivot could depend on how its column's earlier updates were rounded.
+__device__ __forceinline__ long long tie_limit(double best, double tie) {
+    return __double_as_longlong(fmax(fma(best, -tie, best), 0.0));
+}
+__device__ __forceinline__ bool near_tie(double m, long long limit) {  // m = -1: no candidate
+    return __double_as_longlong(m) >= limit;
 }
 // the same of an entry whose magnitude is not at hand, behind a cheap bound
-__device__ __forceinline__ bool near_tie_of(double v, double best, long long tie) {
-    return near_tie(fabs(v), best, tie);
-}
-__device__ __forceinline__ bool near_tie_of(cplx v, double best, long long tie) {
-    const int b = (int)(__double_as_longlong(best) >> 52) - 1;
+__device__ __forceinline__ bool near_tie_of(double v, long long limit) { return near_tie(fabs(v), limit); }
+__device__ __forceinline__ bool near_tie_of(cplx v, long long limit) {
     const int e = max((int)(__double_as_longlong(v.re) >> 52 & 0x7ff), (int)(__double_as_longlong(v.im) >> 52 & 0x7ff));
-    return e >= b && near_tie(mag(v), best, tie);
+    return e + 1 >= (int)(limit >> 52) && near_tie(mag(v), limit);
 }
 
 // ---- panel ----------------------------------------------------------
 template <class T>
 __global__ void __launch_bounds__(1024) k_panel(T *a, int n, int k0, int kb, double limit, long long *piv,
-                                                Status *st, long long tie) {
+                                                Status *st, double tie) {
     __shared__ double s_val[32];
     __shared__ int s_idx[32];
     __shared__ int s_pivot;
@@ -222,7 +221,7 @@ __global__ void __launch_bounds__(1024) k_panel(T *a, int n, int k0, int kb, dou
         __syncthreads();
         if (s_fail) return;
         const int p = s_pivot;
-        const double pivot_mag = s_val[0];
+        const long long tie_at = tie_limit(s_val[0], tie);
         if (p != k) {
             for (int j = k0 + tid; j < k0 + kb; j += nthr) {
                 T t = a[(size_t)k * n + j];
@@ -238,7 +237,7 @@ __global__ void __launch_bounds__(1024) k_panel(T *a, int n, int k0, int kb, dou
         for (int i = k + 1 + tid; i < n; i += nthr) {
             T *row = a + (size_t)i * n + k0;
             if constexpr (!std::is_same<T, cplxf>::value)
-                if (tie > 0 && near_tie_of(row[kk], pivot_mag, tie)) atomicCAS(&st->code, 0, 7);
+                if (tie > 0.0 && near_tie_of(row[kk], tie_at)) atomicCAS(&st->code, 0, 7);
             T m = divide(row[kk], pivot);
             row[kk] = m;
             for (int j = kk + 1; j < kb; ++j) row[j] = msub(row[j], m, s_row[j]);
@@ -331,7 +330,7 @@ __device__ __forceinline__ bool grid_barrier(PanelSlots *ps, unsigned int nblock
 template <class T>
 __global__ void __launch_bounds__(256) k_panel_coop(T *a, int n, int k0, int kb, int rows_per_cta, double limit,
                                                     long long *piv, Status *st, PanelSlots *ps, double *cand_val,
-                                                    int *cand_idx, T *cand_row, T *krow, long long tie) {
+                                                    int *cand_idx, T *cand_row, T *krow, double tie) {
     extern __shared__ unsigned char smem_raw[];
     T *tile = reinterpret_cast<T *>(smem_raw);  // [rows_per_cta][kPS] (padded rows: no bank conflicts)
     using M = typename MagType<T>::type;  // FP32 magnitudes for the FP32 factorisation
@@ -464,7 +463,7 @@ __global__ void __launch_bounds__(256) k_panel_coop(T *a, int n, int k0, int kb,
         __syncthreads();
         if (s_fail) return;
         const int p = s_p, pc = s_pc;
-        const double pivot_mag = (double)s_val[0];
+        const long long tie_at = tie_limit((double)s_val[0], tie);
         // the new row k is the published row p (full panel width: columns
         // < kk hold earlier multipliers and move with the row)
         const T *prow_g = cand_row + ((size_t)par * G + pc) * NB;
@@ -483,7 +482,7 @@ __global__ void __launch_bounds__(256) k_panel_coop(T *a, int n, int k0, int kb,
         for (int i = max(r0, k + 1) + tid; i < r1; i += blockDim.x) {
             T *row = tile + (i - r0) * kPS;
             if constexpr (!std::is_same<T, cplxf>::value)
-                if (tie > 0 && near_tie_of(row[kk], pivot_mag, tie)) atomicCAS(&st->code, 0, 7);
+                if (tie > 0.0 && near_tie_of(row[kk], tie_at)) atomicCAS(&st->code, 0, 7);
             T m = divide(row[kk], pivot);
             row[kk] = m;
             for (int j = kk + 1; j < kb; ++j) row[j] = msub(row[j], m, s_prow[j]);
@@ -777,7 +776,7 @@ __global__ void __launch_bounds__(kLeanThreads) k_panel_lean64(T *a, int n, int 
                                                                long long *piv, Status *st, PanelSlots *ps,
                                                                unsigned long long *flag, int flag_stride,
                                                                int *cand_idx, double *cand_val, T *cand_row,
-                                                               T *krow, long long tie) {
+                                                               T *krow, double tie) {
     __shared__ T tile[kLeanThreads][kPS];
     __shared__ T s_prow[2][NB];
     __shared__ double s_wv[2], s_gb;
@@ -936,7 +935,7 @@ __global__ void __launch_bounds__(kLeanThreads) k_panel_lean64(T *a, int n, int 
         const int p = s_p;
         // (mv still is this row's candidate; every CTA has passed the status
         // check at the top: the flags of this column were all published)
-        if (tie > 0 && mine && i >= k && i != p && near_tie(mv, gb, tie)) atomicCAS(&st->code, 0, 7);
+        if (tie > 0.0 && mine && i >= k && i != p && near_tie(mv, tie_limit(gb, tie))) atomicCAS(&st->code, 0, 7);
         if (p != k) {
             if (warp == 0 && k >= r0 && k < r1 && lane < kb) tile[k - r0][lane] = pcur[lane];
             if (warp == 1 && gc == c && lane < kb) tile[p - r0][lane] = kval;
@@ -2371,6 +2370,14 @@ static const int kDigitsFromReal = 2000;
 static const int kCheckedFromReal = 5000;
 static const int kLuWideFrom = 3000;  // unknowns from which wide outer blocks pay (2102 complex: 45 ms with, 43 without)
 
+// How close two pivot candidates of column k must be to count as a near tie.
+// Candidates by FP64 chains and by digits differ by at most 2^-48 of the pivot in
+// column 64, 2^-46 in 512, 2^-43 in 1024 and 2^-40 in 2048 (PEEC boxes and plates of
+// 2102 to 3668 unknowns from 1 Hz to 100 MHz; random matrices 2^-39 in 3000), and
+// the closest candidates there are at least 100 times that apart but on meshes
+// whose symmetry makes them tie.
+static double near_tie_fraction(int k) { return 0x1p-45 + (double)k * k * 0x1p-63; }
+
 template <class T>
 static bool factor_device(T *d_a, int n, double limit, long long *d_piv, Status *d_st, LuMode mode) {
     LuTiming &tm = g_lu_timing;
@@ -2411,7 +2418,7 @@ static bool factor_device(T *d_a, int n, double limit, long long *d_piv, Status 
     auto rows_of_u = [&](int k0, int kb, int c0, int c1) {
         PEEC_LAUNCH(k_trsm<T>, (c1 - c0 + 63) / 64, 64, 0, d_a, n, k0, kb, c0, c1, d_st);
     };
-    auto panel = [&](int k0, int kb, long long tie) -> bool {
+    auto panel = [&](int k0, int kb, double tie) -> bool {
         CoopPlan<T> pl = coop_plan<T>(n - k0);
         const int lean_g = lean64_panel_ctas<T>(n - k0);
         if (lean_g > 0) {
@@ -2445,7 +2452,7 @@ static bool factor_device(T *d_a, int n, double limit, long long *d_piv, Status 
         for (int k0 = 0; k0 < n; k0 += NB) {
             const int kb = std::min(NB, n - k0), r1 = k0 + kb, rest = n - r1;
             tm.mark(2);
-            if (!panel(k0, kb, 0)) return false;
+            if (!panel(k0, kb, 0.0)) return false;
             tm.mark(0);
             swaps(k0, kb);
             if (rest > 0) rows_of_u(k0, kb, r1, n);
@@ -2490,7 +2497,7 @@ static bool factor_device(T *d_a, int n, double limit, long long *d_piv, Status 
             for (int b0 = K0; b0 < K1; b0 += 2 * NB) {
                 const int b1 = std::min(K1, b0 + 2 * NB);
                 // the first block's entries have seen chains only: the same in every mode
-                const long long tie = mode == LuMode::checked && b0 > 0 ? kTieUlps : 0;
+                const double tie = mode == LuMode::checked && b0 > 0 ? near_tie_fraction(b1) : 0.0;
                 tm.mark(2);
                 if (b0 > K0 && !update(K0, b0, b0, n, b0, b1)) return false;
                 for (int k0 = b0; k0 < b1; k0 += NB) {
@@ -3161,7 +3168,7 @@ extern "C" int peec_gb300_lu_factor_device_noalloc(double *d_a, size_t n, double
         int kb = std::min(NB, ni - k0);
         CoopPlan<double> pl = coop_plan<double>(ni - k0);
         if (pl.G > 0) {
-            long long no_tie = 0;
+            double no_tie = 0.0;
             int rows = pl.rows;
             double *cr = (double *)sc.cand_row, *kr = (double *)sc.krow;
             void *args[] = {&d_a, (void *)&ni, (void *)&k0, &kb, &rows, &limit, &d_piv, &st, &sc.ps, &sc.cand_val,
@@ -3172,7 +3179,7 @@ extern "C" int peec_gb300_lu_factor_device_noalloc(double *d_a, size_t n, double
                 return -1;
             note_launch();
         } else {
-            PEEC_LAUNCH(k_panel<double>, 1, 1024, 0, d_a, ni, k0, kb, limit, d_piv, st, 0LL);
+            PEEC_LAUNCH(k_panel<double>, 1, 1024, 0, d_a, ni, k0, kb, limit, d_piv, st, 0.0);
         }
         PEEC_LAUNCH(k_laswp<double>, (ni + kLaswpCols - 1) / kLaswpCols, 256, 2 * NB * kLaswpCols * sizeof(double), d_a,
                     ni, k0, kb, d_piv, st);
@@ -4006,7 +4013,7 @@ int mixed_solve_impl(const Complex *d_Z, size_t n_, const Complex *d_b, Complex 
                         return -1;
                     note_launch();
                 } else if (pl.G > 0) {
-                    long long no_tie = 0;
+                    double no_tie = 0.0;
                     int rows = pl.rows;
                     cplxf *cr = (cplxf *)sc.cand_row, *kr = (cplxf *)sc.krow;
                     Status *stp = st.p;
@@ -4020,7 +4027,7 @@ int mixed_solve_impl(const Complex *d_Z, size_t n_, const Complex *d_b, Complex 
                         return -1;
                     note_launch();
                 } else {
-                    PEEC_LAUNCH(k_panel<cplxf>, 1, 1024, 0, a, n, k0, kb, limit, piv.p, st.p, 0LL);
+                    PEEC_LAUNCH(k_panel<cplxf>, 1, 1024, 0, a, n, k0, kb, limit, piv.p, st.p, 0.0);
                 }
                 tm.mark(0);
                 pdl_launch(k_laswp<cplxf>, dim3((n + kLaswpCols - 1) / kLaswpCols), dim3(256),
