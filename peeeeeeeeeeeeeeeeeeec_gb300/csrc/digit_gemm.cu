@@ -392,13 +392,13 @@ __device__ __forceinline__ int integer(float x) {
     return (__float_as_int(t) - 0x4B400000) * 2048 + (__float_as_int(r + M) - 0x4B400000);
 }
 
-// v 2^E and the kUnit - 62 low bits of `low` below it, as FP64 bits: rounded once
+// v 2^E and `low` (kUnit - 61 bits) below it, as FP64 bits: rounded once
 // to 53 bits by integer operations (an FP64 conversion takes one of GB300's two
 // FP64 slots per clock and SM).  No branches: eight of these run interleaved.
 // Results below 2^-1022 are zero.
 __device__ __forceinline__ long long compose(long long v, unsigned low, int E) {
     const unsigned sign = (unsigned)((int)(v >> 32) >> 31);
-    constexpr int bits = kUnit - 62;
+    constexpr int bits = kUnit - 61;
     low = ((low ^ sign) & ((1u << bits) - 1u)) - sign;  // negated: ~x + 1 over both words
     const unsigned long long a = ((unsigned long long)v ^ ((unsigned long long)sign << 32 | sign)) + (low >> bits);
     unsigned hi = (unsigned)(a >> 32), lo = (unsigned)a;
@@ -421,14 +421,20 @@ __device__ __forceinline__ long long compose(long long v, unsigned low, int E) {
     return (long long)((unsigned long long)(rh | (sign & 0x80000000u)) << 32 | rl);
 }
 
-// 16 words of this warp's 32 TMEM lanes out and 4 back
-__device__ __forceinline__ void tmem_st16(uint32_t taddr, const int *v) {
+// 8 consecutive FP32 columns of this warp's 32 TMEM lanes
+__device__ __forceinline__ void tmem_ld8(uint32_t taddr, float *v) {
     asm volatile(
-        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};" ::"r"(
-            taddr),
-        "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]), "r"(v[9]),
-        "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15])
+        "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];\n"
+        "tcgen05.wait::ld.sync.aligned;"
+        : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7])
+        : "r"(taddr)
         : "memory");
+}
+// 8 words of this warp's 32 TMEM lanes out and 4 back
+__device__ __forceinline__ void tmem_st8(uint32_t taddr, const int *v) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"r"(taddr), "r"(v[0]),
+                 "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7])
+                 : "memory");
 }
 __device__ __forceinline__ void tmem_ld4(uint32_t taddr, int *v) {
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];"
@@ -455,9 +461,9 @@ struct Args {
 };
 
 static const int kExactBelow = 25;  // entries below 2^-25 of |row| |column| take the FP64 way
-// |v| 2^-62 below 2^-kExactBelow
+// |v| 2^-61 below 2^-kExactBelow
 __device__ __forceinline__ bool below(long long v) {
-    return (unsigned)((int)(v >> 32) + (1 << (30 - kExactBelow))) < (2u << (30 - kExactBelow));
+    return (unsigned)((int)(v >> 32) + (1 << (29 - kExactBelow))) < (2u << (29 - kExactBelow));
 }
 // |z| below 2^(E - kExactBelow)
 __device__ __forceinline__ bool below(double z, int E) {
@@ -534,25 +540,23 @@ __device__ __forceinline__ void copy_commit() { asm volatile("cp.async.commit_gr
 __device__ __forceinline__ void copy_wait1() { asm volatile("cp.async.wait_group 1;" ::: "memory"); }
 
 
-// Passes of a tile over K: four sums i + j each (the last one what is left),
-// from the leading ones on, within a pass from the highest i + j down; the s-th
-// sum of a pass is in accumulator s, 96 TMEM columns.  The 96 columns after the
-// accumulators hold the epilogue's third word.
+// Passes of a tile over K: i + j = 13 .. 10, 9 .. 6, 5 .. 2, within a pass from the
+// highest i + j down; the s-th sum of a pass is in accumulator s, 96 TMEM columns.
+// The longest pass (42 pairs) comes first: it runs while the warps of the
+// epilogue are busy with C of the tile before (with the leading sums first,
+// 10 pairs, the MMAs then waited: 189k instead of 150k cycles a tile at K = 192).
+// The 96 columns after the accumulators hold the epilogue's low words.
 static const int kSlots = 4;
 static const int kSlotCols = 96;
-static const int kPasses = (kDigits + kSlots - 1) / kSlots;
-__host__ __device__ constexpr int pass_top(int pass) { return (pass + 1) * kSlots + 1 < kDigits + 1 ? (pass + 1) * kSlots + 1 : kDigits + 1; }
-__host__ __device__ constexpr int pass_sums(int pass) { return pass_top(pass) - pass * kSlots - 1; }
+static const int kPasses = kDigits / kSlots;
+static_assert(kDigits == kSlots * kPasses, "sums");
+__host__ __device__ constexpr int pass_top(int pass) { return kDigits + 1 - kSlots * pass; }
 __host__ __device__ constexpr int pass_digits(int pass) { return pass_top(pass) - 1; }
-// uses of accumulator s before pass `pass` of this CTA's tile number `tile`
-__device__ __forceinline__ uint32_t slot_use(int pass, int s, int tile) {
-    return (uint32_t)((s < pass_sums(kPasses - 1) ? kPasses : kPasses - 1) * tile + pass);
-}
 // A pass's digits (1-based) in the order in which a block's products are done
 // with them, which is the order of their loads: top - 1, top - 2, ... (one for each
 // sum but the last), then 1, n, 2, n - 1, ... of the rest.
 __host__ __device__ constexpr int digit_order(int pass, int digit) {
-    const int first = pass_sums(pass) - 1, d = pass_digits(pass), rest = d - first;
+    const int first = kSlots - 1, d = pass_digits(pass), rest = d - first;
     return digit > rest ? d - digit : first + (digit <= rest + 1 - digit ? 2 * (digit - 1) : 2 * (rest - digit) + 1);
 }
 __host__ __device__ constexpr int digit_at(int pass, int order) {
@@ -590,7 +594,7 @@ __device__ __forceinline__ bool issue_block(uint32_t base_addr, uint32_t tmem, i
                                             uint64_t *sum_empty, volatile int *abort_flag) {
     typedef Shape<CX> S;
     constexpr uint32_t idesc = tc::idesc_bf16_f32(kBM, kSlotCols);
-    constexpr int top = pass_top(PASS), bottom = top - pass_sums(PASS) + 1;
+    constexpr int top = pass_top(PASS), bottom = top - kSlots + 1;
     const uint64_t desc0 = smem_desc_sw32(base_addr);
     uint32_t at[pass_digits(PASS)];  // ring slot of each digit of the block
     uint32_t wrapped = 0;
@@ -610,9 +614,9 @@ __device__ __forceinline__ bool issue_block(uint32_t base_addr, uint32_t tmem, i
         if (g == (d + 1 > bottom ? d + 1 : bottom)) warp_commit(&empty[at[d - 1]]);
     };
 #pragma unroll
-    for (int s = 0; s < pass_sums(PASS); ++s) {
+    for (int s = 0; s < kSlots; ++s) {
         const int g = top - s;
-        const uint32_t use = slot_use(PASS, s, tile);
+        const uint32_t use = (uint32_t)(kPasses * tile + PASS);  // of this accumulator so far
         if (kc == 0) {
             if (use > 0 && !warp_wait(&sum_empty[s], (use - 1) & 1, abort_flag)) return false;
             fence_after_sync();
@@ -753,7 +757,7 @@ __global__ void __launch_bounds__(32 * (2 + kEpiWarps), 1) k_digit_gemm(Args A) 
         // two runs of 16 accumulator columns: Re and Im, or consecutive ones
         constexpr int o1 = CX ? 48 : 16;
         const uint32_t tb = tmem + ((uint32_t)(32 * q) << 16) + (uint32_t)(h * (CX ? 16 : 32));
-        const uint32_t ts = tmem + ((uint32_t)(32 * q) << 16) + (uint32_t)(kSlots * kSlotCols + h * 32);  // third words
+        const uint32_t ts = tmem + ((uint32_t)(32 * q) << 16) + (uint32_t)(kSlots * kSlotCols + h * 32);  // low words
         unsigned char *mine = stage + (size_t)(warp - 2) * 2 * S::kChunkBytes;
         typedef typename S::Scalar Scalar;
         constexpr int RPI = 32 / S::kCols, kSteps = S::kCols;  // rows per warp access, accesses per chunk
@@ -780,54 +784,48 @@ __global__ void __launch_bounds__(32 * (2 + kEpiWarps), 1) k_digit_gemm(Args A) 
             };
             fetch(0);
             fetch(1);
-            const int er = A.ea[row0 + lane];
-            const int ec = A.eb[col0 + lane % S::kWarpCols];
-            // Sums of i + j <= 9 in units of 2^-61; then the sum in units of 2^-30 goes to
-            // TMEM and its low 64 bits (modulo 2^64) in units of 2^-kUnit stay: what is
-            // still added is below 2^-30.
+            // Sums of i + j >= 10 in units of 2^-kUnit; their bits below 2^-61 go to
+            // TMEM, the rest is summed in units of 2^-61 with the others.
             long long run[32];
 #pragma unroll
             for (int c = 0; c < 32; ++c) run[c] = 0;
 #pragma unroll 1
-            for (int g = pass_top(0), pass = 0, s = 0; pass < kPasses;) {
-                ok = warp_wait(&sum_full[s], slot_use(pass, s, tile) & 1, abort_flag);
+            for (int g = kDigits + 1; g >= 2; --g) {
+                const int pass = (kDigits + 1 - g) / kSlots, s = (kDigits + 1 - g) % kSlots;
+                ok = warp_wait(&sum_full[s], (uint32_t)(kPasses * tile + pass) & 1, abort_flag);
                 if (!ok) goto leave;
                 fence_after_sync();
                 const int shift = 7 * ((g <= 9 ? 9 : kDigits + 1) - g);  // 0 .. 49, never 31
                 const int m_lo = shift < 32 ? 1 << shift : 0, m_hi = shift < 32 ? 0 : 1 << (shift - 32);
 #pragma unroll
-                for (int p = 0; p < 2; ++p) {
-                    float v[16];
-                    tc::tmem_ld16(tb + (uint32_t)(s * kSlotCols + p * o1), v);
+                for (int p = 0; p < 4; ++p) {
+                    float v[8];
+                    tmem_ld8(tb + (uint32_t)(s * kSlotCols + (p >> 1) * o1 + (p & 1) * 8), v);
 #pragma unroll
-                    for (int c = 0; c < 16; ++c) {
+                    for (int c = 0; c < 8; ++c) {
                         const int x = integer(v[c]);
-                        run[16 * p + c] += (long long)x * m_lo + (long long)((unsigned long long)((unsigned)x * (unsigned)m_hi) << 32);
+                        run[8 * p + c] += (long long)x * m_lo + (long long)((unsigned long long)((unsigned)x * (unsigned)m_hi) << 32);
                     }
                 }
                 fence_before_sync();
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&sum_empty[s]);
-                if (g == 6) {  // the last of the leading sums
+                if (g == 10) {
 #pragma unroll
-                    for (int p = 0; p < 2; ++p) {
-                        int top[16];
+                    for (int p = 0; p < 4; ++p) {
+                        int low[8];
 #pragma unroll
-                        for (int c = 0; c < 16; ++c) {
-                            top[c] = (int)(run[16 * p + c] >> 31);
-                            run[16 * p + c] <<= kUnit - 61;
+                        for (int c = 0; c < 8; ++c) {
+                            low[c] = (int)((unsigned)run[8 * p + c] & ((1u << (kUnit - 61)) - 1u));
+                            run[8 * p + c] >>= kUnit - 61;
                         }
-                        tmem_st16(ts + 16 * p, top);
+                        tmem_st8(ts + 8 * p, low);
                     }
-                }
-                --g;
-                if (++s == pass_sums(pass)) {
-                    s = 0;
-                    ++pass;
-                    g = pass_top(pass);
                 }
             }
             tmem_wait_st();
+            const int er = A.ea[row0 + lane];
+            const int ec = A.eb[col0 + lane % S::kWarpCols];
             // C -= sums 2^(row exponent + column exponent), a chunk at a time
             unsigned exact = 0;  // columns of this lane's row left to FP64
 #pragma unroll
@@ -835,30 +833,22 @@ __global__ void __launch_bounds__(32 * (2 + kEpiWarps), 1) k_digit_gemm(Args A) 
                 unsigned char *buf = mine + (ch & 1) * S::kChunkBytes;
                 copy_wait1();
                 __syncwarp();
-                int top[8];
-                tmem_ld4(ts + (CX ? ch * 4 : ch * 8), top);
-                tmem_ld4(ts + (CX ? 16 + ch * 4 : ch * 8 + 4), top + 4);
-                tmem_wait_ld(top, top + 4);
-                // the whole sum in units of 2^-62; the bits below stay in r
-                auto upper = [&](long long r, int t) {
-                    constexpr int top = 94 - kUnit;  // bits of r above 2^-30: t modulo 2^top and a carry from below
-                    const int d = (int)((unsigned)(r >> 32) - ((unsigned)t << (32 - top))) >> (32 - top);
-                    return (long long)(t + d) * (1ll << 32) | (long long)((unsigned long long)r << top >> 32);
-                };
+                int low[8];
+                tmem_ld4(ts + (CX ? ch * 4 : ch * 8), low);
+                tmem_ld4(ts + (CX ? 16 + ch * 4 : ch * 8 + 4), low + 4);
+                tmem_wait_ld(low, low + 4);
                 Scalar *p = reinterpret_cast<Scalar *>(buf + lane * S::kRowStride);
                 double w[8];            // re, im of four columns, or eight columns
                 unsigned small = 0u;    // columns whose update is below the limit
 #pragma unroll
                 for (int c = 0; c < S::kCols; ++c) {
                     const int col = ch * S::kCols + c;  // 0..15 (complex), 0..31 (real)
-                    const int E = er + __shfl_sync(0xffffffffu, ec, col) - 62;
-                    const long long u = upper(run[col], top[c]);
-                    bool sm = below(u);
-                    w[c] = __longlong_as_double(compose(u, (unsigned)run[col], E));
+                    const int E = er + __shfl_sync(0xffffffffu, ec, col) - 61;
+                    bool sm = below(run[col]);
+                    w[c] = __longlong_as_double(compose(run[col], (unsigned)low[c], E));
                     if constexpr (CX) {
-                        const long long v = upper(run[16 + col], top[4 + c]);
-                        sm = sm && below(v);
-                        w[4 + c] = __longlong_as_double(compose(v, (unsigned)run[16 + col], E));
+                        sm = sm && below(run[16 + col]);
+                        w[4 + c] = __longlong_as_double(compose(run[16 + col], (unsigned)low[4 + c], E));
                     }
                     small |= sm ? 1u << c : 0u;
                 }

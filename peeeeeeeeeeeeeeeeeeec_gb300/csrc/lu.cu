@@ -162,6 +162,7 @@ __global__ void __launch_bounds__(1024) k_panel(T *a, int n, int k0, int kb, dou
     __shared__ T s_row[NB];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nthr = blockDim.x;
     if (st->code != 0) return;
+    const bool checked = __double_as_longlong(tie) != 0;  // (an FP64 comparison would cost 64 cycles a column)
     for (int kk = 0; kk < kb; ++kk) {
         const int k = k0 + kk;
         // argmax |a[i][k]|, i >= k; ties -> lowest row; NaN below the diagonal
@@ -221,7 +222,7 @@ __global__ void __launch_bounds__(1024) k_panel(T *a, int n, int k0, int kb, dou
         __syncthreads();
         if (s_fail) return;
         const int p = s_pivot;
-        const long long tie_at = tie_limit(s_val[0], tie);
+        const long long tie_at = checked ? tie_limit(s_val[0], tie) : 0;
         if (p != k) {
             for (int j = k0 + tid; j < k0 + kb; j += nthr) {
                 T t = a[(size_t)k * n + j];
@@ -237,7 +238,7 @@ __global__ void __launch_bounds__(1024) k_panel(T *a, int n, int k0, int kb, dou
         for (int i = k + 1 + tid; i < n; i += nthr) {
             T *row = a + (size_t)i * n + k0;
             if constexpr (!std::is_same<T, cplxf>::value)
-                if (tie > 0.0 && near_tie_of(row[kk], tie_at)) atomicCAS(&st->code, 0, 7);
+                if (checked && near_tie_of(row[kk], tie_at)) atomicCAS(&st->code, 0, 7);
             T m = divide(row[kk], pivot);
             row[kk] = m;
             for (int j = kk + 1; j < kb; ++j) row[j] = msub(row[j], m, s_row[j]);
@@ -346,6 +347,7 @@ __global__ void __launch_bounds__(256) k_panel_coop(T *a, int n, int k0, int kb,
     const int r0 = k0 + c * rows_per_cta, r1 = min(n, r0 + rows_per_cta);
     const int nrows = r1 > r0 ? r1 - r0 : 0;
     if (st->code != 0) return;  // uniform across CTAs (set before launch)
+    const bool checked = __double_as_longlong(tie) != 0;  // (an FP64 comparison would cost 64 cycles a column)
     unsigned int gen = *(volatile unsigned int *)&ps->gen;  // stable between launches
     for (int t = tid; t < nrows * kb; t += blockDim.x) {
         int i = t / kb, j = t % kb;
@@ -463,7 +465,7 @@ __global__ void __launch_bounds__(256) k_panel_coop(T *a, int n, int k0, int kb,
         __syncthreads();
         if (s_fail) return;
         const int p = s_p, pc = s_pc;
-        const long long tie_at = tie_limit((double)s_val[0], tie);
+        const long long tie_at = checked ? tie_limit((double)s_val[0], tie) : 0;
         // the new row k is the published row p (full panel width: columns
         // < kk hold earlier multipliers and move with the row)
         const T *prow_g = cand_row + ((size_t)par * G + pc) * NB;
@@ -482,7 +484,7 @@ __global__ void __launch_bounds__(256) k_panel_coop(T *a, int n, int k0, int kb,
         for (int i = max(r0, k + 1) + tid; i < r1; i += blockDim.x) {
             T *row = tile + (i - r0) * kPS;
             if constexpr (!std::is_same<T, cplxf>::value)
-                if (tie > 0.0 && near_tie_of(row[kk], tie_at)) atomicCAS(&st->code, 0, 7);
+                if (checked && near_tie_of(row[kk], tie_at)) atomicCAS(&st->code, 0, 7);
             T m = divide(row[kk], pivot);
             row[kk] = m;
             for (int j = kk + 1; j < kb; ++j) row[j] = msub(row[j], m, s_prow[j]);
@@ -787,6 +789,7 @@ __global__ void __launch_bounds__(kLeanThreads) k_panel_lean64(T *a, int n, int 
     const int r0 = k0 + c * kLeanThreads, r1 = min(n, r0 + kLeanThreads);
     const int nrows = r1 > r0 ? r1 - r0 : 0;
     if (st->code != 0) return;  // uniform across CTAs (set before launch)
+    const bool checked = __double_as_longlong(tie) != 0;  // (an FP64 comparison would cost 64 cycles a column)
     const unsigned gen0 = *(volatile unsigned *)&ps->gen;
     for (int t = tid; t < nrows * kb; t += kLeanThreads) {
         const int ii = t / kb, j = t % kb;
@@ -935,7 +938,7 @@ __global__ void __launch_bounds__(kLeanThreads) k_panel_lean64(T *a, int n, int 
         const int p = s_p;
         // (mv still is this row's candidate; every CTA has passed the status
         // check at the top: the flags of this column were all published)
-        if (tie > 0.0 && mine && i >= k && i != p && near_tie(mv, tie_limit(gb, tie))) atomicCAS(&st->code, 0, 7);
+        if (checked && mine && i >= k && i != p && near_tie(mv, tie_limit(gb, tie))) atomicCAS(&st->code, 0, 7);
         if (p != k) {
             if (warp == 0 && k >= r0 && k < r1 && lane < kb) tile[k - r0][lane] = pcur[lane];
             if (warp == 1 && gc == c && lane < kb) tile[p - r0][lane] = kval;
@@ -1347,6 +1350,60 @@ __global__ void __launch_bounds__(256) k_trsm(T *a, int n, int k0, int kb, int c
 #pragma unroll
     for (int i = 0; i < NB; ++i)
         if (i < kb) a[(size_t)(k0 + i) * n + j] = x[i];
+}
+
+// The same for the FP64 factorisations, ROWS = 32 or 64 rows of a block at once:
+// 32 columns per CTA, one per lane, the rows dealt to its eight warps (row i to
+// warp i % 8), so that every scheduler's FP64 unit has work: with one thread a
+// column, 64 a CTA, half of them idled (8402 columns, 64 rows complex: 76 us each
+// of the two 32-row solves and 69 us for the product between them).  Each row
+// takes its predecessors in increasing order, as k_trsm.
+static const int kRowsWarps = 8;
+template <class T, int ROWS>
+static constexpr size_t rows_of_u_smem() {
+    return (size_t)ROWS * (ROWS + 1) * sizeof(T) + (size_t)2 * 32 * sizeof(T);
+}
+template <class T, int ROWS>
+__global__ void __launch_bounds__(32 * kRowsWarps) k_rows_of_u(T *a, int n, int k0, int kb, int c0, int c1,
+                                                               const Status *st) {
+    extern __shared__ __align__(16) unsigned char rows_smem[];
+    T *L = reinterpret_cast<T *>(rows_smem);  // [ROWS][ROWS + 1]
+    T *xs = L + ROWS * (ROWS + 1);            // [2][32]: the solved row, by parity
+    if (st->code != 0) return;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int j = c0 + blockIdx.x * 32 + lane;
+    constexpr int R = ROWS / kRowsWarps;
+    T x[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        const int i = r * kRowsWarps + warp;
+        x[r] = (i < kb && j < c1) ? a[(size_t)(k0 + i) * n + j] : T{};
+    }
+    for (int t = threadIdx.x; t < kb * kb; t += blockDim.x) {
+        const int i = t / kb, m = t % kb;
+        L[i * (ROWS + 1) + m] = a[(size_t)(k0 + i) * n + k0 + m];
+    }
+    __syncthreads();
+#pragma unroll
+    for (int rm = 0; rm < R; ++rm)
+#pragma unroll 2
+        for (int w = 0; w < kRowsWarps; ++w) {
+            const int m = rm * kRowsWarps + w;  // the row that is solved next
+            if (m + 1 >= kb) break;             // uniform: no row left below
+            T *s = xs + (m & 1) * 32;
+            if (warp == w) s[lane] = x[rm];
+            __syncthreads();
+            const T xm = s[lane];
+            if (warp > w) x[rm] = msub(x[rm], L[m / kRowsWarps * kRowsWarps * (ROWS + 1) + warp * (ROWS + 1) + m], xm);
+#pragma unroll
+            for (int r = rm + 1; r < R; ++r)
+                x[r] = msub(x[r], L[(r * kRowsWarps + warp) * (ROWS + 1) + m], xm);
+        }
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        const int i = r * kRowsWarps + warp;
+        if (i < kb && j < c1) a[(size_t)(k0 + i) * n + j] = x[r];
+    }
 }
 
 // ---- C -= L U on a rectangle, FP64 pipe -------------------------------
@@ -2360,15 +2417,16 @@ enum class LuMode {
     digits,   // digit GEMMs
     checked,  // digit GEMMs, stopping with status 7 at a near tie of two pivot candidates
 };
-// Unknowns from which digit GEMMs are the faster form (LU of random matrices on
-// GB300, chains / digits in ms: complex 1000: 19.2 / 20.1, 1200: 24.1 / 24.3, 2102:
-// 58.7 / 43.0, 4000: 212 / 97, 8402: 1436 / 285; real 2102: 21.7 / 19.9, 4000: 65.9 / 48,
-// 8402: 386 / 126).  A checked run may have to be done again by chains (real
-// systems of regular meshes nearly always tie), so real ones start later.
+// Unknowns from which digit GEMMs are used (LU of random matrices on GB300,
+// chains / digits in ms: complex 1000: 17.6 / 16.7, 1200: 22.2 / 20.2, 1400: 27.7 /
+// 23.6, 2102: 52.6 / 36.0, 4000: 199 / 86, 8402: 1436 / 248; real 1500: 14.2 / 12.9,
+// 2102: 22.4 / 19.4, 4000: 66.0 / 44.3, 8402: 386 / 111).  A checked run may have to
+// be done again by chains, so the lines lie somewhat above the crossings (and
+// well above for real systems: those of regular meshes nearly always tie).
 static const int kDigitsFromCplx = 1300;
 static const int kDigitsFromReal = 2000;
 static const int kCheckedFromReal = 5000;
-static const int kLuWideFrom = 3000;  // unknowns from which wide outer blocks pay (2102 complex: 45 ms with, 43 without)
+static const int kLuWideFrom = 3000;  // unknowns from which wide outer blocks pay (2102 complex: 45 ms with, 43 without, before the rows of U were solved in one kernel)
 
 // How close two pivot candidates of column k must be to count as a near tie.
 // Candidates by FP64 chains and by digits differ by at most 2^-48 of the pivot in
@@ -2415,8 +2473,18 @@ static bool factor_device(T *d_a, int n, double limit, long long *d_piv, Status 
         PEEC_LAUNCH(k_laswp<T>, (n + kLaswpCols - 1) / kLaswpCols, 256, 2 * NB * kLaswpCols * sizeof(T), d_a, n, k0, kb,
                     d_piv, d_st);
     };
+    // rows k0 .. k0+kb-1 (kb <= 64) of U, columns c0 .. c1-1
+    static const cudaError_t attr = cudaFuncSetAttribute(k_rows_of_u<T, 64>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                         (int)rows_of_u_smem<T, 64>());
+    if (!cuda_ok(attr, "LU shared memory")) return false;
     auto rows_of_u = [&](int k0, int kb, int c0, int c1) {
-        PEEC_LAUNCH(k_trsm<T>, (c1 - c0 + 63) / 64, 64, 0, d_a, n, k0, kb, c0, c1, d_st);
+        const unsigned grid = (unsigned)(c1 - c0 + 31) / 32;
+        if (kb > NB)
+            PEEC_LAUNCH((k_rows_of_u<T, 64>), grid, 32 * kRowsWarps, (rows_of_u_smem<T, 64>()), d_a, n, k0, kb, c0, c1,
+                        d_st);
+        else
+            PEEC_LAUNCH((k_rows_of_u<T, 32>), grid, 32 * kRowsWarps, (rows_of_u_smem<T, 32>()), d_a, n, k0, kb, c0, c1,
+                        d_st);
     };
     auto panel = [&](int k0, int kb, double tie) -> bool {
         CoopPlan<T> pl = coop_plan<T>(n - k0);
@@ -2472,7 +2540,7 @@ static bool factor_device(T *d_a, int n, double limit, long long *d_piv, Status 
         // them: the panels' swaps bring rows from below that lack it too); per
         // outer block, the trailing update with K = W.  A digit GEMM's tile
         // costs an integer epilogue per entry whatever K is (m = n = 4000
-        // complex: 702 us with K = 64, 1350 us with 192), so W is its largest K;
+        // complex: 764 us with K = 64, 1730 us with 192), so W is its largest K;
         // small systems, where launches count, take one inner block.
         const int W = n < kLuWideFrom ? 2 * NB : cx ? kDigitMaxKCplx : kDigitMaxKReal;
         DigitScratch digits;
@@ -2508,7 +2576,9 @@ static bool factor_device(T *d_a, int n, double limit, long long *d_piv, Status 
                     swaps(k0, kb);
                     if (r1 < b1) {  // the block's second panel
                         rows_of_u(k0, kb, r1, b1);
-                        PEEC_LAUNCH((k_gemm_rect<T, 64, 32>), dim3((b1 - r1 + 31) / 32, (n - r1 + 63) / 64), 256, 0,
+                        // 16-row tiles: with 64-row ones each of at most 131 CTAs kept
+                        // its SM's FP64 unit busy for 63 us, however few there were
+                        PEEC_LAUNCH((k_gemm_rect<T, 16, 32>), dim3((b1 - r1 + 31) / 32, (n - r1 + 15) / 16), 256, 0,
                                     d_a, n, k0, kb, r1, n, r1, b1, d_st);
                     }
                     tm.mark(1);
@@ -2517,10 +2587,7 @@ static bool factor_device(T *d_a, int n, double limit, long long *d_piv, Status 
                 // the block's rows to the right of it
                 if (b0 > K0 && !update(K0, b0, b0, b1, b1, n)) return false;
                 tm.mark(2);
-                rows_of_u(b0, NB, b1, n);
-                PEEC_LAUNCH((k_gemm_rect<T, 32, 64>), dim3((n - b1 + 63) / 64, 1), 256, 0, d_a, n, b0, NB, b0 + NB, b1,
-                            b1, n, d_st);
-                rows_of_u(b0 + NB, b1 - b0 - NB, b1, n);
+                rows_of_u(b0, b1 - b0, b1, n);
                 tm.mark(1);
             }
             if (K1 < n && !update(K0, K1, K1, n, K1, n)) return false;
@@ -3185,7 +3252,8 @@ extern "C" int peec_gb300_lu_factor_device_noalloc(double *d_a, size_t n, double
                     ni, k0, kb, d_piv, st);
         int rest = ni - (k0 + kb);
         if (rest > 0) {
-            PEEC_LAUNCH(k_trsm<double>, (rest + 255) / 256, 256, 0, d_a, ni, k0, kb, k0 + kb, ni, st);
+            PEEC_LAUNCH((k_rows_of_u<double, 32>), (rest + 31) / 32, 32 * kRowsWarps, (rows_of_u_smem<double, 32>()), d_a,
+                        ni, k0, kb, k0 + kb, ni, st);
             PEEC_LAUNCH((k_gemm_rect<double, 64, 64>), dim3((rest + 63) / 64, (rest + 63) / 64), 256, 0, d_a, ni, k0, kb,
                         k0 + kb, ni, k0 + kb, ni, st);
         }

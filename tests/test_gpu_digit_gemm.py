@@ -163,3 +163,14 @@ def test_tied_rows_give_the_oracles_pivots(gpu_lib, oracle):
     a[n // 2:, -1] = a[:n // 2, -1]
     _, piv, _, _ = factored(gpu_lib, a, True)
     assert np.array_equal(piv, oracle.complex_lu_factorize(a)[2].astype(np.int64))
+
+
+@pytest.mark.parametrize("n,cplx", [(n, c) for n in (33, 63, 95, 97) for c in (False, True)] + [(1313, True), (1345, True)])
+def test_ragged_columns_right_of_a_block(gpu_lib, n, cplx):
+    """Rows of U are solved in tiles of 32 columns, 32 rows at once in small
+    systems and 64 in large ones: last tiles of 1, 31 and 33 columns."""
+    a = matrix(n, cplx, "normal")
+    lu, piv, rs, cs = factored(gpu_lib, a, cplx)
+    rows = sorted({0, 7, 8, 31, 32, 63, n // 2, n - 1} & set(range(n)))
+    bound = (2 * math.sqrt(2) * n + 4) * U if cplx else n * U / (1 - n * U)
+    assert backward_error(a, lu, piv, rs, cs, cplx, rows) <= bound
