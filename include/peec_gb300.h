@@ -82,9 +82,10 @@ int peec_gb300_potential_device(const Mesh *mesh, const DualMesh *dual,
  * Returns the previous mode.  Not thread-safe against concurrent assemblies. */
 int peec_gb300_set_far_precision(int mode);
 
-/* Reuse of translated near pairs (default on): near patch pairs whose
+/* Reuse of translated copies (default on): near patch pairs whose
  * corners are translated copies of each other (to a few ulps of the largest
- * coordinate) share one adaptive evaluation.  Returns the previous setting. */
+ * coordinate) share one adaptive evaluation, and so do matrix entries without
+ * near pairs one double-float far sum.  Returns the previous setting. */
 int peec_gb300_set_near_reuse(int on);
 
 /* ---- dense factorisations of device-resident matrices (in place) ----
