@@ -13,9 +13,10 @@
 //   3. k_near_scan       per patch i: every partner j of the upper triangle
 //                        whose class is not FAR (counted, scanned, filled:
 //                        a deterministic, i-major, j-sorted list)
-//   4. k_near_eval       one warp per (near pair, triangle pair, direction):
-//                        adaptive outer Gauss rule over the analytic inner
-//                        potential, depth-first with an explicit stack
+//   4. k_level_tree      adaptive outer Gauss rule over the analytic inner
+//                        potential for every (near pair, triangle pair,
+//                        direction), all trees level by level (k_near_eval:
+//                        one warp each, depth-first with an explicit stack)
 //   5. k_near_finalize   per near pair: the 4 triangle-pair values combined in
 //                        the reference's order (both orientations)
 //   6. k_entry_list      the entries of the upper triangle that are evaluated;
@@ -28,6 +29,7 @@
 //      k_entry_scale     every entry's factor; tiles and their mirrors are
 //                        written with coalesced row stores
 // Everything is FP64, or double-float in the far rule.
+#include <cooperative_groups.h>
 #include <math.h>
 #include <stdlib.h>
 #include <string.h>
@@ -288,47 +290,59 @@ __device__ void tri_prepare(const double *v, TriPot &t) {
     }
 }
 
+__device__ __forceinline__ double dot3_fma(const double *a, const double *b) {
+    return fma(a[2], b[2], fma(a[1], b[1], a[0] * b[0]));
+}
+
 // \int_T 1/|r - r0| dS exactly: sum over edges of d_e * (asinh terms) minus
 // |h * solid angle| (van Oosterom's uniform-layer formula, as the reference).
+// Bound by the FP64 pipe (a warp instruction takes 64 cycles of its scheduler), so
+// the instructions count: fused dot products and one division an edge instead of
+// three.
 __device__ double tri_potential(const TriPot &t, const double *r) {
-    double v[3][3], rad[3];
-    for (int i = 0; i < 3; ++i) {
+    double v[3][3];
+    for (int i = 0; i < 3; ++i)
         for (int k = 0; k < 3; ++k) v[i][k] = t.p[i][k] - r[k];
-        rad[i] = norm3(v[i]);
-    }
-    double h = dot3(v[0], t.nrm);
+    const double h = dot3_fma(v[0], t.nrm), h2 = h * h;
     double acc = 0.0;
     for (int i = 0; i < 3; ++i) {
-        double d = dot3(v[i], t.outw[i]);
+        const double d = dot3_fma(v[i], t.outw[i]);
         if (d == 0.0) continue;  // finite limit d log(.) = 0, as the reference
         // Edge integral asinh((s+L)/q) - asinh(s/q), q = hypot(d, h), as
         // log(A2/A1) with A = s + sqrt(s^2 + q^2) (= q e^asinh(s/q)); for
         // s < 0 the equal form q^2 / (sqrt(s^2 + q^2) - s) avoids the
         // cancellation.  The square roots use the same s and q as the
         // asinh arguments (not the vertex distances, which disagree by
-        // rounding when the point lies on the edge's line).  One log and two
-        // square roots instead of two asinh and a hypot.
-        double s = dot3(v[i], t.unit[i]);
-        double s2 = s + t.len[i];
-        double q2 = d * d + h * h;
+        // rounding when the point lies on the edge's line).  One log, one
+        // division (s < s2, so q^2 appears at most once) and two square roots
+        // instead of two asinh and a hypot.
+        const double s = dot3_fma(v[i], t.unit[i]);
+        const double s2 = s + t.len[i];
+        const double q2 = fma(d, d, h2);
         double e;
         if (q2 > 1e-280) {
-            double r1 = sqrt(fma(s, s, q2)), r2 = sqrt(fma(s2, s2, q2));
-            double a1 = s >= 0.0 ? s + r1 : q2 / (r1 - s);
-            double a2 = s2 >= 0.0 ? s2 + r2 : q2 / (r2 - s2);
-            e = log(a2 / a1);
+            const double r1 = sqrt(fma(s, s, q2)), r2 = sqrt(fma(s2, s2, q2));
+            const double b1 = fabs(s) + r1, b2 = fabs(s2) + r2;  // A, or q^2 / A
+            double num = s2 >= 0.0 ? b2 : b1, den = s >= 0.0 ? b1 : b2;
+            if (s < 0.0 && s2 >= 0.0) {
+                num = b1 * b2;
+                den = q2;
+            }
+            e = log(num / den);
         } else {  // q^2 underflows: the reference's form
-            double q = hypot(d, h);
+            const double q = hypot(d, h);
             e = asinh(s2 / q) - asinh(s / q);
         }
-        acc += d * e;
+        acc = fma(d, e, acc);
     }
     if (h != 0.0) {
-        double c[3];
+        double rad[3], c[3];
+        for (int i = 0; i < 3; ++i) rad[i] = sqrt(dot3_fma(v[i], v[i]));
         cross3(v[1], v[2], c);
-        double den = rad[0] * rad[1] * rad[2] + dot3(v[0], v[1]) * rad[2] + dot3(v[1], v[2]) * rad[0] +
-                     dot3(v[2], v[0]) * rad[1];
-        double omega = 2.0 * atan2(dot3(v[0], c), den);
+        const double den = fma(rad[0] * rad[1], rad[2],
+                               fma(dot3_fma(v[0], v[1]), rad[2],
+                                   fma(dot3_fma(v[1], v[2]), rad[0], dot3_fma(v[2], v[0]) * rad[1])));
+        const double omega = 2.0 * atan2(dot3_fma(v[0], c), den);
         acc -= fabs(h * omega);
     }
     return acc;
@@ -597,10 +611,10 @@ __global__ void k_near_finalize(int nrec, const double *slot, const int *kind, d
 // The depth-first warp above serialises a job's whole refinement tree, and a
 // few deep jobs (edge- and vertex-touching pairs refine towards the shared
 // edge to depth ~20) set the time of the launch.  Here the trees of all
-// jobs grow one level per launch: every node of the level is one warp (the
-// same low / high rules and decisions as the reference's recursion), accepted
-// nodes keep `high`, refined nodes append their two children to the next
-// level.  The value is then formed bottom-up exactly as the recursion returns
+// jobs grow level by level in one cooperative launch: every node of the level
+// is one CTA (the same low / high rules and decisions as the reference's
+// recursion), accepted nodes keep `high`, refined nodes append their two
+// children to the next level.  The value is then formed bottom-up exactly as the recursion returns
 // it, value(node) = value(left) + value(right) (quadrature.c:936-937), and a
 // top-down pass numbers the nodes in depth-first order to write the decision
 // trace the reuse replay reads.  The critical path is the tree depth
@@ -622,6 +636,7 @@ struct LevelNode {
     int size;   // nodes in the subtree
     int pos;    // depth-first position in the job's tree
     int edge;   // bisected edge of a refined node
+    double jac; // twice the area
 };
 
 struct LevelArgs {
@@ -637,14 +652,14 @@ struct LevelArgs {
     int *trace_len;
     LevelJob *jobs;        // [njob]
     LevelNode *pool;
-    int *count;            // nodes appended to the next level
+    int *count;            // [kLevels + 1] nodes of every level
     int *overflow;
     unsigned long long *evals;
 };
 
 // One thread per job: zero-area and identical-triangle jobs are finished
 // here (as in k_near_eval); adaptive jobs get their root node.
-__global__ void k_level_init(LevelArgs A, int base0, int cap) {
+__global__ void k_level_init(LevelArgs A, int cap) {
     long long g = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     if (g >= A.njob) return;
     const long long job = A.job0 + g;
@@ -691,13 +706,14 @@ __global__ void k_level_init(LevelArgs A, int base0, int cap) {
             if (at >= cap) {
                 atomicExch(A.overflow, 1);
             } else {
-                LevelNode &nd = A.pool[base0 + at];
+                LevelNode &nd = A.pool[at];
                 for (int k = 0; k < 9; ++k) nd.v[k] = outer[k];
                 nd.tol = 2e-5 * scale;
                 nd.job = (int)g;
                 nd.depth = 0;
                 nd.child = -1;
                 nd.pos = 0;
+                nd.jac = po.twice_area;
             }
         }
     }
@@ -705,140 +721,181 @@ __global__ void k_level_init(LevelArgs A, int base0, int cap) {
     if (kind != 0 && A.trace_len) A.trace_len[job] = 0;
 }
 
-// One warp per node of one level.
-__global__ void __launch_bounds__(256, 2) k_level_eval(LevelArgs A, int base, int n, int next_base, int cap) {
-    __shared__ TriPot s_inner[8];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const long long w = blockIdx.x * 8ll + warp;
-    if (w >= n) return;
-    LevelNode &nd = A.pool[base + w];
-    const LevelJob &J = A.jobs[nd.job];
-    TriPot &inner = s_inner[warp];
-    {
-        const double *src = reinterpret_cast<const double *>(&J.inner);
-        double *dst = reinterpret_cast<double *>(&inner);
-        for (int k = lane; k < (int)(sizeof(TriPot) / sizeof(double)); k += 32) dst[k] = src[k];
-    }
-    double v[9];
-    for (int k = 0; k < 9; ++k) v[k] = nd.v[k];
-    const double tol = nd.tol;
-    const int depth = nd.depth, order = J.order;
-    __syncwarp();
-    const int ql = order <= 6 ? 3 : 4;
-    const int rl = gl_row(ql), rh = gl_row(order);
-    const int nlo = ql * ql, ntot = nlo + order * order;
-    double lo = 0.0, hi = 0.0;
-    for (int k = lane; k < ntot; k += 32) {
-        int ord, row, idx;
-        if (k < nlo) {
-            ord = ql;
-            row = rl;
-            idx = k;
-        } else {
-            ord = order;
-            row = rh;
-            idx = k - nlo;
-        }
-        int i = idx / ord, j = idx % ord;
-        double xi = c_gl_x[row][i], xj = c_gl_x[row][j];
-        double wi = c_gl_w[row][i], wj = c_gl_w[row][j];
-        double r[3], jac;
-        tri_map(v, v + 3, v + 6, 0.5 * (xi + 1.0), 0.5 * (xj + 1.0), r, &jac);
-        double val = 0.25 * wi * wj * jac * tri_potential(inner, r);
-        if (k < nlo)
-            lo += val;
-        else
-            hi += val;
-    }
-    lo = warp_sum(lo);
-    hi = warp_sum(hi);
-    if (lane != 0) return;
-    atomicAdd(A.evals, (unsigned long long)ntot);
-    nd.child = -1;
-    if (!isfinite(lo) || !isfinite(hi)) {
-        nd.val = nan("");
-        return;
-    }
-    int mflags = 0;
-    double thr = tol + 2e-5 * fabs(hi), gap = fabs(hi - lo);
-    if (fabs(gap - thr) <= 1e-6 * thr) mflags |= MARG_THRESHOLD;
-    if (gap <= thr) {
-        nd.val = hi;
-    } else if (depth >= 24) {
-        nd.val = nan("");  // quadrature.c:922
-    } else {
-        int e = 0;
-        double longest = 0.0, len[3];
-        for (int i = 0; i < 3; ++i) {
-            double sl = dist3(v + 3 * i, v + 3 * ((i + 1) % 3));
-            len[i] = sl;
-            if (sl > longest) {
-                longest = sl;
-                e = i;
+// The trees of all jobs: level by level (barriers of the whole grid between), then
+// the values bottom-up and the depth-first numbers top-down.  A node's points (16 +
+// 144 at order 12) go to the five warps of one CTA: with one warp a node, eight a
+// CTA, and a launch for every level, a level of few nodes took 125 us whatever its
+// size (the five evaluations of a warp one after the other, two warps on each
+// scheduler's FP64 unit), and 30 us until the host had read its count.
+// Plate of 16 x 16 cells, both matrices: 7.7 ms in 65 levels and 10 ms with the gaps;
+// now 3.3 ms.  Box of 2 x 1 x 0.5 m at 5 cm: 28 + 3 ms, now 17.9 ms, bound by the
+// FP64 pipe (the large levels).
+static const int kLevels = 25;  // depth 0 .. 24
+static const int kTreeThreads = 160;
+static const int kMaxPoints = 16 * 16 + 4 * 4;
+
+__global__ void __launch_bounds__(kTreeThreads, 3) k_level_tree(LevelArgs A, int cap) {
+    namespace cg = cooperative_groups;
+    cg::grid_group grid = cg::this_grid();
+    __shared__ TriPot s_inner;
+    __shared__ double s_v[9];
+    __shared__ double s_u[kMaxPoints], s_eta[kMaxPoints], s_w[kMaxPoints], s_val[kMaxPoints];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    int have = 0, nlo = 0, ntot = 0;  // order of the table of points
+    unsigned long long evals = 0;
+    int lv = 0, base = 0, n = *(volatile int *)&A.count[0];
+    if (n > cap) return;  // overflow
+    while (n > 0) {
+        const int next_base = base + n;
+        for (int w = blockIdx.x; w < n; w += gridDim.x) {
+            LevelNode &nd = A.pool[base + w];
+            const LevelJob &J = A.jobs[nd.job];
+            const int order = J.order;
+            __syncthreads();  // the node before is done
+            for (int k = tid; k < (int)(sizeof(TriPot) / sizeof(double)); k += kTreeThreads)
+                reinterpret_cast<double *>(&s_inner)[k] = reinterpret_cast<const double *>(&J.inner)[k];
+            if (warp == 4 && lane < 9) s_v[lane] = nd.v[lane];
+            if (order != have) {
+                const int ql = order <= 6 ? 3 : 4;
+                nlo = ql * ql;
+                ntot = nlo + order * order;
+                for (int k = tid; k < ntot; k += kTreeThreads) {
+                    const int ord = k < nlo ? ql : order, row = gl_row(ord), idx = k < nlo ? k : k - nlo;
+                    const int i = idx / ord, j = idx % ord;
+                    const double u = 0.5 * (c_gl_x[row][i] + 1.0);
+                    s_u[k] = u;
+                    s_eta[k] = (1.0 - u) * (0.5 * (c_gl_x[row][j] + 1.0));
+                    s_w[k] = 0.25 * c_gl_w[row][i] * c_gl_w[row][j] * (1.0 - u);
+                }
+                have = order;
+            }
+            __syncthreads();
+            for (int k = tid; k < ntot; k += kTreeThreads) {
+                double r[3];
+#pragma unroll
+                for (int t = 0; t < 3; ++t)
+                    r[t] = fma(s_eta[k], s_v[6 + t] - s_v[t], fma(s_u[k], s_v[3 + t] - s_v[t], s_v[t]));
+                s_val[k] = s_w[k] * tri_potential(s_inner, r);
+            }
+            __syncthreads();
+            if (warp != 0) continue;
+            double lo = 0.0, hi = 0.0;
+            for (int k = lane; k < ntot; k += 32)
+                if (k < nlo)
+                    lo += s_val[k];
+                else
+                    hi += s_val[k];
+            const double jac = nd.jac;
+            lo = jac * warp_sum(lo);
+            hi = jac * warp_sum(hi);
+            evals += ntot;
+            int child = -1, e = 0;
+            double val = hi;
+            int mflags = 0;
+            const double tol = nd.tol, thr = tol + 2e-5 * fabs(hi), gap = fabs(hi - lo);
+            if (!isfinite(lo) || !isfinite(hi)) {
+                val = nan("");
+            } else {
+                if (fabs(gap - thr) <= 1e-6 * thr) mflags |= MARG_THRESHOLD;
+                if (gap > thr) {
+                    val = nan("");
+                    if (nd.depth < 24) {  // quadrature.c:922
+                        const int side = lane % 3;
+                        const double len = dist3(s_v + 3 * side, s_v + 3 * ((side + 1) % 3));
+                        double longest = 0.0;
+#pragma unroll
+                        for (int i = 0; i < 3; ++i) {
+                            const double sl = __shfl_sync(0xffffffffu, len, i);
+                            if (sl > longest) {
+                                longest = sl;
+                                e = i;
+                            }
+                        }
+                        const unsigned tied =
+                            __ballot_sync(0xffffffffu, lane < 3 && lane != e && len >= longest * (1.0 - 1e-10));
+                        if (tied) mflags |= MARG_TIE;
+                        int at = 0;
+                        if (lane == 0) at = atomicAdd(&A.count[lv + 1], 2);
+                        at = __shfl_sync(0xffffffffu, at, 0);
+                        if (next_base + at + 2 > cap) {
+                            if (lane == 0) atomicExch(A.overflow, 1);
+                        } else {
+                            child = next_base + at;
+                            LevelNode &left = A.pool[child], &right = A.pool[child + 1];
+                            const int j = (e + 1) % 3, k = (e + 2) % 3;
+                            if (lane < 9) {
+                                const int p = lane / 3, t = lane % 3;
+                                const double mid = 0.5 * (s_v[3 * e + t] + s_v[3 * j + t]);
+                                left.v[lane] = p == 0 ? s_v[3 * e + t] : p == 1 ? mid : s_v[3 * k + t];
+                                right.v[lane] = p == 0 ? mid : p == 1 ? s_v[3 * j + t] : s_v[3 * k + t];
+                            } else if (lane < 11) {
+                                LevelNode &c = lane == 9 ? left : right;
+                                c.tol = tol * 0.5;
+                                c.jac = jac * 0.5;
+                                c.depth = nd.depth + 1;
+                                c.job = nd.job;
+                                c.child = -1;
+                            }
+                        }
+                    }
+                }
+            }
+            if (lane == 0) {
+                nd.val = val;
+                nd.child = child;
+                nd.edge = e;
+                if (mflags && A.marginal) atomicOr(A.marginal + J.rec, mflags);
             }
         }
-        for (int i = 0; i < 3; ++i)
-            if (i != e && len[i] >= longest * (1.0 - 1e-10)) mflags |= MARG_TIE;
-        nd.edge = e;
-        int at = atomicAdd(A.count, 2);
-        if (at + 2 > cap) {
-            atomicExch(A.overflow, 1);
-            nd.val = nan("");
-        } else {
-            nd.child = next_base + at;
-            LevelNode &left = A.pool[next_base + at], &right = A.pool[next_base + at + 1];
-            int j = (e + 1) % 3, k = (e + 2) % 3;
-            for (int dd = 0; dd < 3; ++dd) {
-                double mid = 0.5 * (v[3 * e + dd] + v[3 * j + dd]);
-                left.v[dd] = v[3 * e + dd];
-                left.v[3 + dd] = mid;
-                left.v[6 + dd] = v[3 * k + dd];
-                right.v[dd] = mid;
-                right.v[3 + dd] = v[3 * j + dd];
-                right.v[6 + dd] = v[3 * k + dd];
+        grid.sync();
+        const int next = lv + 1 < kLevels ? *(volatile int *)&A.count[lv + 1] : 0;
+        if (next_base + next > cap) return;  // overflow: the same for every CTA
+        if (next == 0) break;
+        base = next_base;
+        n = next;
+        ++lv;
+    }
+    if (tid == 0 && evals) atomicAdd(A.evals, evals);
+    const int first = blockIdx.x * kTreeThreads + tid, step = gridDim.x * kTreeThreads;
+    // value(node) = value(left) + value(right); subtree sizes
+    for (int l = lv, b = base; n > 0 && l >= 0; --l) {
+        const int m = *(volatile int *)&A.count[l];
+        for (int i = first; i < m; i += step) {
+            LevelNode &nd = A.pool[b + i];
+            nd.size = 1;
+            if (nd.child >= 0) {
+                const LevelNode &x = A.pool[nd.child], &y = A.pool[nd.child + 1];
+                nd.val = x.val + y.val;
+                nd.size = 1 + x.size + y.size;
             }
-            left.tol = right.tol = tol * 0.5;
-            left.depth = right.depth = depth + 1;
-            left.job = right.job = nd.job;
-            left.child = right.child = -1;
         }
+        grid.sync();
+        if (l > 0) b -= *(volatile int *)&A.count[l - 1];
     }
-    if (mflags && A.marginal) atomicOr(A.marginal + J.rec, mflags);
-}
-
-// value(node) = value(left) + value(right); subtree sizes
-__global__ void k_level_up(LevelNode *pool, int base, int n) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    LevelNode &nd = pool[base + i];
-    if (nd.child >= 0) {
-        const LevelNode &l = pool[nd.child], &r = pool[nd.child + 1];
-        nd.val = l.val + r.val;
-        nd.size = 1 + l.size + r.size;
-    } else {
-        nd.size = 1;
-    }
-}
-
-// depth-first positions of the children; the decision trace
-__global__ void k_level_down(LevelArgs A, int base, int n) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const LevelNode &nd = A.pool[base + i];
-    if (A.trace && nd.pos < kTraceCap)
-        A.trace[(size_t)(A.job0 + nd.job) * kTraceCap + nd.pos] = nd.child >= 0 ? (unsigned char)nd.edge : kAccept;
-    if (nd.child >= 0) {
-        LevelNode &l = A.pool[nd.child], &r = A.pool[nd.child + 1];
-        l.pos = nd.pos + 1;
-        r.pos = nd.pos + 1 + l.size;
+    // depth-first positions of the children; the decision trace
+    for (int l = 0, b = 0; n > 0 && l <= lv; ++l) {
+        const int m = *(volatile int *)&A.count[l];
+        for (int i = first; i < m; i += step) {
+            const LevelNode &nd = A.pool[b + i];
+            if (A.trace && nd.pos < kTraceCap)
+                A.trace[(size_t)(A.job0 + nd.job) * kTraceCap + nd.pos] =
+                    nd.child >= 0 ? (unsigned char)nd.edge : kAccept;
+            if (nd.child >= 0) {
+                LevelNode &x = A.pool[nd.child], &y = A.pool[nd.child + 1];
+                x.pos = nd.pos + 1;
+                y.pos = nd.pos + 1 + x.size;
+            }
+        }
+        if (l < lv) grid.sync();
+        b += m;
     }
 }
 
 // roots: the job's value, trace length, full-trace flag
-__global__ void k_level_roots(LevelArgs A, int base, int n) {
+__global__ void k_level_roots(LevelArgs A) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const LevelNode &nd = A.pool[base + i];
+    if (i >= A.count[0] || *A.overflow) return;
+    const LevelNode &nd = A.pool[i];
     const LevelJob &J = A.jobs[nd.job];
     A.slot[J.slot] = nd.val;
     if (A.trace_len) A.trace_len[A.job0 + nd.job] = nd.size < kTraceCap ? nd.size : kTraceCap;
@@ -854,9 +911,8 @@ static bool near_levels_enabled() {
     return on;
 }
 
-// All 8 jobs of the first nrec records of E's list, level by level, in
-// chunks whose trees fit the node pool (a chunk that overflows is retried
-// with half the jobs).
+// All 8 jobs of the first nrec records of E's list, in chunks whose trees fit
+// the node pool (a chunk that overflows is retried with half the jobs).
 static bool near_eval_levels(const NearEvalArgs &E, int nrec) {
     static const int kPoolNodes = 1 << 21;
     const long long total = (long long)nrec * 8;
@@ -864,8 +920,15 @@ static bool near_eval_levels(const NearEvalArgs &E, int nrec) {
     long long chunk = total < (1 << 16) ? total : (1 << 16);
     DBuf<LevelNode> pool(kPoolNodes);
     DBuf<LevelJob> jobs((size_t)chunk);
-    DBuf<int> cnt(1), ovf(1);
-    if (!pool.p || !jobs.p || !cnt.p || !ovf.p) return false;
+    DBuf<int> cnt(kLevels + 2);
+    if (!pool.p || !jobs.p || !cnt.p) return false;
+    int dev = 0, sms = 0, per_sm = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (!cuda_ok(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_level_tree, kTreeThreads, 0),
+                 "near-field levels") ||
+        per_sm < 1)
+        return false;
     LevelArgs L;
     L.corner = E.corner;
     L.rec = E.rec;
@@ -879,37 +942,24 @@ static bool near_eval_levels(const NearEvalArgs &E, int nrec) {
     L.jobs = jobs.p;
     L.pool = pool.p;
     L.count = cnt.p;
-    L.overflow = ovf.p;
+    L.overflow = cnt.p + kLevels + 1;
     L.evals = E.evals;
-    std::vector<int> base, cnt_l;
     for (long long job0 = 0; job0 < total;) {
         const long long nj = std::min(chunk, total - job0);
         L.job0 = job0;
         L.njob = nj;
-        base.assign(1, 0);
-        cnt_l.clear();
-        int h[2] = {0, 0};
-        cudaMemsetAsync(cnt.p, 0, sizeof(int), stream());
-        cudaMemsetAsync(ovf.p, 0, sizeof(int), stream());
-        PEEC_LAUNCH(k_level_init, (unsigned)((nj + 127) / 128), 128, 0, L, 0, kPoolNodes);
-        cudaMemcpyAsync(&h[0], cnt.p, sizeof(int), cudaMemcpyDeviceToHost, stream());
-        cudaMemcpyAsync(&h[1], ovf.p, sizeof(int), cudaMemcpyDeviceToHost, stream());
-        if (!sync("near-field roots")) return false;
-        bool overflow = h[1] != 0;
-        cnt_l.push_back(h[0]);
-        while (!overflow && cnt_l.back() > 0) {
-            const int lv = (int)cnt_l.size() - 1;
-            const int next_base = base[lv] + cnt_l[lv];
-            cudaMemsetAsync(cnt.p, 0, sizeof(int), stream());
-            PEEC_LAUNCH(k_level_eval, (unsigned)((cnt_l[lv] + 7) / 8), 256, 0, L, base[lv], cnt_l[lv], next_base,
-                        kPoolNodes - next_base);
-            cudaMemcpyAsync(&h[0], cnt.p, sizeof(int), cudaMemcpyDeviceToHost, stream());
-            cudaMemcpyAsync(&h[1], ovf.p, sizeof(int), cudaMemcpyDeviceToHost, stream());
-            if (!sync("near-field level")) return false;
-            overflow = h[1] != 0;
-            base.push_back(next_base);
-            cnt_l.push_back(h[0]);
-        }
+        int overflow = 0, cap = kPoolNodes;
+        cudaMemsetAsync(cnt.p, 0, (kLevels + 2) * sizeof(int), stream());
+        PEEC_LAUNCH(k_level_init, (unsigned)((nj + 127) / 128), 128, 0, L, cap);
+        void *args[] = {&L, &cap};
+        note_launch();
+        if (!cuda_ok(cudaLaunchCooperativeKernel((const void *)k_level_tree, dim3(sms * per_sm), dim3(kTreeThreads), args,
+                                                 0, stream()),
+                     "near-field levels"))
+            return false;
+        PEEC_LAUNCH(k_level_roots, (unsigned)((nj + 255) / 256), 256, 0, L);
+        cudaMemcpyAsync(&overflow, L.overflow, sizeof(int), cudaMemcpyDeviceToHost, stream());
+        if (!sync("near-field levels")) return false;
         if (overflow) {
             if (nj == 1) {
                 set_error("near-field quadrature: one refinement tree exceeds %d nodes", kPoolNodes);
@@ -918,12 +968,6 @@ static bool near_eval_levels(const NearEvalArgs &E, int nrec) {
             chunk = (nj + 1) / 2;
             continue;
         }
-        const int levels = (int)cnt_l.size() - 1;  // the last level is empty
-        for (int lv = levels - 1; lv >= 0; --lv)
-            PEEC_LAUNCH(k_level_up, (unsigned)((cnt_l[lv] + 255) / 256), 256, 0, pool.p, base[lv], cnt_l[lv]);
-        for (int lv = 0; lv < levels; ++lv)
-            PEEC_LAUNCH(k_level_down, (unsigned)((cnt_l[lv] + 255) / 256), 256, 0, L, base[lv], cnt_l[lv]);
-        if (cnt_l[0] > 0) PEEC_LAUNCH(k_level_roots, (unsigned)((cnt_l[0] + 255) / 256), 256, 0, L, base[0], cnt_l[0]);
         if (!launch_ok("near-field levels")) return false;
         job0 += nj;
     }
