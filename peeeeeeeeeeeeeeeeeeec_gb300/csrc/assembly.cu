@@ -371,6 +371,9 @@ struct NearWarpSmem {
 enum : int { MARG_THRESHOLD = 1, MARG_TIE = 2, MARG_TRACE_FULL = 4 };
 static const int kTraceCap = 256;       // decisions recorded per job
 static const unsigned char kAccept = 0xFF;
+// A refined node's entry is its bisected edge, plus kClose if another edge is within
+// 1e-6 of its length: at other nodes no copy can find another edge longest.
+static const unsigned char kClose = 4;
 
 __device__ double warp_adaptive(const double *outer, NearWarpSmem &sm, int order, double abs_tol,
                                 unsigned long long &evals, int &mflags, unsigned char *trace, int &trace_len) {
@@ -451,7 +454,7 @@ __device__ double warp_adaptive(const double *outer, NearWarpSmem &sm, int order
             if (i != e && len[i] >= longest * (1.0 - 1e-10)) mflags |= MARG_TIE;
         if (trace) {
             if (trace_len < kTraceCap) {
-                if (lane == 0) trace[trace_len] = (unsigned char)e;
+                if (lane == 0) trace[trace_len] = (unsigned char)(e | kClose);
                 ++trace_len;
             } else {
                 mflags |= MARG_TRACE_FULL;
@@ -635,7 +638,7 @@ struct LevelNode {
     int child;  // first child (left; right = child + 1) or -1
     int size;   // nodes in the subtree
     int pos;    // depth-first position in the job's tree
-    int edge;   // bisected edge of a refined node
+    int edge;   // bisected edge of a refined node, + kClose
     double jac; // twice the area
 };
 
@@ -789,7 +792,7 @@ __global__ void __launch_bounds__(kTreeThreads, 3) k_level_tree(LevelArgs A, int
             lo = jac * warp_sum(lo);
             hi = jac * warp_sum(hi);
             evals += ntot;
-            int child = -1, e = 0;
+            int child = -1, e = 0, close = 0;
             double val = hi;
             int mflags = 0;
             const double tol = nd.tol, thr = tol + 2e-5 * fabs(hi), gap = fabs(hi - lo);
@@ -814,6 +817,7 @@ __global__ void __launch_bounds__(kTreeThreads, 3) k_level_tree(LevelArgs A, int
                         const unsigned tied =
                             __ballot_sync(0xffffffffu, lane < 3 && lane != e && len >= longest * (1.0 - 1e-10));
                         if (tied) mflags |= MARG_TIE;
+                        if (__any_sync(0xffffffffu, lane < 3 && lane != e && len >= longest * (1.0 - 1e-6))) close = kClose;
                         int at = 0;
                         if (lane == 0) at = atomicAdd(&A.count[lv + 1], 2);
                         at = __shfl_sync(0xffffffffu, at, 0);
@@ -843,7 +847,7 @@ __global__ void __launch_bounds__(kTreeThreads, 3) k_level_tree(LevelArgs A, int
             if (lane == 0) {
                 nd.val = val;
                 nd.child = child;
-                nd.edge = e;
+                nd.edge = e | close;
                 if (mflags && A.marginal) atomicOr(A.marginal + J.rec, mflags);
             }
         }
@@ -1150,16 +1154,19 @@ __global__ void k_round_replay(int nrec, const int *rep, const int *rep_pos, con
             ++pos;
             continue;
         }
-        int e = 0;
-        double longest = 0.0;
-        for (int i = 0; i < 3; ++i) {
-            double sl = dist3(v + 3 * i, v + 3 * ((i + 1) % 3));
-            if (sl > longest) {
-                longest = sl;
-                e = i;
+        int e = c & 3;
+        if (c & kClose) {
+            double longest = 0.0;
+            e = 0;
+            for (int i = 0; i < 3; ++i) {
+                double sl = dist3(v + 3 * i, v + 3 * ((i + 1) % 3));
+                if (sl > longest) {
+                    longest = sl;
+                    e = i;
+                }
             }
         }
-        if (e != (int)c || sp + 2 > kStackCap) {
+        if (e != (c & 3) || sp + 2 > kStackCap) {
             code = (jb << 12) | (pos << 2) | (e & 3);
             break;
         }
