@@ -84,6 +84,7 @@ struct RegionsDev {
     float4 *boxf = nullptr;    // [np*2]  box rounded to FP32: (lo, size), (hi, 0) -- the scan's far filter
     int *axis = nullptr;       // [n]     0/1/2 when dir is exactly +-e_axis, else -1 (inductance)
     double cmax = 0.0;         // largest |corner coordinate| (scale of the rounding noise)
+    double mid[3] = {};        // middle of the bounding box
 };
 
 // one far-rule point: position and weight (32-byte aligned for vector loads)
@@ -93,6 +94,7 @@ struct alignas(32) FarPt {
 
 // The same point as unevaluated float pairs (hi + lo == the double to 2^-48
 // relative): the far rule runs on the FP32 pipes in double-float arithmetic.
+// For the double-float rule the coordinates are taken from the mesh's middle.
 struct alignas(32) FarPtF {
     float xh, yh, zh, wh, xl, yl, zl, wl;
 };
@@ -123,7 +125,7 @@ __global__ void k_patch_prep(RegionsDev R) {
 // Far-rule points of patch p: triangle t (0: corners 0,1,2; 1: 0,2,3), point
 // (iu, iv) at index t*q*q + iu*q + iv; weight (0.5 w_iu)(0.5 w_iv) J
 // (reference quadrature.c:679-783 evaluates the same points per pair).
-__global__ void k_far_points(RegionsDev R, int q, int row, FarPt *pts, FarPtF *ptf) {
+__global__ void k_far_points(RegionsDev R, int q, int row, FarPt *pts, FarPtF *ptf, int centred) {
     int np = R.np, per = 2 * q * q;
     long long g = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (g >= (long long)np * per) return;
@@ -138,6 +140,7 @@ __global__ void k_far_points(RegionsDev R, int q, int row, FarPt *pts, FarPtF *p
     double w = wu * wv * jac;
     pts[g] = FarPt{r[0], r[1], r[2], w};
     FarPtF f;
+    for (int k = 0; k < 3 && centred; ++k) r[k] -= R.mid[k];
     split_df(r[0], f.xh, f.xl);
     split_df(r[1], f.yh, f.yl);
     split_df(r[2], f.zh, f.zl);
@@ -1330,19 +1333,9 @@ __device__ __forceinline__ f2 quick_two_sum(float a, float b) {  // |a| >= |b|
     float s = a + b;
     return f2{s, b - (s - a)};
 }
-__device__ __forceinline__ f2 df_sub(f2 a, f2 b) {
-    f2 s = two_sum(a.h, -b.h);
-    return quick_two_sum(s.h, s.l + (a.l - b.l));
-}
 __device__ __forceinline__ f2 df_add(f2 a, f2 b) {
     f2 s = two_sum(a.h, b.h);
     return quick_two_sum(s.h, s.l + (a.l + b.l));
-}
-__device__ __forceinline__ f2 df_sqr(f2 a) {
-    float p = a.h * a.h;
-    float e = fmaf(a.h, a.h, -p);
-    e = fmaf(a.h + a.h, a.l, e);
-    return quick_two_sum(p, e);
 }
 __device__ __forceinline__ f2 df_mul(f2 a, f2 b) {
     float p = a.h * b.h;
@@ -1362,17 +1355,41 @@ __device__ __forceinline__ float rsqrt_hw(float x) {
     return y;
 }
 
-// 1/sqrt(x) for x > 0 to ~1e-14 relative: hardware rsqrtf seed y, residual
-// r = 1 - x y^2 in double-float, one Halley step y (1 + r/2 + 3 r^2 / 8)
-// (third-order convergence from the 2^-22 seed).
-__device__ __forceinline__ f2 df_rsqrt(f2 x) {
-    float y = rsqrt_hw(x.h);
-    float yy = y * y;
-    f2 y2 = f2{yy, fmaf(y, y, -yy)};
-    f2 t = df_mul(x, y2);
-    float r = (1.0f - t.h) - t.l;
-    float c = y * fmaf(0.375f * r, r, 0.5f * r);
-    return quick_two_sum(y, c);
+// Adds w / |a - b| to the double-float sum (hi, lo): 83 FP32 instructions,
+// against 113 with a normalised double-float result after every operation
+// (box of 2 x 1 x 0.5 m at 5 cm, entries of P: 24.6 ms, now 18.1; the
+// rms error against the FP64 rule is the same 1.5e-15, the largest 9e-15 instead of 1.3e-14).
+//  - The high parts' differences with their errors, the low parts added to
+//    these: dh + dl.
+//  - |d|^2 as the three squares of dh with their FMA errors, one sum of them,
+//    2 dh dl and dl^2 (2^-48 of it, but always positive: without, sums came out
+//    6e-16 too large); renormalised once.
+//  - 1/sqrt(x): hardware seed y, r = 1 - x y^2 from the same parts (1 - xh y^2
+//    is exact), one Halley step y + r y / 2 + 3 r^2 y / 8, third order from 2^-22
+//    (with y r (1/2 + 3 r / 8) the rounding next to 1/2 left a mean of 2e-16).
+//  - The sum's low part is left as it grows (<= 2^-24 of the sum a term).
+__device__ __forceinline__ void df_add_inverse(const float4 ah, const float4 al, const float4 bh, const float4 bl,
+                                               float &hi, float &lo) {
+    const f2 ux = two_sum(ah.x, -bh.x), uy = two_sum(ah.y, -bh.y), uz = two_sum(ah.z, -bh.z);
+    const float dx = ux.h, dy = uy.h, dz = uz.h;
+    const float lx = ux.l + (al.x - bl.x), ly = uy.l + (al.y - bl.y), lz = uz.l + (al.z - bl.z);
+    const float px = dx * dx, py = dy * dy, pz = dz * dz;
+    const f2 s = two_sum(px, py), q = two_sum(s.h, pz);
+    const float cross = fmaf(dz, lz, fmaf(dy, ly, dx * lx));
+    const float low = fmaf(lz, lz, fmaf(ly, ly, lx * lx));
+    const float e = (fmaf(dx, dx, -px) + fmaf(dy, dy, -py)) + (fmaf(dz, dz, -pz) + ((s.l + q.l) + low));
+    const f2 x = quick_two_sum(q.h, fmaf(2.0f, cross, e));
+    const float y = rsqrt_hw(x.h);
+    const float yy = y * y, ye = fmaf(y, y, -yy);
+    const float p = x.h * yy;
+    const float r = (1.0f - p) - fmaf(x.l, yy, fmaf(x.h, ye, fmaf(x.h, yy, -p)));
+    const float ry = r * y;
+    const float cy = fmaf(0.375f * r, ry, 0.5f * ry);
+    const float t = bh.w * y;
+    const float te = fmaf(bl.w, y, fmaf(bh.w, cy, fmaf(bh.w, y, -t)));
+    const f2 n = two_sum(hi, t);
+    hi = n.h;
+    lo += n.l + te;
 }
 
 // FP32 form accumulating into this lane's running double-float sum `acc`
@@ -1503,30 +1520,20 @@ __device__ __forceinline__ void far_entry_f32(const FarPtF *ptf, int i0, int ni,
 // staged in the warp's shared slot (two float4 a point) as above.
 __device__ __forceinline__ void far_pair_df_acc32(const FarPtF *pa, const FarPtF *pb, float4 *slot, f2 &acc) {
     const int lane = threadIdx.x & 31;
-    const FarPtF A = pa[lane];
-    const float4 *pbv = reinterpret_cast<const float4 *>(pb);
+    const float4 *pav = reinterpret_cast<const float4 *>(pa), *pbv = reinterpret_cast<const float4 *>(pb);
+    const float4 ah = pav[2 * lane], al = pav[2 * lane + 1];  // (xh, yh, zh, wh), (xl, yl, zl, wl)
     const float4 b0 = pbv[lane], b1 = pbv[32 + lane];
     __syncwarp();
     slot[lane] = b0;
     slot[32 + lane] = b1;
     __syncwarp();
-    const f2 ax = {A.xh, A.xl}, ay = {A.yh, A.yl}, az = {A.zh, A.zl};
-    f2 s0 = {0.0f, 0.0f}, s1 = {0.0f, 0.0f};
-#pragma unroll 4
-    for (int q = 0; q < 32; ++q) {
-        // point q: float4 2q (xh, yh, zh, wh) and 2q + 1 (xl, yl, zl, wl)
-        const float4 h = slot[2 * q], l = slot[2 * q + 1];
-        const f2 dx = df_sub(ax, f2{h.x, l.x});
-        const f2 dy = df_sub(ay, f2{h.y, l.y});
-        const f2 dz = df_sub(az, f2{h.z, l.z});
-        const f2 r2 = df_add(df_add(df_sqr(dx), df_sqr(dy)), df_sqr(dz));
-        const f2 t = df_mul(f2{h.w, l.w}, df_rsqrt(r2));
-        if (q & 1)
-            s1 = df_add(s1, t);
-        else
-            s0 = df_add(s0, t);
+    float hi0 = 0.0f, hi1 = 0.0f, lo0 = 0.0f, lo1 = 0.0f;
+#pragma unroll 2
+    for (int q = 0; q < 32; q += 2) {
+        df_add_inverse(ah, al, slot[2 * q], slot[2 * q + 1], hi0, lo0);
+        df_add_inverse(ah, al, slot[2 * q + 2], slot[2 * q + 3], hi1, lo1);
     }
-    acc = df_add(acc, df_mul(f2{A.wh, A.wl}, df_add(s0, s1)));
+    acc = df_add(acc, df_mul(f2{ah.w, al.w}, df_add(f2{hi0, lo0}, f2{hi1, lo1})));
 }
 
 // Double-float form, accumulating into this lane's running sum `acc` (the
@@ -1536,31 +1543,19 @@ __device__ __forceinline__ void far_pair_df_acc32(const FarPtF *pa, const FarPtF
 // per lane keep the dependent add chains short.  A NaN propagates into `acc`.
 __device__ __forceinline__ void far_pair_df_acc(const FarPtF *pa, const FarPtF *pb, int npts, f2 &acc) {
     const int lane = threadIdx.x & 31;
+    const float4 *pav = reinterpret_cast<const float4 *>(pa), *pbv = reinterpret_cast<const float4 *>(pb);
     for (int p = lane; p < npts; p += 32) {
-        FarPtF A = pa[p];
-        f2 ax = {A.xh, A.xl}, ay = {A.yh, A.yl}, az = {A.zh, A.zl};
-        f2 s0 = {0.0f, 0.0f}, s1 = {0.0f, 0.0f};
+        const float4 ah = pav[2 * p], al = pav[2 * p + 1];
+        float hi0 = 0.0f, hi1 = 0.0f, lo0 = 0.0f, lo1 = 0.0f;
+        // no R <= 0 test: FAR patches of nonzero size never share a
+        // point (the caller skips zero-size patches, whose weights are
+        // zero), and a NaN reaches the entry's sum, which the epilogue
+        // checks; npts = 2 q^2 is even
         for (int q = 0; q < npts; q += 2) {
-#pragma unroll
-            for (int u = 0; u < 2; ++u) {
-                if (q + u >= npts) break;
-                FarPtF B = pb[q + u];
-                f2 dx = df_sub(ax, f2{B.xh, B.xl});
-                f2 dy = df_sub(ay, f2{B.yh, B.yl});
-                f2 dz = df_sub(az, f2{B.zh, B.zl});
-                // no R <= 0 test: FAR patches of nonzero size never share a
-                // point (the caller skips zero-size patches, whose weights are
-                // zero), and a NaN reaches the entry's sum, which the epilogue
-                // checks
-                f2 r2 = df_add(df_add(df_sqr(dx), df_sqr(dy)), df_sqr(dz));
-                f2 t = df_mul(f2{B.wh, B.wl}, df_rsqrt(r2));
-                if (u == 0)
-                    s0 = df_add(s0, t);
-                else
-                    s1 = df_add(s1, t);
-            }
+            df_add_inverse(ah, al, pbv[2 * q], pbv[2 * q + 1], hi0, lo0);
+            df_add_inverse(ah, al, pbv[2 * q + 2], pbv[2 * q + 3], hi1, lo1);
         }
-        acc = df_add(acc, df_mul(f2{A.wh, A.wl}, df_add(s0, s1)));
+        acc = df_add(acc, df_mul(f2{ah.w, al.w}, df_add(f2{hi0, lo0}, f2{hi1, lo1})));
     }
 }
 
@@ -1571,44 +1566,6 @@ __device__ __forceinline__ f2 warp_sum_df2(f2 v) {
         v = df_add(v, o);
     }
     return v;
-}
-
-__device__ __forceinline__ double warp_sum_df(f2 v) {
-#pragma unroll
-    for (int m = 16; m > 0; m >>= 1) {
-        f2 o = {__shfl_xor_sync(0xffffffffu, v.h, m), __shfl_xor_sync(0xffffffffu, v.l, m)};
-        v = df_add(v, o);
-    }
-    return (double)v.h + (double)v.l;
-}
-
-// Double-float form of the same sum: every point difference, square, the
-// reciprocal square root and the accumulation carry ~48 significant bits,
-// on the FP32 pipes; per-lane partial sums are combined in FP64.
-__device__ __forceinline__ double far_pair_df(const FarPtF *pa, const FarPtF *pb, int npts) {
-    const int lane = threadIdx.x & 31;
-    double acc = 0.0;
-    for (int p = lane; p < npts; p += 32) {
-        FarPtF A = pa[p];
-        f2 ax = {A.xh, A.xl}, ay = {A.yh, A.yl}, az = {A.zh, A.zl};
-        f2 s = {0.0f, 0.0f};
-        bool bad = false;
-#pragma unroll 2
-        for (int q = 0; q < npts; ++q) {
-            FarPtF B = pb[q];
-            f2 dx = df_sub(ax, f2{B.xh, B.xl});
-            f2 dy = df_sub(ay, f2{B.yh, B.yl});
-            f2 dz = df_sub(az, f2{B.zh, B.zl});
-            f2 r2 = df_add(df_add(df_sqr(dx), df_sqr(dy)), df_sqr(dz));
-            if (r2.h <= 0.0f) continue;  // the reference skips R <= 0
-            if (!(r2.h == r2.h) || !(B.wh == B.wh)) bad = true;  // NaN, as the reference propagates it
-            s = df_add(s, df_mul(f2{B.wh, B.wl}, df_rsqrt(r2)));
-        }
-        double sd = (double)s.h + (double)s.l;
-        if (bad) sd = nan("");
-        acc = fma((double)A.wh + (double)A.wl, sd, acc);
-    }
-    return warp_sum(acc);
 }
 
 __device__ __forceinline__ bool near_lookup(const TileArgs &T, int i, int j, double &k) {
@@ -2236,7 +2193,14 @@ struct DeviceRegions {
         view.dir = dir.p;
         view.scale = scale.p;
         view.cmax = 0.0;
-        for (double v : H.corner) view.cmax = fmax(view.cmax, fabs(v));
+        double lo[3] = {}, hi[3] = {};
+        for (size_t t = 0; t < H.corner.size(); ++t) {
+            const double v = H.corner[t];
+            view.cmax = fmax(view.cmax, fabs(v));
+            lo[t % 3] = t < 3 ? v : fmin(lo[t % 3], v);
+            hi[t % 3] = t < 3 ? v : fmax(hi[t % 3], v);
+        }
+        for (int k = 0; k < 3; ++k) view.mid[k] = 0.5 * (lo[k] + hi[k]);
         if (ok && np) {
             PEEC_LAUNCH(k_patch_prep, (np + 127) / 128, 128, 0, view);
             ok = launch_ok("patch preparation");
@@ -2290,6 +2254,11 @@ static int run_assembly(DeviceRegions &D, int kind, const AssemblyOptions &o, do
     const RegionsDev &R = D.view;
     const int n = R.n, np = R.np;
     const int q = o.orders[0], npts = 2 * q * q;
+    // The double-float and FP32 far loops carry no R <= 0 test, which relies
+    // on FAR patches being apart: true for near_factor > 0 (a positive box
+    // gap).  With near_factor == 0 overlapping patches are FAR, so the FP64
+    // form, which skips R <= 0 as the reference does, takes them.
+    const int far_df = o.near_factor > 0.0 ? far_mode_df() : 0;
     cudaEvent_t ev[4];
     for (auto &e : ev) cudaEventCreate(&e);
     cudaEventRecord(ev[0], stream());
@@ -2306,7 +2275,8 @@ static int run_assembly(DeviceRegions &D, int kind, const AssemblyOptions &o, do
     cudaMemsetAsync(counter.p, 0, sizeof(int), stream());
     if (np) {
         long long tot = (long long)np * npts;
-        PEEC_LAUNCH(k_far_points, (unsigned)((tot + 255) / 256), 256, 0, R, q, gl_row(q), pts.p, ptf.p);
+        PEEC_LAUNCH(k_far_points, (unsigned)((tot + 255) / 256), 256, 0, R, q, gl_row(q), pts.p, ptf.p,
+                    far_df == 1);
         ScanArgs s{R, kind, o.near_factor, o.dir_tol, only_a, only_b};
         PEEC_LAUNCH(k_near_scan, (unsigned)(((long long)np * 32 + 255) / 256), 256, 0, s, 0, count.p, nullptr, nullptr,
                     farcount.p);
@@ -2496,11 +2466,7 @@ static int run_assembly(DeviceRegions &D, int kind, const AssemblyOptions &o, do
     T.pts = pts.p;
     T.ptf = ptf.p;
     T.npts = npts;
-    // The double-float and FP32 far loops carry no R <= 0 test, which relies
-    // on FAR patches being apart: true for near_factor > 0 (a positive box
-    // gap).  With near_factor == 0 overlapping patches are FAR, so the FP64
-    // form, which skips R <= 0 as the reference does, takes them.
-    T.far_df = o.near_factor > 0.0 ? far_mode_df() : 0;
+    T.far_df = far_df;
     T.near_off = near_off.p;
     T.near_rec = rec.p;
     T.near_k = kval.p;
@@ -2723,7 +2689,8 @@ static int assemble_retarded(const Mesh *mesh, const DualMesh *dual, int kind, c
         pts.alloc((size_t)tot);
         ptf.alloc((size_t)tot);
         if (!pts.p || !ptf.p) return false;
-        PEEC_LAUNCH(k_far_points, (unsigned)((tot + 255) / 256), 256, 0, R, order, gl_row(order), pts.p, ptf.p);
+        PEEC_LAUNCH(k_far_points, (unsigned)((tot + 255) / 256), 256, 0, R, order, gl_row(order), pts.p, ptf.p,
+                    0);
         return true;
     };
     DBuf<FarPt> pts, pts3, pts2;
