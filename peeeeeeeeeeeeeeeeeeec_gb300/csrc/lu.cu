@@ -10,13 +10,14 @@
 // (data[i*n+j], complex interleaved {re, im}), so the packed L\U factor is
 // downloaded without any transpose.  Blocked right-looking algorithm with
 // panel width NB:
-//   k_panel     one CTA factors rows k0..n-1 of columns k0..k0+NB-1 column by
+//   k_panel     factors rows k0..n-1 of columns k0..k0+NB-1 column by
 //               column: argmax (first maximum wins, as the reference), row
 //               swap inside the panel, multipliers, rank-1 update of the
-//               remaining panel columns;
+//               remaining panel columns (one CTA; k_panel_cl64 one cluster,
+//               k_panel_lean64 and k_panel_coop one grid);
 //   k_laswp     replays the panel's row swaps on the columns left and right
 //               of the panel;
-//   k_trsm      U12 = L11^-1 A12 (one thread per column, L11 in shared memory);
+//   k_rows_of_u U12 = L11^-1 A12 (k_trsm in the mixed path);
 //   A22 -= L21 U12: k_gemm_rect, register-tiled FP64 (complex: 4 real FMAs per
 //               complex multiply-add), or from about a thousand unknowns on
 //               the digit GEMM on the tensor cores (digit_gemm.cu).
@@ -757,7 +758,7 @@ __global__ void __launch_bounds__(kLeanThreads) k_panel_lean(cplxf *a, int n, in
     if (c == 0 && tid == 0) atomicExch(&ps->gen, gen0 + (unsigned)kb);
 }
 
-// ---- lean FP64 panel (the plain LU) --------------------------------
+// ---- lean FP64 panel (the plain LU, panels too large for one cluster) ---
 // The lean panel's structure for the FP64 factorisations, with the
 // reference's arithmetic kept bit for bit (FP64 |z|, first maximum wins,
 // NaN never wins, L = a / pivot by the same complex division, one msub per
@@ -1243,6 +1244,340 @@ static bool launch_cl_panel(cplxf *a, int n, int k0, int kb, double limit, long 
     return cuda_ok(cudaLaunchKernelEx(&cfg, k_panel_cl, a, n, k0, kb, rows, limit, piv, st), "cluster FP32 panel launch");
 }
 
+
+// ---- cluster FP64 panel ---------------------------------------------
+// k_panel_cl's structure for the FP64 factorisations, with k_panel_lean64's
+// arithmetic and pivots bit for bit.  Sixteen SMs share the FP64 work (84
+// instructions a row and column, complex), but a column costs one cluster
+// barrier instead of an exchange of flags through L2 (panels of a whole
+// factorisation, lean / cluster, in ms: real 833: 4.7 / 2.2, 2102: 13.2 / 5.8, 8402:
+// 47 / 35; complex 833: 9.5 / 3.4, 2102: 24.0 / 9.9, 6000: 69 / 43, 8402: 95 / 70).
+// What keeps the FP64 units (a warp instruction takes 64 cycles of its
+// scheduler) off the critical path:
+//  - magnitudes are compared as integer keys.  Complex: keys of |z|^2; the
+//    correctly rounded |z| decides only where two keys are within 16 ulps or the
+//    largest is not well inside the exponent range (exact_key: one more barrier);
+//  - the column's quotients share one correctly rounded reciprocal; two
+//    corrections by the exact remainder round each correctly (Markstein,
+//    "Computation of elementary functions on the IBM RISC System/6000",
+//    1990), with exponents for which nothing under- or overflows;
+//  - the deferred row updates are dealt to up to four threads a row, so that
+//    every scheduler has work when a CTA holds few rows.
+template <class T>
+struct Cl64Slot {
+    T row[2][NB], krow[2][NB];       // candidate row, row k when owned here; by column parity
+    unsigned long long key[2], xkey[2];
+    int idx[2], xidx[2], close[2];
+};
+
+static const unsigned long long kInfKey = (0x7ffull << 52) + 1;
+static const unsigned long long kCloseUlps = 16;
+
+// 0: never a pivot (NaN below the diagonal), else the magnitude's bits + 1
+__device__ __forceinline__ unsigned long long exact_key(double v, bool diag) {
+    const unsigned long long b = (unsigned long long)__double_as_longlong(v) & ~(1ull << 63);
+    return b >= kInfKey ? (diag ? kInfKey : 0) : b + 1;
+}
+__device__ __noinline__ unsigned long long exact_key(cplx v, bool diag) {
+    return exact_key(hypot_cr(v.re, v.im), diag);
+}
+__device__ __forceinline__ unsigned long long col_key(double v, bool diag) { return exact_key(v, diag); }
+__device__ __forceinline__ unsigned long long col_key(cplx v, bool diag) {
+    const unsigned long long b = (unsigned long long)__double_as_longlong(fma(v.re, v.re, v.im * v.im));
+    if (b < kInfKey - 1) return b + 1;
+    return exact_key(v, diag) ? kInfKey : 0;
+}
+__device__ __forceinline__ bool wide_key(unsigned long long key) {  // not well inside the exponent range
+    const unsigned e = (unsigned)((key - 1) >> 52);
+    return e < 123 || e > 1923;
+}
+
+// largest key, lowest row among equals; the same in every lane
+__device__ __forceinline__ void warp_top(unsigned long long &key, int &idx) {
+    const unsigned hi = (unsigned)(key >> 32), lo = (unsigned)key;
+    const unsigned mh = __reduce_max_sync(0xffffffffu, hi);
+    const unsigned ml = __reduce_max_sync(0xffffffffu, hi == mh ? lo : 0u);
+    idx = __reduce_min_sync(0xffffffffu, hi == mh && lo == ml ? idx : 0x7fffffff);
+    key = (unsigned long long)mh << 32 | ml;
+}
+
+__device__ __forceinline__ bool mid_range(double v) {  // 2^-500 <= |v| < 2^500
+    return ((unsigned)(__double_as_longlong(v) >> 52 & 0x7ff) - 523u) < 1000u;
+}
+// a / b, r the correctly rounded 1 / b
+__device__ __forceinline__ double divide_by(double a, double b, double r) {
+    double q = a * r;
+    if (mid_range(a) && mid_range(b)) {
+        q = fma(fma(-q, b, a), r, q);
+        return fma(fma(-q, b, a), r, q);
+    }
+    return a == 0.0 && mid_range(b) ? q : a / b;
+}
+__device__ __forceinline__ double divisor(double b) { return b; }
+__device__ __forceinline__ double divisor(cplx b) { return b.re * b.re + b.im * b.im; }
+__device__ __forceinline__ double divide_by(double a, double, double den, double r) { return divide_by(a, den, r); }
+__device__ __forceinline__ cplx divide_by(cplx a, cplx b, double den, double r) {  // as divide(a, b)
+    return cplx{divide_by(a.re * b.re + a.im * b.im, den, r), divide_by(a.im * b.re - a.re * b.im, den, r)};
+}
+
+template <class T>
+__global__ void __launch_bounds__(kClMaxThreads) k_panel_cl64(T *a, int n, int k0, int kb, int rows_per_cta,
+                                                              int row_threads, double limit, long long *piv,
+                                                              Status *st, double tie) {
+    namespace cg = cooperative_groups;
+    cg::cluster_group cluster = cg::this_cluster();
+    constexpr bool cx = sizeof(T) == sizeof(cplx);
+    extern __shared__ __align__(16) unsigned char cl_smem[];
+    T(*tile)[kPS] = reinterpret_cast<T(*)[kPS]>(cl_smem);  // [rows_per_cta][kPS]
+    __shared__ Cl64Slot<T> slot;
+    __shared__ T s_prow[2][NB];
+    __shared__ unsigned long long s_wu[32], s_tie;
+    __shared__ int s_wi[32], s_close[2], s_gc, s_p, s_exact, s_bad;
+    __shared__ double s_den, s_rcp, s_val;
+    __shared__ unsigned long long s_key;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int parts = blockDim.x / row_threads, part = tid / row_threads, rt = tid - part * row_threads;
+    const int nrw = row_threads >> 5;  // warps with part == 0
+    const int C = (int)cluster.num_blocks(), c = (int)cluster.block_rank();
+    const int r0 = k0 + c * rows_per_cta, r1 = min(n, r0 + rows_per_cta);
+    const int nrows = r1 > r0 ? r1 - r0 : 0;
+    if (st->code != 0) return;  // uniform over the cluster (set before launch, or after its first barrier)
+    const bool checked = __double_as_longlong(tie) != 0;
+    for (int t = tid; t < nrows * kb; t += blockDim.x) {
+        const int ii = t / kb, j = t % kb;
+        tile[ii][j] = a[(size_t)(r0 + ii) * n + k0 + j];
+    }
+    if (tid < 2) s_close[tid] = 0;
+    __syncthreads();
+    const int i = r0 + rt;
+    const bool mine = rt < nrows, lead = part == 0;
+    T *row = tile[mine ? rt : 0];
+    unsigned long long key = lead && mine ? col_key(row[0], i == k0) : 0;
+    bool failed = false;
+    // the CTA's largest key of `u`, in every lane of every warp
+    auto cta_top = [&](unsigned long long u, unsigned long long &bu, int &bi) {
+        if (lead) {
+            int wi = i;
+            unsigned long long wu = u;
+            warp_top(wu, wi);
+            if (lane == 0) {
+                s_wu[warp] = wu;
+                s_wi[warp] = wi;
+            }
+        }
+        __syncthreads();
+        bu = lane < nrw ? s_wu[lane] : 0;
+        bi = lane < nrw ? s_wi[lane] : 0x7fffffff;
+        warp_top(bu, bi);
+    };
+    for (int kk = 0; kk < kb; ++kk) {
+        const int k = k0 + kk, par = kk & 1;
+        const T *pprev = s_prow[par ^ 1];
+        T *pcur = s_prow[par];
+        const unsigned long long u = mine && i >= k ? key : 0;
+        unsigned long long bu;
+        int bi;
+        cta_top(u, bu, bi);
+        // publish: the candidate as it is (pending the previous column's update)
+        if (warp == 0) {
+            if (lane < kb) slot.row[par][lane] = bu ? tile[bi - r0][lane] : T{};
+            if (lane == 0) {
+                slot.key[par] = bu;
+                slot.idx[par] = bi;
+                s_close[par ^ 1] = 0;
+            }
+        }
+        if (warp == 1 && k >= r0 && k < r1 && lane < kb) slot.krow[par][lane] = tile[k - r0][lane];
+        if (cx && lead && u && i != bi && bu - u <= kCloseUlps) s_close[par] = 1;
+        __syncthreads();
+        if (cx && tid == 0) slot.close[par] = s_close[par];
+        __syncwarp();
+        cluster_arrive();
+        // the previous column's deferred update, between arrive and wait
+        if (kk > 0 && mine && i >= k) {
+            const T m = row[kk - 1];
+#pragma unroll 4
+            for (int j = kk + 1 + part; j < kb; j += parts) row[j] = msub(row[j], m, pprev[j]);
+        }
+        __syncwarp();
+        cluster_wait();
+        // the winner over the cluster
+        auto cluster_top = [&](bool exact) {
+            if (warp == 0) {
+                const Cl64Slot<T> *rs = cluster.map_shared_rank(&slot, lane < C ? lane : 0);
+                const unsigned long long lu = lane < C ? (exact ? rs->xkey[par] : rs->key[par]) : 0;
+                const int li = lane < C ? (exact ? rs->xidx[par] : rs->idx[par]) : 0x7fffffff;
+                unsigned long long wu = lu;
+                int wi = li;
+                warp_top(wu, wi);
+                const bool won = lu == wu && li == wi && lane < C;
+                const unsigned who = __ballot_sync(0xffffffffu, won);
+                bool close = false;
+                if (cx && !exact)
+                    close = __any_sync(0xffffffffu, lane < C && lu && (won ? rs->close[par] != 0 : wu - lu <= kCloseUlps));
+                if (lane == 0) {
+                    s_gc = wu ? __ffs(who) - 1 : -1;
+                    s_p = wi;
+                    s_key = wu;
+                    s_exact = cx && !exact && wu && (close || wide_key(wu));
+                }
+            }
+            __syncthreads();
+        };
+        cluster_top(false);
+        bool pending = kk > 0;  // is the published row short of the previous column's update?
+        const bool exact = s_exact;
+        if (exact) {  // uniform over the cluster: every CTA read the same slots
+            const unsigned long long x = lead && u ? exact_key(row[kk], i == k) : 0;
+            cta_top(x, bu, bi);
+            if (warp == 0) {
+                if (lane < kb) slot.row[par][lane] = bu ? tile[bi - r0][lane] : T{};
+                if (lane == 0) {
+                    slot.xkey[par] = bu;
+                    slot.xidx[par] = bi;
+                }
+            }
+            __syncthreads();
+            cluster_arrive();
+            cluster_wait();
+            cluster_top(true);
+            pending = false;
+        }
+        const int gc = s_gc, p = s_p;
+        // the pivot row, and row k for the owner of p, with the pending update
+        T kval = T{};
+        if (warp == 0) {
+            if (gc >= 0) {
+                const Cl64Slot<T> *ws = cluster.map_shared_rank(&slot, gc);
+                if (lane < kb) {
+                    T v = ws->row[par][lane];
+                    if (pending && lane > kk) v = msub(v, ws->row[par][kk - 1], pprev[lane]);
+                    pcur[lane] = v;
+                }
+                __syncwarp();
+            }
+            const T pv = gc >= 0 ? pcur[kk] : T{};
+            const double den = divisor(pv);
+            // pivot check by the exact magnitude, unless |z|^2 is clear of it
+            const unsigned long long wk = s_key;
+            double gb = -1.0;
+            bool bad = gc < 0;
+            if (!bad) {
+                const double v = __longlong_as_double((long long)(wk - 1));
+                if (cx && !exact && v > limit * limit * (1.0 + 1e-9)) {
+                    gb = INFINITY;  // not needed
+                } else {
+                    gb = cx && !exact ? mag(pv) : v;
+                    bad = !isfinite(gb) || gb <= limit;
+                }
+            }
+            if (lane == 0) {
+                s_bad = bad;
+                s_val = gb;
+                s_den = den;
+                s_rcp = 1.0 / den;
+                if (checked) {  // keys from here on are near ties (twice the fraction for |z|^2)
+                    const unsigned long long pk = col_key(pv, true);
+                    const double v = __longlong_as_double((long long)(pk - 1));
+                    const unsigned long long b = (unsigned long long)tie_limit(v, cx ? 2.0 * tie : tie);
+                    s_tie = b > kCloseUlps ? b + 1 - kCloseUlps : 1;
+                }
+            }
+        }
+        if (warp == 1 && gc == c && p != k && lane < kb) {
+            const Cl64Slot<T> *ks = cluster.map_shared_rank(&slot, (k - k0) / rows_per_cta);
+            kval = ks->krow[par][lane];
+            if (kk > 0 && lane > kk) kval = msub(kval, ks->krow[par][kk - 1], pprev[lane]);
+        }
+        __syncthreads();
+        if (s_bad) {  // uniform over the cluster
+            if (c == 0 && tid == 0) {
+                st->code = 2;
+                st->column = k;
+                st->value = s_val;
+            }
+            failed = true;
+            break;
+        }
+        if (checked && lead && u >= s_tie && i != p) atomicCAS(&st->code, 0, 7);
+        if (p != k) {
+            if (warp == 0 && k >= r0 && k < r1 && lane < kb) tile[k - r0][lane] = pcur[lane];
+            if (warp == 1 && gc == c && lane < kb) tile[p - r0][lane] = kval;
+        }
+        if (c == 0 && tid == 0) piv[k] = p;
+        __syncthreads();
+        if (k + 1 >= n) break;
+        key = 0;
+        if (lead && mine && i > k) {
+            const T m = divide_by(row[kk], pcur[kk], s_den, s_rcp);
+            row[kk] = m;
+            if (kk + 1 < kb) {
+                row[kk + 1] = msub(row[kk + 1], m, pcur[kk + 1]);
+                key = col_key(row[kk + 1], i == k + 1);
+            }
+        }
+    }
+    if (!failed) {
+        __syncthreads();
+        for (int t = tid; t < nrows * kb; t += blockDim.x) {
+            const int ii = t / kb, j = t % kb;
+            a[(size_t)(r0 + ii) * n + k0 + j] = tile[ii][j];
+        }
+    }
+    // no CTA leaves while another may still read its shared memory
+    __syncthreads();
+    cluster_arrive();
+    cluster_wait();
+}
+
+// The cluster FP64 panel for m = n - k0 rows, wherever the rows fit the shared
+// memory of 16 SMs (complex 6.5 k rows, real 10 k: larger panels gain as
+// well, 6000 complex unknowns: panels 43 ms, with the lean form above 2500 rows
+// 53).  `applies` is false where it does not apply (PEEC_GB300_PANEL=coop / lean
+// select the other forms); false on errors.
+template <class T>
+static bool launch_cl64_panel(T *a, int n, int k0, int kb, double limit, long long *piv, Status *st, double tie,
+                              bool &applies) {
+    const int m = n - k0;
+    applies = false;
+    static const size_t kMaxSmem = 212 * 1024;
+    static const bool on = [] {
+        const char *e = getenv("PEEC_GB300_PANEL");
+        if (e && (strcmp(e, "coop") == 0 || strcmp(e, "lean") == 0)) return false;
+        cudaFuncSetAttribute(k_panel_cl64<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxSmem);
+        cudaFuncSetAttribute(k_panel_cl64<T>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(16);
+        cfg.blockDim = dim3(kClMaxThreads);
+        cfg.dynamicSmemBytes = kMaxSmem;
+        int c = 0;
+        if (cudaOccupancyMaxPotentialClusterSize(&c, k_panel_cl64<T>, &cfg) != cudaSuccess) c = 0;
+        cudaGetLastError();
+        return c >= 16;
+    }();
+    if (!on) return true;
+    const int C = m > 32 ? 16 : 1;
+    const int rows = (m + C - 1) / C, row_threads = (rows + 31) / 32 * 32;
+    const size_t smem = (size_t)rows * kPS * sizeof(T);
+    if (row_threads > kClMaxThreads || smem > kMaxSmem) return true;
+    const int parts = row_threads * 4 <= kClMaxThreads ? 4 : row_threads * 2 <= kClMaxThreads ? 2 : 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(C);
+    cfg.blockDim = dim3(row_threads * parts);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream();
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = C;
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    applies = true;
+    note_launch();
+    return cuda_ok(cudaLaunchKernelEx(&cfg, k_panel_cl64<T>, a, n, k0, kb, rows, row_threads, limit, piv, st, tie),
+                   "cluster FP64 panel launch");
+}
 
 // ---- row swaps outside the panel -------------------------------------
 static const int kLaswpCols = 32;  // columns per k_laswp block (shared memory 2 NB x 32 x 16 bytes at most)
@@ -2487,6 +2822,9 @@ static bool factor_device(T *d_a, int n, double limit, long long *d_piv, Status 
                         d_st);
     };
     auto panel = [&](int k0, int kb, double tie) -> bool {
+        bool done = false;
+        if (!launch_cl64_panel<T>(d_a, n, k0, kb, limit, d_piv, d_st, tie, done)) return false;
+        if (done) return true;
         CoopPlan<T> pl = coop_plan<T>(n - k0);
         const int lean_g = lean64_panel_ctas<T>(n - k0);
         if (lean_g > 0) {
