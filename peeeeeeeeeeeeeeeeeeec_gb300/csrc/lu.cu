@@ -13,7 +13,7 @@
 //   k_panel     factors rows k0..n-1 of columns k0..k0+NB-1 column by
 //               column: argmax (first maximum wins, as the reference), row
 //               swap inside the panel, multipliers, rank-1 update of the
-//               remaining panel columns (one CTA; k_panel_cl64 one cluster,
+//               remaining panel columns (one CTA; k_panel_cl one cluster,
 //               k_panel_lean64 and k_panel_coop one grid);
 //   k_laswp     replays the panel's row swaps on the columns left and right
 //               of the panel;
@@ -968,306 +968,62 @@ __global__ void __launch_bounds__(kLeanThreads) k_panel_lean64(T *a, int n, int 
     if (c == 0 && tid == 0) atomicExch(&ps->gen, gen0 + (unsigned)kb);
 }
 
-// ---- cluster FP32 panel (the mixed path) ---------------------------
-// The lean panel's per-column exchange still crosses the GPU: measured on
-// GB300, a release store takes ~2 us to reach pollers on other SMs, while a
-// thread-block cluster barrier takes 0.2 us and a distributed-shared-memory
-// load 0.1 us.  Here the whole panel lives in one cluster of C (1-16) CTAs,
-// one row per thread (up to 640 rows per CTA), candidates in each CTA's
-// shared memory: per column a CTA argmax, one split cluster barrier (the
-// previous column's deferred update runs between arrive and wait), the
-// winner read from its CTA's shared memory, the swap, and the multiplier
-// plus next column of every row.  Published rows are copied before the
-// deferred update; readers apply it (the row's multiplier in column kk-1
-// times the previous pivot row), exactly as the owner does.  The pivot rule
-// is the lean panel's (first maximum of |z| in FP32, lowest row on ties).
-struct ClSlot {
-    cplxf row[2][NB];   // candidate row, by column parity
-    cplxf krow[2][NB];  // row k when owned here
-    float val[2];
-    int idx[2];
-};
-
-__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
-__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
-
-static const int kClMaxThreads = 640;  // rows per CTA at most (registers: 102 a thread)
-static const int kClStride = NB + 2;   // tile row stride (complex): 16-byte aligned rows
-
-__global__ void __launch_bounds__(kClMaxThreads) k_panel_cl(cplxf *a, int n, int k0, int kb, int rows_per_cta,
-                                                            double limit, long long *piv, Status *st) {
-    pdl_wait();
-    pdl_trigger();
-    namespace cg = cooperative_groups;
-    cg::cluster_group cluster = cg::this_cluster();
-    extern __shared__ __align__(16) unsigned char cl_smem[];
-    cplxf(*tile)[kClStride] = reinterpret_cast<cplxf(*)[kClStride]>(cl_smem);  // [rows_per_cta][kClStride]
-    __shared__ ClSlot slot;
-    __shared__ __align__(16) cplxf s_prow[2][NB];
-    __shared__ float s_wv[32], s_gb;
-    __shared__ int s_wi[32], s_gc, s_p;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarps = blockDim.x >> 5;
-    const int C = (int)cluster.num_blocks(), c = (int)cluster.block_rank();
-    const int r0 = k0 + c * rows_per_cta, r1 = min(n, r0 + rows_per_cta);
-    const int nrows = r1 > r0 ? r1 - r0 : 0;
-    if (st->code != 0) return;  // uniform over the cluster (set before launch)
-    const float limf = float_at_most(limit);
-    for (int t = tid; t < nrows * kb; t += blockDim.x) {
-        const int ii = t / kb, j = t % kb;
-        tile[ii][j] = a[(size_t)(r0 + ii) * n + k0 + j];
-    }
-    __syncthreads();
-    const int i = r0 + tid;
-    const bool mine = tid < nrows;
-    cplxf *row = tile[mine ? tid : 0];
-    float mv = mine ? lean_mag(row[0], i == k0) : -1.0f;
-    cplxf mreg = {0.0f, 0.0f};
-    bool failed = false;
-    for (int kk = 0; kk < kb; ++kk) {
-        const int k = k0 + kk, par = kk & 1;
-        const cplxf *pprev = s_prow[par ^ 1];
-        // CTA candidate (largest magnitude, lowest row)
-        float bv = (mine && i >= k) ? mv : -1.0f;
-        int bi = bv >= 0.0f ? i : n;
-#pragma unroll
-        for (int sh = 16; sh > 0; sh >>= 1) {
-            const float ov = __shfl_xor_sync(0xffffffffu, bv, sh);
-            const int oi = __shfl_xor_sync(0xffffffffu, bi, sh);
-            if (ov > bv || (ov == bv && oi < bi)) {
-                bv = ov;
-                bi = oi;
-            }
-        }
-        if (lane == 0) {
-            s_wv[warp] = bv;
-            s_wi[warp] = bi;
-        }
-        __syncthreads();
-        if (warp == 0) {
-            bv = lane < nwarps ? s_wv[lane] : -1.0f;
-            bi = lane < nwarps ? s_wi[lane] : n;
-#pragma unroll
-            for (int sh = 16; sh > 0; sh >>= 1) {
-                const float ov = __shfl_xor_sync(0xffffffffu, bv, sh);
-                const int oi = __shfl_xor_sync(0xffffffffu, bi, sh);
-                if (ov > bv || (ov == bv && oi < bi)) {
-                    bv = ov;
-                    bi = oi;
-                }
-            }
-            // publish: the candidate as it is (pending the previous column's update)
-            if (lane < kb) slot.row[par][lane] = bi < n ? tile[bi - r0][lane] : cplxf{0.0f, 0.0f};
-            if (lane == 0) {
-                slot.val[par] = bi < n ? bv : -1.0f;
-                slot.idx[par] = bi;
-            }
-        }
-        if (warp == 1 && k >= r0 && k < r1 && lane < kb) slot.krow[par][lane] = tile[k - r0][lane];
-        __syncthreads();
-        cluster_arrive();
-        // the previous column's deferred update, between arrive and wait: the
-        // row in registers (16-byte shared-memory accesses, compile-time
-        // column indices), columns kk+1 .. kb-1 only
-        if (kk > 0 && mine && i >= k) {
-            float4 *r4 = reinterpret_cast<float4 *>(row);
-            const float4 *p4 = reinterpret_cast<const float4 *>(pprev);
-#pragma unroll
-            for (int q = 0; q < NB / 2; ++q) {
-                if (2 * q + 1 <= kk || 2 * q >= kb) continue;
-                float4 r = r4[q];
-                const float4 u = p4[q];
-                if (2 * q > kk) {
-                    r.x = fmaf(-mreg.re, u.x, r.x);
-                    r.x = fmaf(mreg.im, u.y, r.x);
-                    r.y = fmaf(-mreg.re, u.y, r.y);
-                    r.y = fmaf(-mreg.im, u.x, r.y);
-                }
-                if (2 * q + 1 < kb) {
-                    r.z = fmaf(-mreg.re, u.z, r.z);
-                    r.z = fmaf(mreg.im, u.w, r.z);
-                    r.w = fmaf(-mreg.re, u.w, r.w);
-                    r.w = fmaf(-mreg.im, u.z, r.w);
-                }
-                r4[q] = r;
-            }
-        }
-        __syncwarp();
-        cluster_wait();
-
-        // the winner over the cluster
-        if (warp == 0) {
-            float fv = -1.0f;
-            int fi = n, fq = -1;
-            if (lane < C) {
-                const ClSlot *rs = cluster.map_shared_rank(&slot, lane);
-                fv = rs->val[par];
-                fi = rs->idx[par];
-                fq = fi < n ? lane : -1;
-                if (fq < 0) fv = -1.0f;
-            }
-#pragma unroll
-            for (int sh = 16; sh > 0; sh >>= 1) {
-                const float ov = __shfl_xor_sync(0xffffffffu, fv, sh);
-                const int oi = __shfl_xor_sync(0xffffffffu, fi, sh);
-                const int oq = __shfl_xor_sync(0xffffffffu, fq, sh);
-                if (oq >= 0 && (fq < 0 || ov > fv || (ov == fv && oi < fi))) {
-                    fv = ov;
-                    fi = oi;
-                    fq = oq;
-                }
-            }
-            if (lane == 0) {
-                s_gc = fq;
-                s_gb = fv;
-                s_p = fi;
-            }
-        }
-        __syncthreads();
-        const int gc = s_gc, p = s_p;
-        const float gb = s_gb;
-        if (gc < 0 || !isfinite(gb) || gb <= limf) {
-            if (c == 0 && tid == 0) {
-                st->code = 2;
-                st->column = k;
-                st->value = gc < 0 ? -1.0 : (double)gb;
-            }
-            failed = true;
-            break;  // uniform over the cluster: every CTA read the same slots
-        }
-        // the pivot row, and row k for the owner of p, with the pending update
-        cplxf *pcur = s_prow[par];
-        cplxf kval = {0.0f, 0.0f};
-        if (warp == 0 && lane < kb) {
-            const ClSlot *ws = cluster.map_shared_rank(&slot, gc);
-            cplxf v = ws->row[par][lane];
-            if (kk > 0 && lane > kk) v = msub(v, ws->row[par][kk - 1], pprev[lane]);
-            pcur[lane] = v;
-        }
-        if (warp == 1 && gc == c && p != k && lane < kb) {
-            const ClSlot *ks = cluster.map_shared_rank(&slot, (k - k0) / rows_per_cta);
-            kval = ks->krow[par][lane];
-            if (kk > 0 && lane > kk) kval = msub(kval, ks->krow[par][kk - 1], pprev[lane]);
-        }
-        __syncthreads();
-        if (p != k) {
-            if (warp == 0 && k >= r0 && k < r1 && lane < kb) tile[k - r0][lane] = pcur[lane];
-            if (warp == 1 && gc == c && lane < kb) tile[p - r0][lane] = kval;
-        }
-        if (c == 0 && tid == 0) piv[k] = p;
-        __syncthreads();
-        if (k + 1 >= n) break;
-        if (mine && i > k) {
-            const cplxf pv = pcur[kk];
-            const float den = pv.re * pv.re + pv.im * pv.im;
-            const cplxf inv = {pv.re / den, -pv.im / den};
-            const cplxf x = row[kk];
-            mreg = cplxf{x.re * inv.re - x.im * inv.im, x.re * inv.im + x.im * inv.re};
-            row[kk] = mreg;
-            if (kk + 1 < kb) {
-                row[kk + 1] = msub(row[kk + 1], mreg, pcur[kk + 1]);
-                mv = lean_mag(row[kk + 1], i == k + 1);
-            } else {
-                mv = -1.0f;
-            }
-        } else {
-            mv = -1.0f;
-        }
-    }
-    if (!failed) {
-        __syncthreads();
-        for (int t = tid; t < nrows * kb; t += blockDim.x) {
-            const int ii = t / kb, j = t % kb;
-            a[(size_t)(r0 + ii) * n + k0 + j] = tile[ii][j];
-        }
-    }
-    // no CTA leaves while another may still read its shared memory
-    __syncthreads();
-    cluster_arrive();
-    cluster_wait();
-}
-
-
-// Cluster FP32 panel for m rows: one CTA up to 640 rows, else C = 16 CTAs
-// (8 where 16 is not available), one row per thread; false when it does
-// not apply.
-static bool launch_cl_panel(cplxf *a, int n, int k0, int kb, double limit, long long *piv, Status *st) {
-    const int m = n - k0;
-    if (m < 1) return false;
-    static const size_t kMaxSmem = 200 * 1024;
-    static const int max_c = [] {
-        cudaFuncSetAttribute(k_panel_cl, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxSmem);
-        cudaFuncSetAttribute(k_panel_cl, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3(16);
-        cfg.blockDim = dim3(kClMaxThreads);
-        cfg.dynamicSmemBytes = kMaxSmem;
-        cudaLaunchAttribute at[1];
-        at[0].id = cudaLaunchAttributeClusterDimension;
-        at[0].val.clusterDim.x = 16;
-        at[0].val.clusterDim.y = 1;
-        at[0].val.clusterDim.z = 1;
-        cfg.attrs = at;
-        cfg.numAttrs = 1;
-        int c = 0;
-        if (cudaOccupancyMaxPotentialClusterSize(&c, k_panel_cl, &cfg) != cudaSuccess) c = 0;
-        cudaGetLastError();
-        return c >= 16 ? 16 : c >= 8 ? 8 : 0;
-    }();
-    if (max_c == 0) return false;
-    // a panel of up to kClMaxThreads rows fits one CTA: a cluster of one,
-    // whose barriers are the CTA's own (measured: the tail panels of a small
-    // system take ~30 us instead of ~240 us with the single-CTA global-
-    // memory panel, and the SMs left free serve the other streams of a
-    // batched sweep).  Larger panels take the widest cluster: intermediate
-    // sizes (2-8 CTAs) made the 8402-unknown factorisation 2 ms slower.
-    const int C = m <= kClMaxThreads ? 1 : max_c;
-    const int rows = (m + C - 1) / C;
-    if (rows > kClMaxThreads) return false;
-    const size_t smem = (size_t)rows * kClStride * sizeof(cplxf);
-    if (smem > kMaxSmem) return false;
-    const int threads = std::max(64, (rows + 31) / 32 * 32);
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(C);
-    cfg.blockDim = dim3(threads);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = stream();
-    cudaLaunchAttribute at[2];
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = C;
-    at[0].val.clusterDim.y = 1;
-    at[0].val.clusterDim.z = 1;
-    at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;  // a programmatic dependent (pdl_wait)
-    at[1].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 2;
-    note_launch();
-    return cuda_ok(cudaLaunchKernelEx(&cfg, k_panel_cl, a, n, k0, kb, rows, limit, piv, st), "cluster FP32 panel launch");
-}
-
-
-// ---- cluster FP64 panel ---------------------------------------------
-// k_panel_cl's structure for the FP64 factorisations, with k_panel_lean64's
-// arithmetic and pivots bit for bit.  Sixteen SMs share the FP64 work (84
-// instructions a row and column, complex), but a column costs one cluster
-// barrier instead of an exchange of flags through L2 (panels of a whole
-// factorisation, lean / cluster, in ms: real 833: 4.7 / 2.2, 2102: 13.2 / 5.8, 8402:
-// 47 / 35; complex 833: 9.5 / 3.4, 2102: 24.0 / 9.9, 6000: 69 / 43, 8402: 95 / 70).
-// What keeps the FP64 units (a warp instruction takes 64 cycles of its
-// scheduler) off the critical path:
-//  - magnitudes are compared as integer keys.  Complex: keys of |z|^2; the
-//    correctly rounded |z| decides only where two keys are within 16 ulps or the
-//    largest is not well inside the exponent range (exact_key: one more barrier);
-//  - the column's quotients share one correctly rounded reciprocal; two
-//    corrections by the exact remainder round each correctly (Markstein,
+// ---- cluster panel ---------------------------------------------------
+// The lean panel's per-column exchange crosses the GPU: measured on GB300, a
+// release store takes ~2 us to reach pollers on other SMs, while a thread-block
+// cluster barrier takes 0.2 us and a distributed-shared-memory load 0.1 us.
+// Here the whole panel lives in one cluster of C (1-16) CTAs, one row per lead
+// thread.  Per column: a CTA argmax, its key pushed into every CTA's inbox; one
+// split cluster barrier with the previous column's deferred row update between
+// arrive and wait; every warp finds the winner in its own shared memory; warp 0
+// fetches the pivot row from its CTA, warp 1 row k for the owner of the winner
+// (pushing the candidate rows as well, 16 x 16 of them, cost more than the
+// fetch: complex FP64 2102 unknowns 11.6 ms instead of 8.9); then the multiplier
+// and next column of every row.  Published rows are copied before the deferred
+// update; readers apply it (the row's multiplier in column kk-1 times the
+// previous pivot row), exactly as the owner does.  Pivots and arithmetic are the
+// lean panels' (first maximum of |z|, lowest row on ties).
+//
+// The panel is bound by the latency of this chain, and in FP64 by the FP64 units
+// of 16 SMs (a warp instruction takes 64 cycles of its scheduler).  So
+//  - magnitudes are compared as integer keys, a warp's by redux.  FP64 complex:
+//    keys of |z|^2; the correctly rounded |z| decides only where two keys are
+//    within 16 ulps or the largest is not well inside the exponent range
+//    (exact_key: one more barrier);
+//  - FP64 quotients share one correctly rounded reciprocal of the column (real:
+//    from more than eight warps of rows on; below, a division each is shorter);
+//    two corrections by the exact remainder round each correctly (Markstein,
 //    "Computation of elementary functions on the IBM RISC System/6000",
 //    1990), with exponents for which nothing under- or overflows;
 //  - the deferred row updates are dealt to up to four threads a row, so that
 //    every scheduler has work when a CTA holds few rows.
+// Panels of a whole factorisation, lean / cluster, in ms: real 833 unknowns 4.7 /
+// 1.9, 2102: 13.2 / 5.1, 8402: 47 / 31; complex 833: 9.5 / 3.0, 2102: 24.0 / 8.9, 6000:
+// 69 / 40, 8402: 95 / 67.  FP32 8402: 25.8 with keys fetched instead of pushed, two
+// more CTA barriers a column and shuffles for redux, now 19.7.
+static const int kClMaxThreads = 640;  // rows per CTA at most (registers: 102 a thread)
+
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+
 template <class T>
-struct Cl64Slot {
-    T row[2][NB], krow[2][NB];       // candidate row, row k when owned here; by column parity
-    unsigned long long key[2], xkey[2];
-    int idx[2], xidx[2], close[2];
+struct ClType {
+    using Key = unsigned long long;
+    static const int stride = kPS;  // of the tile's rows
+};
+template <>
+struct ClType<cplxf> {
+    using Key = unsigned;
+    static const int stride = NB + 2;  // 16-byte aligned rows
+};
+
+// by column parity: the CTA's candidate row, and row k when owned here; what the
+// CTAs of the cluster (second index) send
+template <class T>
+struct ClInbox {
+    T row[2][NB], krow[2][NB];
+    typename ClType<T>::Key key[2][16], xkey[16];
+    int idx[2][16], xidx[16], close[2][16];
 };
 
 static const unsigned long long kInfKey = (0x7ffull << 52) + 1;
@@ -1320,21 +1076,35 @@ __device__ __forceinline__ cplx divide_by(cplx a, cplx b, double den, double r) 
     return cplx{divide_by(a.re * b.re + a.im * b.im, den, r), divide_by(a.im * b.re - a.re * b.im, den, r)};
 }
 
+__device__ __forceinline__ unsigned col_key(cplxf v, bool diag) {
+    const float m = lean_mag(v, diag);
+    return m < 0.0f ? 0u : __float_as_uint(m) + 1u;
+}
+__device__ __forceinline__ void warp_top(unsigned &key, int &idx) {
+    const unsigned m = __reduce_max_sync(0xffffffffu, key);
+    idx = __reduce_min_sync(0xffffffffu, key == m ? idx : 0x7fffffff);
+    key = m;
+}
+
 template <class T>
-__global__ void __launch_bounds__(kClMaxThreads) k_panel_cl64(T *a, int n, int k0, int kb, int rows_per_cta,
-                                                              int row_threads, double limit, long long *piv,
-                                                              Status *st, double tie) {
+__global__ void __launch_bounds__(kClMaxThreads) k_panel_cl(T *a, int n, int k0, int kb, int rows_per_cta,
+                                                            int row_threads, double limit, long long *piv, Status *st,
+                                                            double tie) {
+    constexpr bool cx = std::is_same<T, cplx>::value, f32 = std::is_same<T, cplxf>::value;
+    using Key = typename ClType<T>::Key;
+    if constexpr (f32) {
+        pdl_wait();
+        pdl_trigger();
+    }
     namespace cg = cooperative_groups;
     cg::cluster_group cluster = cg::this_cluster();
-    constexpr bool cx = sizeof(T) == sizeof(cplx);
     extern __shared__ __align__(16) unsigned char cl_smem[];
-    T(*tile)[kPS] = reinterpret_cast<T(*)[kPS]>(cl_smem);  // [rows_per_cta][kPS]
-    __shared__ Cl64Slot<T> slot;
-    __shared__ T s_prow[2][NB];
-    __shared__ unsigned long long s_wu[32], s_tie;
-    __shared__ int s_wi[32], s_close[2], s_gc, s_p, s_exact, s_bad;
-    __shared__ double s_den, s_rcp, s_val;
-    __shared__ unsigned long long s_key;
+    T(*tile)[ClType<T>::stride] = reinterpret_cast<T(*)[ClType<T>::stride]>(cl_smem);  // [rows_per_cta]
+    __shared__ __align__(16) ClInbox<T> in;
+    __shared__ __align__(16) T s_prow[2][NB];
+    __shared__ Key s_wu[32];
+    __shared__ int s_wi[32], s_close[2];
+    __shared__ double s_den, s_rcp;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int parts = blockDim.x / row_threads, part = tid / row_threads, rt = tid - part * row_threads;
     const int nrw = row_threads >> 5;  // warps with part == 0
@@ -1342,23 +1112,35 @@ __global__ void __launch_bounds__(kClMaxThreads) k_panel_cl64(T *a, int n, int k
     const int r0 = k0 + c * rows_per_cta, r1 = min(n, r0 + rows_per_cta);
     const int nrows = r1 > r0 ? r1 - r0 : 0;
     if (st->code != 0) return;  // uniform over the cluster (set before launch, or after its first barrier)
-    const bool checked = __double_as_longlong(tie) != 0;
+    // keys of magnitudes <= limit; of |z|^2 that may be; near ties in ulps of the winner's key at 1.0
+    Key limit_key, square_key = 0;
+    if constexpr (f32) {
+        const float f = float_at_most(limit);
+        limit_key = f >= 0.0f ? __float_as_uint(fabsf(f)) + 1u : 0u;
+    } else {
+        limit_key = limit >= 0.0 ? (Key)__double_as_longlong(fabs(limit)) + 1 : 0;
+        if (limit >= 0.0) square_key = (Key)__double_as_longlong(limit * limit * (1.0 + 1e-9)) + 1;
+    }
+    const unsigned long long tie_ulps = (unsigned long long)ceil((cx ? 2.0 : 1.0) * tie * 4503599627370496.0);
+    const bool shared_rcp = cx || (!f32 && nrw > 8);
     for (int t = tid; t < nrows * kb; t += blockDim.x) {
         const int ii = t / kb, j = t % kb;
         tile[ii][j] = a[(size_t)(r0 + ii) * n + k0 + j];
     }
     if (tid < 2) s_close[tid] = 0;
     __syncthreads();
+    cluster_arrive();  // (every CTA runs before the first push to its inbox)
+    cluster_wait();
     const int i = r0 + rt;
     const bool mine = rt < nrows, lead = part == 0;
     T *row = tile[mine ? rt : 0];
-    unsigned long long key = lead && mine ? col_key(row[0], i == k0) : 0;
+    Key key = lead && mine ? col_key(row[0], i == k0) : 0;
     bool failed = false;
     // the CTA's largest key of `u`, in every lane of every warp
-    auto cta_top = [&](unsigned long long u, unsigned long long &bu, int &bi) {
+    auto cta_top = [&](Key u, Key &bu, int &bi) {
         if (lead) {
             int wi = i;
-            unsigned long long wu = u;
+            Key wu = u;
             warp_top(wu, wi);
             if (lane == 0) {
                 s_wu[warp] = wu;
@@ -1373,147 +1155,168 @@ __global__ void __launch_bounds__(kClMaxThreads) k_panel_cl64(T *a, int n, int k
     for (int kk = 0; kk < kb; ++kk) {
         const int k = k0 + kk, par = kk & 1;
         const T *pprev = s_prow[par ^ 1];
-        T *pcur = s_prow[par];
-        const unsigned long long u = mine && i >= k ? key : 0;
-        unsigned long long bu;
+        const Key u = mine && i >= k ? key : 0;
+        Key bu;
         int bi;
         cta_top(u, bu, bi);
-        // publish: the candidate as it is (pending the previous column's update)
+        // publish: the candidate and row k as they are (pending the previous column's update)
+        const bool own_k = k >= r0 && k < r1;
         if (warp == 0) {
-            if (lane < kb) slot.row[par][lane] = bu ? tile[bi - r0][lane] : T{};
-            if (lane == 0) {
-                slot.key[par] = bu;
-                slot.idx[par] = bi;
-                s_close[par ^ 1] = 0;
+            if (bu && lane < kb) in.row[par][lane] = tile[bi - r0][lane];
+            if (lane < C) {
+                ClInbox<T> *to = cluster.map_shared_rank(&in, lane);
+                to->key[par][c] = bu;
+                to->idx[par][c] = bi;
             }
         }
-        if (warp == 1 && k >= r0 && k < r1 && lane < kb) slot.krow[par][lane] = tile[k - r0][lane];
-        if (cx && lead && u && i != bi && bu - u <= kCloseUlps) s_close[par] = 1;
+        if (warp == 1 && own_k && lane < kb) in.krow[par][lane] = tile[k - r0][lane];
+        if (cx) {
+            if (tid == 0) s_close[par ^ 1] = 0;
+            if (lead && u && i != bi && bu - u <= kCloseUlps) s_close[par] = 1;
+        }
         __syncthreads();
-        if (cx && tid == 0) slot.close[par] = s_close[par];
+        if (cx && tid < C) cluster.map_shared_rank(&in, tid)->close[par][c] = s_close[par];
         __syncwarp();
         cluster_arrive();
-        // the previous column's deferred update, between arrive and wait
+        // the previous column's deferred update, columns kk+1 .. kb-1, between arrive and wait
         if (kk > 0 && mine && i >= k) {
             const T m = row[kk - 1];
+            if constexpr (f32) {  // two columns at a time (16-byte shared-memory accesses)
+                float4 *r4 = reinterpret_cast<float4 *>(row);
+                const float4 *p4 = reinterpret_cast<const float4 *>(pprev);
 #pragma unroll 4
-            for (int j = kk + 1 + part; j < kb; j += parts) row[j] = msub(row[j], m, pprev[j]);
-        }
-        __syncwarp();
-        cluster_wait();
-        // the winner over the cluster
-        auto cluster_top = [&](bool exact) {
-            if (warp == 0) {
-                const Cl64Slot<T> *rs = cluster.map_shared_rank(&slot, lane < C ? lane : 0);
-                const unsigned long long lu = lane < C ? (exact ? rs->xkey[par] : rs->key[par]) : 0;
-                const int li = lane < C ? (exact ? rs->xidx[par] : rs->idx[par]) : 0x7fffffff;
-                unsigned long long wu = lu;
-                int wi = li;
-                warp_top(wu, wi);
-                const bool won = lu == wu && li == wi && lane < C;
-                const unsigned who = __ballot_sync(0xffffffffu, won);
-                bool close = false;
-                if (cx && !exact)
-                    close = __any_sync(0xffffffffu, lane < C && lu && (won ? rs->close[par] != 0 : wu - lu <= kCloseUlps));
-                if (lane == 0) {
-                    s_gc = wu ? __ffs(who) - 1 : -1;
-                    s_p = wi;
-                    s_key = wu;
-                    s_exact = cx && !exact && wu && (close || wide_key(wu));
+                for (int q = ((kk + 1) >> 1) + part; 2 * q < kb; q += parts) {
+                    float4 r = r4[q];
+                    const float4 w = p4[q];
+                    if (2 * q > kk) {
+                        r.x = fmaf(-m.re, w.x, r.x);
+                        r.x = fmaf(m.im, w.y, r.x);
+                        r.y = fmaf(-m.re, w.y, r.y);
+                        r.y = fmaf(-m.im, w.x, r.y);
+                    }
+                    if (2 * q + 1 < kb) {
+                        r.z = fmaf(-m.re, w.z, r.z);
+                        r.z = fmaf(m.im, w.w, r.z);
+                        r.w = fmaf(-m.re, w.w, r.w);
+                        r.w = fmaf(-m.im, w.z, r.w);
+                    }
+                    r4[q] = r;
                 }
+            } else {
+#pragma unroll 4
+                for (int j = kk + 1 + part; j < kb; j += parts) row[j] = msub(row[j], m, pprev[j]);
             }
-            __syncthreads();
-        };
-        cluster_top(false);
-        bool pending = kk > 0;  // is the published row short of the previous column's update?
-        const bool exact = s_exact;
-        if (exact) {  // uniform over the cluster: every CTA read the same slots
-            const unsigned long long x = lead && u ? exact_key(row[kk], i == k) : 0;
-            cta_top(x, bu, bi);
-            if (warp == 0) {
-                if (lane < kb) slot.row[par][lane] = bu ? tile[bi - r0][lane] : T{};
-                if (lane == 0) {
-                    slot.xkey[par] = bu;
-                    slot.xidx[par] = bi;
-                }
-            }
-            __syncthreads();
-            cluster_arrive();
-            cluster_wait();
-            cluster_top(true);
-            pending = false;
-        }
-        const int gc = s_gc, p = s_p;
-        // the pivot row, and row k for the owner of p, with the pending update
-        T kval = T{};
-        if (warp == 0) {
-            if (gc >= 0) {
-                const Cl64Slot<T> *ws = cluster.map_shared_rank(&slot, gc);
-                if (lane < kb) {
-                    T v = ws->row[par][lane];
-                    if (pending && lane > kk) v = msub(v, ws->row[par][kk - 1], pprev[lane]);
-                    pcur[lane] = v;
-                }
-                __syncwarp();
-            }
-            const T pv = gc >= 0 ? pcur[kk] : T{};
-            const double den = divisor(pv);
-            // pivot check by the exact magnitude, unless |z|^2 is clear of it
-            const unsigned long long wk = s_key;
-            double gb = -1.0;
-            bool bad = gc < 0;
-            if (!bad) {
-                const double v = __longlong_as_double((long long)(wk - 1));
-                if (cx && !exact && v > limit * limit * (1.0 + 1e-9)) {
-                    gb = INFINITY;  // not needed
-                } else {
-                    gb = cx && !exact ? mag(pv) : v;
-                    bad = !isfinite(gb) || gb <= limit;
-                }
-            }
-            if (lane == 0) {
-                s_bad = bad;
-                s_val = gb;
-                s_den = den;
-                s_rcp = 1.0 / den;
-                if (checked) {  // keys from here on are near ties (twice the fraction for |z|^2)
-                    const unsigned long long pk = col_key(pv, true);
-                    const double v = __longlong_as_double((long long)(pk - 1));
-                    const unsigned long long b = (unsigned long long)tie_limit(v, cx ? 2.0 * tie : tie);
-                    s_tie = b > kCloseUlps ? b + 1 - kCloseUlps : 1;
-                }
-            }
-        }
-        if (warp == 1 && gc == c && p != k && lane < kb) {
-            const Cl64Slot<T> *ks = cluster.map_shared_rank(&slot, (k - k0) / rows_per_cta);
-            kval = ks->krow[par][lane];
-            if (kk > 0 && lane > kk) kval = msub(kval, ks->krow[par][kk - 1], pprev[lane]);
         }
         __syncthreads();
-        if (s_bad) {  // uniform over the cluster
+        cluster_wait();
+        // the winner over the cluster, in every warp
+        Key wu = lane < C ? in.key[par][lane] : 0;
+        int p = lane < C ? in.idx[par][lane] : 0x7fffffff;
+        Key lu = wu;
+        int li = p;
+        warp_top(wu, p);
+        int gc = __ffs(__ballot_sync(0xffffffffu, lane < C && lu == wu && li == p)) - 1;
+        bool pending = kk > 0, exact = false;  // pending: the candidate rows lack the previous column's update
+        if constexpr (cx) {
+            exact = wu && (wide_key(wu) || __any_sync(0xffffffffu, lane < C && lu &&
+                                                                       (lane == gc ? in.close[par][lane] != 0
+                                                                                   : wu - lu <= kCloseUlps)));
+            if (exact) {  // uniform over the cluster: every CTA was sent the same keys
+                const Key x = lead && u ? exact_key(row[kk], i == k) : 0;
+                cta_top(x, bu, bi);
+                if (warp == 0) {
+                    if (bu && lane < kb) in.row[par][lane] = tile[bi - r0][lane];
+                    if (lane < C) {
+                        ClInbox<T> *to = cluster.map_shared_rank(&in, lane);
+                        to->xkey[c] = bu;
+                        to->xidx[c] = bi;
+                    }
+                }
+                __syncwarp();
+                cluster_arrive();
+                cluster_wait();
+                lu = wu = lane < C ? in.xkey[lane] : 0;
+                li = p = lane < C ? in.xidx[lane] : 0x7fffffff;
+                warp_top(wu, p);
+                gc = __ffs(__ballot_sync(0xffffffffu, lane < C && lu == wu && li == p)) - 1;
+                pending = false;
+            }
+        }
+        const T *wr = cluster.map_shared_rank(&in, gc < 0 ? 0 : gc)->row[par];
+        bool bad;
+        if constexpr (f32)
+            bad = wu == 0 || wu >= 0x7f800001u || wu <= limit_key;
+        else
+            bad = wu == 0 || wu >= kInfKey || wu <= (!cx || exact ? limit_key : square_key);
+        double gb = -1.0;
+        if (bad && wu) {
+            if constexpr (f32) {
+                gb = (double)__uint_as_float(wu - 1u);
+            } else {
+                gb = !cx || exact ? __longlong_as_double((long long)(wu - 1)) : mag(wr[kk]);
+                bad = !isfinite(gb) || gb <= limit;
+            }
+        }
+        if (bad) {  // uniform over the cluster
             if (c == 0 && tid == 0) {
                 st->code = 2;
                 st->column = k;
-                st->value = s_val;
+                st->value = gb;
             }
             failed = true;
             break;
         }
-        if (checked && lead && u >= s_tie && i != p) atomicCAS(&st->code, 0, 7);
-        if (p != k) {
-            if (warp == 0 && k >= r0 && k < r1 && lane < kb) tile[k - r0][lane] = pcur[lane];
-            if (warp == 1 && gc == c && lane < kb) tile[p - r0][lane] = kval;
+        if constexpr (!f32)
+            if (tie_ulps && lead && u && i != p) {
+                const Key top = exact ? col_key(wr[kk], true) : wu;
+                const Key margin = tie_ulps + __umul64hi((top - 1) << 12, tie_ulps) + kCloseUlps;
+                if (u + margin >= top) atomicCAS(&st->code, 0, 7);
+            }
+        T *pcur = s_prow[par];
+        if (warp == 0) {  // the pivot row
+            if (lane < kb) {
+                T v = wr[lane];
+                if (pending && lane > kk) v = msub(v, wr[kk - 1], pprev[lane]);
+                pcur[lane] = v;
+                if (p != k && own_k) tile[k - r0][lane] = v;
+            }
+            __syncwarp();
+            if constexpr (!f32)
+                if (shared_rcp) {
+                    const double den = divisor(pcur[kk]);
+                    if (lane == 0) {
+                        s_den = den;
+                        s_rcp = 1.0 / den;
+                    }
+                }
+            if (c == 0 && lane == 0) piv[k] = p;
         }
-        if (c == 0 && tid == 0) piv[k] = p;
+        if (warp == 1 && gc == c && p != k && lane < kb) {
+            const T *kr = cluster.map_shared_rank(&in, (k - k0) / rows_per_cta)->krow[par];
+            T v = kr[lane];
+            if (kk > 0 && lane > kk) v = msub(v, kr[kk - 1], pprev[lane]);
+            tile[p - r0][lane] = v;
+        }
         __syncthreads();
         if (k + 1 >= n) break;
         key = 0;
         if (lead && mine && i > k) {
-            const T m = divide_by(row[kk], pcur[kk], s_den, s_rcp);
+            const bool next = kk + 1 < kb;
+            const T x0 = row[kk];
+            T m;
+            if constexpr (f32) {
+                const T pv = pcur[kk];
+                const float den = pv.re * pv.re + pv.im * pv.im;
+                const cplxf inv = {pv.re / den, -pv.im / den};
+                m = cplxf{x0.re * inv.re - x0.im * inv.im, x0.re * inv.im + x0.im * inv.re};
+            } else {
+                m = shared_rcp ? divide_by(x0, pcur[kk], s_den, s_rcp) : divide(x0, pcur[kk]);
+            }
             row[kk] = m;
-            if (kk + 1 < kb) {
-                row[kk + 1] = msub(row[kk + 1], m, pcur[kk + 1]);
-                key = col_key(row[kk + 1], i == k + 1);
+            if (next) {
+                const T x1 = msub(row[kk + 1], m, pcur[kk + 1]);
+                row[kk + 1] = x1;
+                key = col_key(x1, i == k + 1);
             }
         }
     }
@@ -1524,60 +1327,82 @@ __global__ void __launch_bounds__(kClMaxThreads) k_panel_cl64(T *a, int n, int k
             a[(size_t)(r0 + ii) * n + k0 + j] = tile[ii][j];
         }
     }
-    // no CTA leaves while another may still read its shared memory
+    // no CTA leaves while another may still write to its shared memory
     __syncthreads();
     cluster_arrive();
     cluster_wait();
 }
 
-// The cluster FP64 panel for m = n - k0 rows, wherever the rows fit the shared
-// memory of 16 SMs (complex 6.5 k rows, real 10 k: larger panels gain as
-// well, 6000 complex unknowns: panels 43 ms, with the lean form above 2500 rows
-// 53).  `applies` is false where it does not apply (PEEC_GB300_PANEL=coop / lean
-// select the other forms); false on errors.
+// CTAs of the widest cluster available (16, 8 or 0)
 template <class T>
-static bool launch_cl64_panel(T *a, int n, int k0, int kb, double limit, long long *piv, Status *st, double tie,
-                              bool &applies) {
-    const int m = n - k0;
-    applies = false;
-    static const size_t kMaxSmem = 212 * 1024;
-    static const bool on = [] {
-        const char *e = getenv("PEEC_GB300_PANEL");
-        if (e && (strcmp(e, "coop") == 0 || strcmp(e, "lean") == 0)) return false;
-        cudaFuncSetAttribute(k_panel_cl64<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxSmem);
-        cudaFuncSetAttribute(k_panel_cl64<T>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+static const size_t kClMaxSmem = std::is_same<T, cplx>::value ? 206 * 1024 : 200 * 1024;
+template <class T>
+static int cl_widest() {
+    static const int widest = [] {
+        cudaFuncSetAttribute(k_panel_cl<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kClMaxSmem<T>);
+        cudaFuncSetAttribute(k_panel_cl<T>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3(16);
         cfg.blockDim = dim3(kClMaxThreads);
-        cfg.dynamicSmemBytes = kMaxSmem;
+        cfg.dynamicSmemBytes = kClMaxSmem<T>;
+        cudaLaunchAttribute at[1];
+        at[0].id = cudaLaunchAttributeClusterDimension;
+        at[0].val.clusterDim.x = 16;
+        at[0].val.clusterDim.y = 1;
+        at[0].val.clusterDim.z = 1;
+        cfg.attrs = at;
+        cfg.numAttrs = 1;
         int c = 0;
-        if (cudaOccupancyMaxPotentialClusterSize(&c, k_panel_cl64<T>, &cfg) != cudaSuccess) c = 0;
+        if (cudaOccupancyMaxPotentialClusterSize(&c, k_panel_cl<T>, &cfg) != cudaSuccess) c = 0;
         cudaGetLastError();
-        return c >= 16;
+        return c >= 16 ? 16 : c >= 8 ? 8 : 0;
     }();
-    if (!on) return true;
-    const int C = m > 32 ? 16 : 1;
+    return widest;
+}
+
+// Rows up to which one CTA is the faster form: its barriers are the CTA's own, and
+// the SMs left free serve the other streams of a batched sweep (FP32, up to 640 /
+// up to 320 rows: panels of 8 systems of 777 unknowns 12.5 / 10.3 ms, of one of 8402
+// 20.1 / 19.7).  FP64 panels want the FP64 units of more SMs at once.
+template <class T>
+static const int kClOne = std::is_same<T, cplxf>::value ? 320 : 32;
+
+// The cluster panel for m = n - k0 rows, wherever the rows fit the shared memory
+// of the cluster (of 16: FP64 complex 6.3 k rows, FP64 real and FP32 10 k; large
+// panels gain as well, 6000 complex unknowns: FP64 panels 40 ms, with the lean
+// form above 2500 rows 52).  `applies` is false where it does not apply; false on errors.
+template <class T>
+static bool launch_cl_panel(T *a, int n, int k0, int kb, double limit, long long *piv, Status *st, double tie,
+                            bool &applies) {
+    constexpr bool f32 = std::is_same<T, cplxf>::value;
+    applies = false;
+    const int m = n - k0, widest = cl_widest<T>();
+    if (m < 1 || widest == 0) return true;
+    const int C = m <= kClOne<T> ? 1 : widest;
     const int rows = (m + C - 1) / C, row_threads = (rows + 31) / 32 * 32;
-    const size_t smem = (size_t)rows * kPS * sizeof(T);
-    if (row_threads > kClMaxThreads || smem > kMaxSmem) return true;
+    const size_t smem = (size_t)rows * ClType<T>::stride * sizeof(T);
+    if (row_threads > kClMaxThreads || smem > kClMaxSmem<T>) return true;
     const int parts = row_threads * 4 <= kClMaxThreads ? 4 : row_threads * 2 <= kClMaxThreads ? 2 : 1;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(C);
     cfg.blockDim = dim3(row_threads * parts);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream();
-    cudaLaunchAttribute at[1];
+    cudaLaunchAttribute at[2];
     at[0].id = cudaLaunchAttributeClusterDimension;
     at[0].val.clusterDim.x = C;
     at[0].val.clusterDim.y = 1;
     at[0].val.clusterDim.z = 1;
+    at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;  // a programmatic dependent (pdl_wait)
+    at[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = f32 ? 2 : 1;
     applies = true;
     note_launch();
-    return cuda_ok(cudaLaunchKernelEx(&cfg, k_panel_cl64<T>, a, n, k0, kb, rows, row_threads, limit, piv, st, tie),
-                   "cluster FP64 panel launch");
+    return cuda_ok(cudaLaunchKernelEx(&cfg, k_panel_cl<T>, a, n, k0, kb, rows, row_threads, limit, piv, st, tie),
+                   "cluster panel launch");
 }
+
 
 // ---- row swaps outside the panel -------------------------------------
 static const int kLaswpCols = 32;  // columns per k_laswp block (shared memory 2 NB x 32 x 16 bytes at most)
@@ -2681,6 +2506,16 @@ static int lean_panel_ctas(int m) {
     return g <= cap && g <= 32 * kLeanPoll ? g : 0;
 }
 
+// The FP64 panels: the cluster panel where it fits, else the lean one, else the
+// cooperative one.  PEEC_GB300_PANEL=lean / coop selects a form.
+static bool cl64_enabled() {
+    static const bool on = [] {
+        const char *e = getenv("PEEC_GB300_PANEL");
+        return !(e && (strcmp(e, "lean") == 0 || strcmp(e, "coop") == 0));
+    }();
+    return on;
+}
+
 // CTAs of the lean FP64 panel (k_panel_lean64) for m rows, 0 where it does
 // not apply (PEEC_GB300_PANEL=coop selects the cooperative grid panel).
 template <class T>
@@ -2823,7 +2658,7 @@ static bool factor_device(T *d_a, int n, double limit, long long *d_piv, Status 
     };
     auto panel = [&](int k0, int kb, double tie) -> bool {
         bool done = false;
-        if (!launch_cl64_panel<T>(d_a, n, k0, kb, limit, d_piv, d_st, tie, done)) return false;
+        if (cl64_enabled() && !launch_cl_panel<T>(d_a, n, k0, kb, limit, d_piv, d_st, tie, done)) return false;
         if (done) return true;
         CoopPlan<T> pl = coop_plan<T>(n - k0);
         const int lean_g = lean64_panel_ctas<T>(n - k0);
@@ -4402,7 +4237,9 @@ int mixed_solve_impl(const Complex *d_Z, size_t n_, const Complex *d_b, Complex 
                 tm.mark(2);
                 CoopPlan<cplxf> pl = coop_plan<cplxf>(n - k0);
                 const int lean_g = lean_panel_ctas(n - k0);
-                if (cl_panel_enabled() && launch_cl_panel(a, n, k0, kb, limit, piv.p, st.p)) {
+                bool done = false;
+                if (cl_panel_enabled() && !launch_cl_panel<cplxf>(a, n, k0, kb, limit, piv.p, st.p, 0.0, done)) return -1;
+                if (done) {
                 } else if (lean_g > 0) {
                     Status *stp = st.p;
                     long long *pivp = piv.p;
