@@ -20,6 +20,7 @@
 #include <math.h>
 #include <string.h>
 
+#include <algorithm>
 #include <functional>
 #include <vector>
 
@@ -241,100 +242,120 @@ __device__ __forceinline__ void pair_mac(float2 &s, float2 a, float2 b) {
     s.y += e + err;
 }
 
-// out[r] = sum_j row[j] v[r][j] (j < n) for every run r < R, by the whole
-// warp (every lane returns the sums).  Each lane reads two elements at a
-// time (16 B) and keeps up to 8 such loads in flight (4 KB per warp and
-// iteration), so the memory system, not each warp's load-to-use latency,
-// sets the pace.  v: run r's vector at v + r ldv (float pairs); ALIGNED:
-// row and v + r ldv 16-byte aligned and n even (M^-1's padded layout), the
-// vector then read two pairs at a time too.
-template <int R, bool ALIGNED = false>
-__device__ __forceinline__ void row_dot_df(const float2 *row, int n, const float2 *v, size_t ldv, int lane,
-                                           double *out) {
+// A step streams its matrices once (0.24 ms of HBM time at 8402 unknowns), but
+// every row also meets the vectors of all runs (8 bytes an element and run: they
+// do not fit L1 together), and an element costs 12 FP32 instructions a run.  So
+// a warp takes two rows against each vector load, and the kernels are
+// instantiated for exactly 1, 2, 3, 4, 6 or 8 runs (from 6 on: one row, for the registers).
+// 8402 unknowns, 3 runs: one row a warp and 4 runs 0.69 ms a step, now
+// 0.51; 1 run 0.35 and 0.34 (one row: two cost 10 % there), 2: 0.42 and 0.38, 4: 0.71
+// and 0.62, 8: 1.55 and 1.35 (CTAs of 128 threads instead of 256); four rows a
+// warp: 3 runs 0.60.
+template <int R>
+static constexpr int kRows = R == 1 || R >= 6 ? 1 : 2;
+static const int kStepWarps = 4;  // of a CTA
+
+// out[q][r] = sum_j row_q[j] v[r][j] (j < n) for the ROWS rows at `row` (`next`
+// elements apart) and every run r < R, by the whole warp (every lane returns the
+// sums).  Each lane reads two elements at a time (16 B) and keeps up to 8 such
+// loads in flight (4 KB per warp and iteration), so the memory system, not each
+// warp's load-to-use latency, sets the pace.  v: run r's vector at v + r ldv
+// (float pairs); rows and v + r ldv 16-byte aligned and n even (the padded
+// layouts).
+template <int R, int ROWS>
+__device__ __forceinline__ void row_dot_df(const float2 *row, size_t next, int n, const float2 *v, size_t ldv, int lane,
+                                           double (*out)[R]) {
     // loads in flight: fewer with more runs, whose products give each load
     // more work (and whose accumulators need the registers)
-    constexpr int kDotDepth = R >= 8 ? 4 : 8;
-    float2 acc[2][R];
+    constexpr int kDotDepth = R >= 6 ? 4 : 8;  // blocks of 64 elements an iteration
+    constexpr int kBatch = kDotDepth / ROWS;
+    float2 acc[ROWS][2][R];
 #pragma unroll
-    for (int r = 0; r < R; ++r) acc[0][r] = acc[1][r] = make_float2(0.0f, 0.0f);
-    // 16-byte loads start at the first 16-byte aligned element of the row
-    const int head = n > 0 && (reinterpret_cast<uintptr_t>(row) & 8) ? 1 : 0;
-    if (head && lane == 0) {
+    for (int q = 0; q < ROWS; ++q)
 #pragma unroll
-        for (int r = 0; r < R; ++r) pair_mac(acc[0][r], row[0], v[(size_t)r * ldv]);
-    }
-    const int body = (n - head) / 2;  // float4 pairs of elements after the head
-    const float4 *row4 = reinterpret_cast<const float4 *>(row + head);
+        for (int r = 0; r < R; ++r) acc[q][0][r] = acc[q][1][r] = make_float2(0.0f, 0.0f);
+    const int body = n / 2;
     int t = lane;
     for (; t + 32 * (kDotDepth - 1) < body; t += 32 * kDotDepth) {
-        float4 m[kDotDepth];
 #pragma unroll
-        for (int u = 0; u < kDotDepth; ++u) m[u] = __ldcs(row4 + t + 32 * u);
+        for (int h = 0; h < kDotDepth; h += kBatch) {
+            float4 m[ROWS][kBatch];
 #pragma unroll
-        for (int u = 0; u < kDotDepth; ++u) {
-            const int j = head + 2 * (t + 32 * u);
+            for (int q = 0; q < ROWS; ++q)
 #pragma unroll
-            for (int r = 0; r < R; ++r) {
-                const float2 *vr = v + (size_t)r * ldv + j;
-                if constexpr (ALIGNED) {  // both pairs in one 16-byte load
-                    const float4 w = *reinterpret_cast<const float4 *>(vr);
-                    pair_mac(acc[u & 1][r], make_float2(m[u].x, m[u].y), make_float2(w.x, w.y));
-                    pair_mac(acc[u & 1][r], make_float2(m[u].z, m[u].w), make_float2(w.z, w.w));
-                } else {
-                    pair_mac(acc[u & 1][r], make_float2(m[u].x, m[u].y), vr[0]);
-                    pair_mac(acc[u & 1][r], make_float2(m[u].z, m[u].w), vr[1]);
+                for (int u = 0; u < kBatch; ++u)
+                    m[q][u] = __ldcs(reinterpret_cast<const float4 *>(row + q * next) + t + 32 * (h + u));
+#pragma unroll
+            for (int u = 0; u < kBatch; ++u)
+#pragma unroll
+                for (int r = 0; r < R; ++r) {
+                    const float4 w = reinterpret_cast<const float4 *>(v + (size_t)r * ldv)[t + 32 * (h + u)];
+#pragma unroll
+                    for (int q = 0; q < ROWS; ++q) {
+                        pair_mac(acc[q][u & 1][r], make_float2(m[q][u].x, m[q][u].y), make_float2(w.x, w.y));
+                        pair_mac(acc[q][u & 1][r], make_float2(m[q][u].z, m[q][u].w), make_float2(w.z, w.w));
+                    }
                 }
-            }
         }
     }
     for (; t < body; t += 32) {
-        const float4 m = __ldcs(row4 + t);
-        const int j = head + 2 * t;
+        float4 m[ROWS];
+#pragma unroll
+        for (int q = 0; q < ROWS; ++q) m[q] = __ldcs(reinterpret_cast<const float4 *>(row + q * next) + t);
 #pragma unroll
         for (int r = 0; r < R; ++r) {
-            const float2 *vr = v + (size_t)r * ldv + j;
-            pair_mac(acc[0][r], make_float2(m.x, m.y), vr[0]);
-            pair_mac(acc[0][r], make_float2(m.z, m.w), vr[1]);
+            const float4 w = reinterpret_cast<const float4 *>(v + (size_t)r * ldv)[t];
+#pragma unroll
+            for (int q = 0; q < ROWS; ++q) {
+                pair_mac(acc[q][0][r], make_float2(m[q].x, m[q].y), make_float2(w.x, w.y));
+                pair_mac(acc[q][0][r], make_float2(m[q].z, m[q].w), make_float2(w.z, w.w));
+            }
         }
     }
-    const int tail = head + 2 * body;  // one element left when n - head is odd
-    if (tail < n && lane == 1) {
 #pragma unroll
-        for (int r = 0; r < R; ++r) pair_mac(acc[1][r], row[tail], v[(size_t)r * ldv + tail]);
-    }
+    for (int q = 0; q < ROWS; ++q)
 #pragma unroll
-    for (int r = 0; r < R; ++r)
-        out[r] = warp_sum(((double)acc[0][r].x + (double)acc[1][r].x) + ((double)acc[0][r].y + (double)acc[1][r].y));
+        for (int r = 0; r < R; ++r)
+            out[q][r] = warp_sum(((double)acc[q][0][r].x + (double)acc[q][1][r].x) +
+                                 ((double)acc[q][0][r].y + (double)acc[q][1][r].y));
+}
+
+// a warp's first row, and the distance to its second (0 where there is none)
+template <int R>
+__device__ __forceinline__ int step_row(int rows, int &more) {
+    const int i = (blockIdx.x * kStepWarps + (threadIdx.x >> 5)) * kRows<R>;
+    more = kRows<R> > 1 && i + 1 < rows ? 1 : 0;
+    return i;
 }
 
 // Right-hand side of one step for every run (transient.c:1421-1631, edge
 // voltages absent): blocks [0, eb) take the edge rows, one warp per row and
 // all runs; the rest the (node, run) pairs.
 template <int R>
-__global__ void __launch_bounds__(256) k_transient_rhs(StepArgs A, int eb) {
+__global__ void __launch_bounds__(32 * kStepWarps) k_transient_rhs(StepArgs A, int eb) {
     pdl_wait();
     pdl_trigger();
     const double omt = 1.0 - A.theta;
     const int nt = A.ne + A.nv;
     if (blockIdx.x == 0 && A.probes && A.record_row >= 0) record_probes(A, A.record_row);
     if ((int)blockIdx.x < eb) {
-        const int i = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+        const int lane = threadIdx.x & 31;
+        int more, i = step_row<R>(A.ne, more);
         if (i >= A.ne) return;
-        double s[R], sa[R];
-        row_dot_df<R, true>(A.Lf + (size_t)i * A.lde, A.lde, A.xI, A.lde, lane, s);
+        double s[kRows<R>][R], sa[kRows<R>][R] = {};
+        row_dot_df<R, kRows<R>>(A.Lf + (size_t)i * A.lde, (size_t)more * A.lde, A.lde, A.xI, A.lde, lane, s);
         if (omt != 0.0)
-            row_dot_df<R, true>(A.ASf + (size_t)i * A.ldn, A.ldn, A.xV, A.ldn, lane, sa);
-        else
+            row_dot_df<R, kRows<R>>(A.ASf + (size_t)i * A.ldn, (size_t)more * A.ldn, A.ldn, A.xV, A.ldn, lane, sa);
 #pragma unroll
-            for (int r = 0; r < R; ++r) sa[r] = 0.0;
+        for (int q = 0; q < kRows<R>; ++q, ++i)
 #pragma unroll
-        for (int r = 0; r < R; ++r) {
-            const double ls = s[r], as = sa[r];
-            if (lane == 0 && r < A.nrun) {
-                const double *I = A.x + (size_t)r * nt;
-                A.rhs[(size_t)r * nt + i] = ls / A.dt - omt * A.R[i] * I[i] - omt * as;
+            for (int r = 0; r < R; ++r) {
+                const double ls = s[q][r], as = sa[q][r];
+                if (lane == 0 && r < A.nrun && q <= more) {
+                    const double *I = A.x + (size_t)r * nt;
+                    A.rhs[(size_t)r * nt + i] = ls / A.dt - omt * A.R[i] * I[i] - omt * as;
+                }
             }
-        }
         return;
     }
     const int t = (blockIdx.x - eb) * blockDim.x + threadIdx.x;
@@ -366,20 +387,24 @@ __global__ void __launch_bounds__(256) k_transient_rhs(StepArgs A, int eb) {
 }
 
 // y[r][i] = y0[r][i] (when set) + sum_q Minv[i][q] v[r][q] for every run,
-// one warp per row of M^-1 (streamed once for all runs); vs: v as float
+// M^-1 streamed once for all runs; vs: v as float
 // pairs (k_split_rows), [run][ldm] with zero padding.
 template <int R>
-__global__ void __launch_bounds__(256) k_minv_apply(const float2 *Minv, int nt, int ldm, const float2 *vs,
+__global__ void __launch_bounds__(32 * kStepWarps) k_minv_apply(const float2 *Minv, int nt, int ldm, const float2 *vs,
                                                     const double *y0, double *y, int nrun) {
     pdl_wait();
     pdl_trigger();
-    const int i = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    const int lane = threadIdx.x & 31;
+    int more, i = step_row<R>(nt, more);
     if (i >= nt) return;
-    double s[R];
-    row_dot_df<R, true>(Minv + (size_t)i * ldm, ldm, vs, ldm, lane, s);
+    double s[kRows<R>][R];
+    row_dot_df<R, kRows<R>>(Minv + (size_t)i * ldm, (size_t)more * ldm, ldm, vs, ldm, lane, s);
 #pragma unroll
-    for (int r = 0; r < R; ++r)
-        if (lane == 0 && r < nrun) y[(size_t)r * nt + i] = (y0 ? y0[(size_t)r * nt + i] : 0.0) + s[r];
+    for (int q = 0; q < kRows<R>; ++q, ++i)
+#pragma unroll
+        for (int r = 0; r < R; ++r)
+            if (lane == 0 && r < nrun && q <= more)
+                y[(size_t)r * nt + i] = (y0 ? y0[(size_t)r * nt + i] : 0.0) + s[q][r];
 }
 
 // out[r] = sum_j row[j] v[r][j] (j < n) in FP32 (FP64 across the warp),
@@ -388,91 +413,102 @@ __global__ void __launch_bounds__(256) k_minv_apply(const float2 *Minv, int nt, 
 // apply streams half the bytes (the high parts alone).  row and v + r ldv
 // 16-byte aligned, n a multiple of 4 (M^-1's padded layout): matrix and
 // vector are read four elements at a time.
-template <int R>
-__device__ __forceinline__ void row_dot_f32(const float *row, int n, const float *v, size_t ldv, int lane,
-                                            double *out) {
-    float acc[2][R];
+template <int R, int ROWS>
+__device__ __forceinline__ void row_dot_f32(const float *row, size_t next, int n, const float *v, size_t ldv, int lane,
+                                            double (*out)[R]) {
+    float acc[ROWS][2][R];
 #pragma unroll
-    for (int r = 0; r < R; ++r) acc[0][r] = acc[1][r] = 0.0f;
+    for (int q = 0; q < ROWS; ++q)
+#pragma unroll
+        for (int r = 0; r < R; ++r) acc[q][0][r] = acc[q][1][r] = 0.0f;
     const int body = n / 4;
-    const float4 *row4 = reinterpret_cast<const float4 *>(row);
     constexpr int kDepth = 4;
+    auto mac = [](float a, const float4 m, const float4 w) {
+        a = fmaf(m.x, w.x, a);
+        a = fmaf(m.y, w.y, a);
+        a = fmaf(m.z, w.z, a);
+        return fmaf(m.w, w.w, a);
+    };
     int t = lane;
     for (; t + 32 * (kDepth - 1) < body; t += 32 * kDepth) {
-        float4 m[kDepth];
+        float4 m[ROWS][kDepth];
 #pragma unroll
-        for (int u = 0; u < kDepth; ++u) m[u] = __ldcs(row4 + t + 32 * u);
+        for (int q = 0; q < ROWS; ++q)
 #pragma unroll
-        for (int u = 0; u < kDepth; ++u) {
+            for (int u = 0; u < kDepth; ++u)
+                m[q][u] = __ldcs(reinterpret_cast<const float4 *>(row + q * next) + t + 32 * u);
+#pragma unroll
+        for (int u = 0; u < kDepth; ++u)
 #pragma unroll
             for (int r = 0; r < R; ++r) {
                 const float4 w = reinterpret_cast<const float4 *>(v + (size_t)r * ldv)[t + 32 * u];
-                float a = acc[u & 1][r];
-                a = fmaf(m[u].x, w.x, a);
-                a = fmaf(m[u].y, w.y, a);
-                a = fmaf(m[u].z, w.z, a);
-                a = fmaf(m[u].w, w.w, a);
-                acc[u & 1][r] = a;
+#pragma unroll
+                for (int q = 0; q < ROWS; ++q) acc[q][u & 1][r] = mac(acc[q][u & 1][r], m[q][u], w);
             }
-        }
     }
     for (; t < body; t += 32) {
-        const float4 m = __ldcs(row4 + t);
+        float4 m[ROWS];
+#pragma unroll
+        for (int q = 0; q < ROWS; ++q) m[q] = __ldcs(reinterpret_cast<const float4 *>(row + q * next) + t);
 #pragma unroll
         for (int r = 0; r < R; ++r) {
             const float4 w = reinterpret_cast<const float4 *>(v + (size_t)r * ldv)[t];
-            float a = acc[0][r];
-            a = fmaf(m.x, w.x, a);
-            a = fmaf(m.y, w.y, a);
-            a = fmaf(m.z, w.z, a);
-            a = fmaf(m.w, w.w, a);
-            acc[0][r] = a;
+#pragma unroll
+            for (int q = 0; q < ROWS; ++q) acc[q][0][r] = mac(acc[q][0][r], m[q], w);
         }
     }
 #pragma unroll
-    for (int r = 0; r < R; ++r) out[r] = warp_sum((double)acc[0][r] + (double)acc[1][r]);
+    for (int q = 0; q < ROWS; ++q)
+#pragma unroll
+        for (int r = 0; r < R; ++r) out[q][r] = warp_sum((double)acc[q][0][r] + (double)acc[q][1][r]);
 }
 
 // y[r][i] = y0[r][i] + sum_q Minv_hi[i][q] v[r][q] for every run (the
-// refinement step's correction), one warp per row; vh: the high parts of
+// refinement step's correction); vh: the high parts of
 // the vector, [run][ldm] with zero padding.
 template <int R>
-__global__ void __launch_bounds__(256) k_minv_apply_hi(const float *Mh, int nt, int ldm, const float *vh,
+__global__ void __launch_bounds__(32 * kStepWarps) k_minv_apply_hi(const float *Mh, int nt, int ldm, const float *vh,
                                                        const double *y0, double *y, int nrun) {
     pdl_wait();
     pdl_trigger();
-    const int i = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    const int lane = threadIdx.x & 31;
+    int more, i = step_row<R>(nt, more);
     if (i >= nt) return;
-    double s[R];
-    row_dot_f32<R>(Mh + (size_t)i * ldm, ldm, vh, ldm, lane, s);
+    double s[kRows<R>][R];
+    row_dot_f32<R, kRows<R>>(Mh + (size_t)i * ldm, (size_t)more * ldm, ldm, vh, ldm, lane, s);
 #pragma unroll
-    for (int r = 0; r < R; ++r)
-        if (lane == 0 && r < nrun) y[(size_t)r * nt + i] = y0[(size_t)r * nt + i] + s[r];
+    for (int q = 0; q < kRows<R>; ++q, ++i)
+#pragma unroll
+        for (int r = 0; r < R; ++r)
+            if (lane == 0 && r < nrun && q <= more) y[(size_t)r * nt + i] = y0[(size_t)r * nt + i] + s[q][r];
 }
 
 // res = b - M x for every run (M of k_transient_fill applied from its
 // blocks: Lp / dt, theta R, theta AS, -theta A^T through the adjacency,
 // F / dt), rows split as in k_transient_rhs.
 template <int R>
-__global__ void __launch_bounds__(256) k_transient_resid(StepArgs A, const double *b, double *res, int eb) {
+__global__ void __launch_bounds__(32 * kStepWarps) k_transient_resid(StepArgs A, const double *b, double *res, int eb) {
     pdl_wait();
     pdl_trigger();
     const int nt = A.ne + A.nv;
     if ((int)blockIdx.x < eb) {
-        const int i = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+        const int lane = threadIdx.x & 31;
+        int more, i = step_row<R>(A.ne, more);
         if (i >= A.ne) return;
-        double s[R], sa[R];
-        row_dot_df<R, true>(A.Lf + (size_t)i * A.lde, A.lde, A.xI, A.lde, lane, s);
-        row_dot_df<R, true>(A.ASf + (size_t)i * A.ldn, A.ldn, A.xV, A.ldn, lane, sa);
+        double s[kRows<R>][R], sa[kRows<R>][R];
+        row_dot_df<R, kRows<R>>(A.Lf + (size_t)i * A.lde, (size_t)more * A.lde, A.lde, A.xI, A.lde, lane, s);
+        row_dot_df<R, kRows<R>>(A.ASf + (size_t)i * A.ldn, (size_t)more * A.ldn, A.ldn, A.xV, A.ldn, lane, sa);
 #pragma unroll
-        for (int r = 0; r < R; ++r) {
-            const double ls = s[r], as = sa[r];
-            if (lane == 0 && r < A.nrun) {
-                const double *x = A.x + (size_t)r * nt;
-                const double mx = ls / A.dt + A.theta * A.R[i] * x[i] + A.theta * as;
-                res[(size_t)r * nt + i] = b[(size_t)r * nt + i] - mx;
+        for (int q = 0; q < kRows<R>; ++q, ++i)
+#pragma unroll
+            for (int r = 0; r < R; ++r) {
+                const double ls = s[q][r], as = sa[q][r];
+                if (lane == 0 && r < A.nrun && q <= more) {
+                    const double *x = A.x + (size_t)r * nt;
+                    const double mx = ls / A.dt + A.theta * A.R[i] * x[i] + A.theta * as;
+                    res[(size_t)r * nt + i] = b[(size_t)r * nt + i] - mx;
+                }
             }
-        }
         return;
     }
     const int t = (blockIdx.x - eb) * blockDim.x + threadIdx.x;
@@ -616,24 +652,26 @@ struct StepBuffers {
 };
 template <int R>
 static void launch_step(const TransientSystem &S, const StepArgs &A, const StepArgs &Ares, const StepBuffers &b,
-                        int grid, int eb, int mgrid, int nrun) {
-    const int nt = S.nt;
+                        int nrun) {
+    const int nt = S.nt, per = kStepWarps * kRows<R>, threads = 32 * kStepWarps;
+    const int eb = (S.ne + per - 1) / per, grid = eb + (S.nv * nrun + threads - 1) / threads;
+    const int mgrid = (nt + per - 1) / per;
     const unsigned xgrid = (unsigned)(((size_t)R * (S.lde + S.ldn) + 255) / 256);
     // the step's chain as programmatic dependents: each kernel waits for the
     // one before it (pdl_wait) and lets the next be scheduled at once
     pdl_launch(k_split_state, dim3(xgrid), dim3(256), 0, (const double *)b.x, R, S.ne, S.nv, S.lde, S.ldn, b.xI,
                b.xV);
-    pdl_launch(k_transient_rhs<R>, dim3(grid), dim3(256), 0, A, eb);
+    pdl_launch(k_transient_rhs<R>, dim3(grid), dim3(threads), 0, A, eb);
     const int ldm = S.ldm;
     const unsigned pgrid = (unsigned)(((size_t)R * ldm + 255) / 256);
     pdl_launch(k_split_rows, dim3(pgrid), dim3(256), 0, (const double *)b.rhs, R, nt, ldm, b.vs, (float *)nullptr);
-    pdl_launch(k_minv_apply<R>, dim3(mgrid), dim3(256), 0, (const float2 *)S.minv, nt, ldm, (const float2 *)b.vs,
+    pdl_launch(k_minv_apply<R>, dim3(mgrid), dim3(threads), 0, (const float2 *)S.minv, nt, ldm, (const float2 *)b.vs,
                (const double *)nullptr, b.x0, nrun);
     pdl_launch(k_split_state, dim3(xgrid), dim3(256), 0, (const double *)b.x0, R, S.ne, S.nv, S.lde, S.ldn, b.x0I,
                b.x0V);
-    pdl_launch(k_transient_resid<R>, dim3(grid), dim3(256), 0, Ares, (const double *)b.rhs, b.res, eb);
+    pdl_launch(k_transient_resid<R>, dim3(grid), dim3(threads), 0, Ares, (const double *)b.rhs, b.res, eb);
     pdl_launch(k_split_rows, dim3(pgrid), dim3(256), 0, (const double *)b.res, R, nt, ldm, b.vs, b.vh);
-    pdl_launch(k_minv_apply_hi<R>, dim3(mgrid), dim3(256), 0, (const float *)S.minv_hi, nt, ldm,
+    pdl_launch(k_minv_apply_hi<R>, dim3(mgrid), dim3(threads), 0, (const float *)S.minv_hi, nt, ldm,
                (const float *)b.vh, (const double *)b.x0, b.x, nrun);
 }
 
@@ -642,10 +680,10 @@ static int run_lightning(const TransientSystem &S, const LightningArgs *src, int
                          long long n_steps, double *d_X, const int *probe_nodes, int n_probe_nodes,
                          const int *probe_edges, int n_probe_edges, double *probes) {
     const int ne = S.ne, nv = S.nv, nt = S.nt;
-    // the step kernels are instantiated for 1, 2, 4 or 8 runs and read that
-    // many states: pad with zero states (measured: a 16-run instantiation
+    // the step kernels are instantiated for 1, 2, 3, 4, 6 or 8 runs and read
+    // that many states: pad with zero states (measured: a 16-run instantiation
     // stepped 16 runs slower than two batches of 8)
-    const int cap = nrun <= 1 ? 1 : nrun <= 2 ? 2 : nrun <= 4 ? 4 : 8;
+    const int cap = nrun <= 4 ? std::max(nrun, 1) : nrun <= 6 ? 6 : 8;
     DBuf<double> x((size_t)nt * cap), rhs((size_t)nt * cap), x0((size_t)nt * cap), res((size_t)nt * cap);
     // float pairs of the vectors: of an apply (vs), of the state x (xs) and of
     // x0 (x0s) for the right-hand side and the residual products
@@ -683,8 +721,6 @@ static int run_lightning(const TransientSystem &S, const LightningArgs *src, int
     A.n_probe_nodes = n_probe_nodes;
     A.n_probe_edges = n_probe_edges;
     A.probes = (n_probe_nodes + n_probe_edges) > 0 ? probes : nullptr;
-    const int eb = (ne + 7) / 8, grid = eb + (nv * nrun + 255) / 256;
-    const int mgrid = (nt + 7) / 8;
     StepArgs Ares = A;  // the residual reads x0 as its state
     Ares.x = x0.p;
     Ares.xI = x0I.p;
@@ -694,10 +730,12 @@ static int run_lightning(const TransientSystem &S, const LightningArgs *src, int
         A.step = step0 + k;
         A.record_row = k - 1;
         switch (cap) {
-            case 1: launch_step<1>(S, A, Ares, bufs, grid, eb, mgrid, nrun); break;
-            case 2: launch_step<2>(S, A, Ares, bufs, grid, eb, mgrid, nrun); break;
-            case 4: launch_step<4>(S, A, Ares, bufs, grid, eb, mgrid, nrun); break;
-            default: launch_step<8>(S, A, Ares, bufs, grid, eb, mgrid, nrun); break;
+            case 1: launch_step<1>(S, A, Ares, bufs, nrun); break;
+            case 2: launch_step<2>(S, A, Ares, bufs, nrun); break;
+            case 3: launch_step<3>(S, A, Ares, bufs, nrun); break;
+            case 4: launch_step<4>(S, A, Ares, bufs, nrun); break;
+            case 6: launch_step<6>(S, A, Ares, bufs, nrun); break;
+            default: launch_step<8>(S, A, Ares, bufs, nrun); break;
         }
         if ((k & 255) == 255 && !launch_ok("transient step")) return -1;
     }
