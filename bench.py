@@ -1234,7 +1234,7 @@ def main():
             if ms and pairs and p32.value:
                 a = pairs / (ms * 1e-3) / 1e9
                 pk = p32.value * 1e12 / 2 / 32 * (32 / 7.25) / 1e9
-                roofs.append({"kernel": "k_assemble_tiles far rule, %s (FP32, mixed path)" % tag, "bound": "issue",
+                roofs.append({"kernel": "k_entry_eval far rule, %s (FP32, mixed path)" % tag, "bound": "issue",
                               "achieved": a, "peak": pk, "unit": "Gpoint-pairs/s", "frac": a / pk, "ms": ms,
                               "traffic": None,
                               "peak_source": "measured FP32 FMA rate / 2 / 32 lanes x 32 / 7.25 point pairs per "
@@ -1280,7 +1280,7 @@ def main():
         dist.destroy_process_group()
 
 
-DF_FP32_INSTR_PER_PAIR = 106  # double-float far rule: FP32 instructions per point pair (csrc/assembly.cu)
+DIGIT_PAIRS = 78  # products of digits i + j <= 13 of 12 a factor (csrc/digit_gemm.cu)
 
 
 def load_traffic():
@@ -1311,21 +1311,24 @@ def roofline(phases, lu, m, fp64_peak, fp32_peak, work):
     out = []
     if lu.get("update_ms"):
         a = lu["update_flops"] / (lu["update_ms"] * 1e-3) / 1e12
-        out.append({"kernel": "k_gemm_cplx (complex LU trailing update, FP64 FMA)", "bound": "fp64",
-                    "achieved": a, "peak": fp64_peak, "unit": "TFLOP/s", "frac": a / fp64_peak if fp64_peak else None,
-                    "ms": lu["update_ms"], "traffic": traffic.get("k_gemm_cplx"),
-                    "peak_source": "measured (bench FMA loop)"})
+        bf16 = peaks.get("bf16_tflops", 1900.0)
+        out.append({"kernel": "k_digit_gemm (complex LU updates, FP64 results from exact integer digits on the "
+                              "tensor cores; with their digit splits)", "bound": "tensor",
+                    "achieved": DIGIT_PAIRS * a, "peak": bf16, "unit": "TFLOP/s", "frac": DIGIT_PAIRS * a / bf16,
+                    "ms": lu["update_ms"], "traffic": traffic.get("k_digit_gemm"),
+                    "peak_source": "measured (MEASURED_PEAKS.json, cuBLAS BF16 burst)",
+                    "note": "issued BF16 flops: %d digit pairs a real product; %.2f TFLOP/s of FP64 results"
+                            % (DIGIT_PAIRS, a)})
     far_pairs = {"Lp": work.get("Lp_far_point_pairs", 0), "P": work.get("P_far_point_pairs", 0)}
     for tag in ("Lp", "P"):
         ms = phases.get(tag + "_far")
         if ms:
             a = far_pairs[tag] / (ms * 1e-3) / 1e9
-            pk = fp32_peak * 1e12 / 2 / DF_FP32_INSTR_PER_PAIR / 1e9
-            out.append({"kernel": "k_assemble_tiles far rule, %s (double-float on the FP32 pipe)" % tag,
-                        "bound": "fp32", "achieved": a, "peak": pk, "unit": "Gpoint-pairs/s", "frac": a / pk,
-                        "ms": ms, "traffic": traffic.get("k_assemble_tiles"),
-                        "peak_source": "measured FP32 FMA rate / %d FP32 instructions per point pair"
-                                       % DF_FP32_INSTR_PER_PAIR})
+            out.append({"kernel": "k_entry_eval far rule, %s (double-float on the FP32 pipe)" % tag,
+                        "bound": "fp32", "achieved": a, "peak": None, "unit": "Gpoint-pairs/s", "frac": None,
+                        "ms": ms, "traffic": traffic.get("k_entry_eval"),
+                        "note": "point pairs covered: entries that are translated copies of one another share one "
+                                "sum, so the rate has no instruction bound to be compared with"})
     if phases.get("mna_fill"):
         b = 16.0 * n * n + 8.0 * ne * ne + 8.0 * nv * nv  # Z written, Lp read, P read (its rows gathered)
         a = b / (phases["mna_fill"] * 1e-3) / 1e9
