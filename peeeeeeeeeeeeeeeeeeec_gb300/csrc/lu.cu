@@ -1090,12 +1090,10 @@ template <class T>
 __global__ void __launch_bounds__(kClMaxThreads) k_panel_cl(T *a, int n, int k0, int kb, int rows_per_cta,
                                                             int row_threads, double limit, long long *piv, Status *st,
                                                             double tie) {
+    pdl_wait();  // (FP64: an ordinary launch, nothing to wait for)
     constexpr bool cx = std::is_same<T, cplx>::value, f32 = std::is_same<T, cplxf>::value;
     using Key = typename ClType<T>::Key;
-    if constexpr (f32) {
-        pdl_wait();
-        pdl_trigger();
-    }
+    if constexpr (f32) pdl_trigger();
     namespace cg = cooperative_groups;
     cg::cluster_group cluster = cg::this_cluster();
     extern __shared__ __align__(16) unsigned char cl_smem[];
