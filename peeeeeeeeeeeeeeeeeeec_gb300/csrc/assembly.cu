@@ -2043,10 +2043,15 @@ static bool assemble_entries(const TileArgs &T, int nrec, bool reuse) {
     U.overflow = counts.p + 1;
     unsigned long long slots = 1024;
     while (slots < (unsigned long long)n * n && slots < kMaxReuseSlots) slots <<= 1;
-    // without memory for the table, every entry by itself
-    if (reuse && cudaMallocAsync((void **)&U.tab, slots * sizeof(EntrySlot), stream()) != cudaSuccess) {
+    // without memory for the tables, every entry by itself
+    const size_t words = ((size_t)n * n + 31) / 32;
+    unsigned long long cap = 1;
+    while (cap < 4ull * (unsigned long long)n) cap <<= 1;
+    bool room = reuse;
+    if (room && cudaMallocAsync((void **)&U.tab, slots * sizeof(EntrySlot), stream()) != cudaSuccess) {
         cudaGetLastError();
         U.tab = nullptr;
+        room = false;
     }
     struct Freer {
         void *p;
@@ -2054,13 +2059,12 @@ static bool assemble_entries(const TileArgs &T, int nrec, bool reuse) {
             if (p) cudaFreeAsync(p, stream());
         }
     } freer{U.tab};
+    if (room && (!hash.alloc(n) || !ok.alloc(n) || !slot_of.alloc(n) || !cls.alloc(n) || !ctab.alloc(cap) ||
+                 !near_bits.alloc(words) || !mass.alloc(n))) {
+        cudaGetLastError();
+        U.tab = nullptr;
+    }
     if (U.tab) {
-        const size_t words = ((size_t)n * n + 31) / 32;
-        unsigned long long cap = 1;
-        while (cap < 4ull * (unsigned long long)n) cap <<= 1;
-        if (!hash.alloc(n) || !ok.alloc(n) || !slot_of.alloc(n) || !cls.alloc(n) || !ctab.alloc(cap) ||
-            !near_bits.alloc(words) || !mass.alloc(n))
-            return false;
         U.cls = cls.p;
         U.mask = slots - 1;
         U.near_bits = near_bits.p;
@@ -2084,9 +2088,13 @@ static bool assemble_entries(const TileArgs &T, int nrec, bool reuse) {
     if (!cuda_ok(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_entry_eval, kTileWarps * 32, 0), "assembly"))
         return false;
     // in bands of tile rows whose list has at most 2^22 entries (or one tile row)
-    const int rows = std::max(1, std::min(nt, (1 << 22) / (kTile * kTile * nt)));
-    DBuf<unsigned long long> list((size_t)rows * nt * kTile * kTile);
-    if (!list.p) return false;
+    int rows = std::max(1, std::min(nt, (1 << 22) / (kTile * kTile * nt)));
+    DBuf<unsigned long long> list;
+    while (!list.alloc((size_t)rows * nt * kTile * kTile)) {
+        if (rows == 1) return false;
+        cudaGetLastError();
+        rows /= 2;
+    }
     for (int ta0 = 0; ta0 < nt; ta0 += rows) {
         cudaMemsetAsync(count.p, 0, sizeof(unsigned), stream());
         PEEC_LAUNCH(k_entry_list, dim3(nt, std::min(rows, nt - ta0)), 256, 0, T, U, ta0, list.p, count.p);
