@@ -204,51 +204,62 @@ __global__ void __launch_bounds__(256) k_cgemm_sub(const c32 *A, int lda, const 
 
 // ---- real FP64: the inverse of an LU-factored matrix (transient system) ----
 
-// The real diagonal block solved for every right-hand side, one warp per
-// right-hand side (as k_trsm_diag).
+// The real diagonal block solved for every right-hand side: 32 right-hand sides
+// per CTA, one per lane, the rows dealt to its eight warps (row i to warp i % 8).
+// Bound by the FP64 pipe: 64 x 64 / 2 FMAs and 64 quotients a right-hand side.
+// (One warp a right-hand side with the rows in its lanes spent two FMAs of 32 lanes
+// on every row, and the quotient in all of them: 3552 right-hand sides, upper 133
+// us, lower 30; now 31 and 25.)  A quotient is y r, r the row's reciprocal,
+// corrected by its remainder.
 template <bool LOWER>
 __global__ void __launch_bounds__(256) k_trsm_diag_d(const double *lu, int n, int r0, int nrow, double *Y,
                                                      int nrhs) {
     __shared__ double B[kDB][kDB + 1];
+    __shared__ double rcp[kDB], xs[2][32];  // xs: the solved row, by parity
     for (int t = threadIdx.x; t < kDB * kDB; t += blockDim.x) {
         const int i = t / kDB, j = t % kDB;
-        double v = i == j ? 1.0 : 0.0;
-        if (i < nrow && j < nrow) v = lu[(size_t)(r0 + i) * n + r0 + j];
-        B[i][j] = v;
+        if (i < nrow && j < nrow) B[i][j] = lu[(size_t)(r0 + i) * n + r0 + j];
+    }
+    constexpr int R = kDB / 8;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int q = blockIdx.x * 32 + lane;
+    double v[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        const int i = r * 8 + warp;
+        v[r] = i < nrow && q < nrhs ? Y[(size_t)(r0 + i) * nrhs + q] : 0.0;
     }
     __syncthreads();
-    const int lane = threadIdx.x & 31;
-    const int q = blockIdx.x * 8 + (threadIdx.x >> 5);
-    if (q >= nrhs) return;
-    double v0 = lane < nrow ? Y[(size_t)(r0 + lane) * nrhs + q] : 0.0;
-    double v1 = lane + 32 < nrow ? Y[(size_t)(r0 + lane + 32) * nrhs + q] : 0.0;
-    if (LOWER) {
-        for (int j = 0; j < kDB - 1; ++j) {
-            const double xj = __shfl_sync(0xffffffffu, j < 32 ? v0 : v1, j & 31);
-            if (lane > j) v0 = fma(-B[lane][j], xj, v0);
-            if (lane + 32 > j) v1 = fma(-B[lane + 32][j], xj, v1);
-        }
-    } else {
-        // reciprocals of the diagonal once; a quotient is then y r corrected by its
-        // remainder (three FP64 operations a step where a division takes about ten)
-        const double r0d = 1.0 / B[lane][lane], r1d = 1.0 / B[lane + 32][lane + 32];
-        for (int j = kDB - 1; j >= 0; --j) {
-            const double y = __shfl_sync(0xffffffffu, j < 32 ? v0 : v1, j & 31);
-            const double r = __shfl_sync(0xffffffffu, j < 32 ? r0d : r1d, j & 31);
-            const double q = y * r;
-            const double xj = fma(fma(-q, B[j][j], y), r, q);
-            if (lane < j) v0 = fma(-B[lane][j], xj, v0);
-            if (lane + 32 < j) v1 = fma(-B[lane + 32][j], xj, v1);
-            if (lane == (j & 31)) {
-                if (j < 32)
-                    v0 = xj;
-                else
-                    v1 = xj;
+    if (!LOWER && threadIdx.x < nrow) rcp[threadIdx.x] = 1.0 / B[threadIdx.x][threadIdx.x];
+    __syncthreads();
+#pragma unroll
+    for (int s = 0; s < R; ++s) {
+        const int rm = LOWER ? s : R - 1 - s;
+#pragma unroll 2
+        for (int t = 0; t < 8; ++t) {
+            const int w = LOWER ? t : 7 - t, m = rm * 8 + w;  // the row that is solved next
+            if (m >= nrow) continue;                          // uniform
+            double *x = xs[m & 1];
+            if (warp == w) {
+                if (!LOWER) {
+                    const double y = v[rm], c = rcp[m], z = y * c;
+                    v[rm] = fma(fma(-z, B[m][m], y), c, z);
+                }
+                x[lane] = v[rm];
             }
+            __syncthreads();
+            const double xm = x[lane];
+            if (LOWER ? warp > w : warp < w) v[rm] = fma(-B[rm * 8 + warp][m], xm, v[rm]);
+#pragma unroll
+            for (int r = 0; r < R; ++r)
+                if (LOWER ? r > rm : r < rm) v[r] = fma(-B[r * 8 + warp][m], xm, v[r]);
         }
     }
-    if (lane < nrow) Y[(size_t)(r0 + lane) * nrhs + q] = v0;
-    if (lane + 32 < nrow) Y[(size_t)(r0 + lane + 32) * nrhs + q] = v1;
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        const int i = r * 8 + warp;
+        if (i < nrow && q < nrhs) Y[(size_t)(r0 + i) * nrhs + q] = v[r];
+    }
 }
 
 // C[i][q] -= sum_k A[i][k] Bm[k][q] in FP64 (as k_cgemm_sub).
@@ -489,7 +500,7 @@ __global__ void k_mark_done(const unsigned long long *be_q, int *done, int nrhs,
 bool inverse_from_lu_real(const double *lu, const int *perm, int n, double *Minv) {
     using namespace mrhs;
     PEEC_LAUNCH(k_permuted_identity, (unsigned)(((size_t)n * n + 255) / 256), 256, 0, perm, n, Minv);
-    const unsigned dgrid = (unsigned)((n + 7) / 8);
+    const unsigned dgrid = (unsigned)((n + 31) / 32);
     auto block = [&](bool lower, int r0, int nrow) {
         if (lower)
             PEEC_LAUNCH(k_trsm_diag_d<true>, dgrid, 256, 0, lu, n, r0, nrow, Minv, n);

@@ -6,7 +6,9 @@ import numpy as np
 import pytest
 
 from conftest import golden
-from test_gpu_transient import DeviceTransient
+from helpers import inductance, potential
+from peeeeeeeeeeeeeeeeeeec_gb300.mesh import SynthMesh
+from test_gpu_transient import I_TOL, V_TOL, DeviceTransient, werr
 
 pytestmark = pytest.mark.gpu
 
@@ -33,3 +35,24 @@ def test_batch_of_n_runs(gpu_lib, n):
             assert np.array_equal(X[r, :ne], I) and np.array_equal(X[r, ne:], V)
     finally:
         t.close()
+
+
+@pytest.mark.parametrize("nx,ny", [(1, 1), (1, 12), (4, 4), (1, 25), (1, 26)])
+def test_inverse_at_block_edges(gpu_lib, oracle, nx, ny):
+    """8, 63, 65, 128 and 133 unknowns: whole and ragged 64-row blocks of the
+    substitution that forms the inverse."""
+    with SynthMesh.plate(0.05 * nx, 0.05 * ny, nx, ny) as m:
+        _, L = inductance(gpu_lib, m)
+        _, P = potential(gpu_lib, m)
+        edges = np.ascontiguousarray(m.edges())
+        R = 1e-3 * np.ones(m.n_edges)
+        src = (102900.0, 1500.0, 1.0e6, 0.0, 0, m.n_nodes - 1)
+        t = DeviceTransient(gpu_lib, L, P, edges, R, 2, 1e-7)
+        try:
+            s, I, V, _ = t.run(src, 20)
+            so, Io, Vo, _ = oracle.transient_lightning(L, P, edges, R, 2, 1e-7, src, 20, probe_nodes=range(m.n_nodes),
+                                                       probe_edges=range(m.n_edges))
+            assert s == 0 and so == 0
+            assert werr(I, Io) < I_TOL and werr(V, Vo) < V_TOL
+        finally:
+            t.close()
