@@ -202,6 +202,68 @@ __global__ void __launch_bounds__(256) k_cgemm_sub(const c32 *A, int lda, const 
     }
 }
 
+// The same with 16 x 64 output tiles and all of K staged at once, for few tiles:
+// with up to two tiles of 64 x 64 an SM (a 3776-unknown system with 64 right-hand
+// sides: 58 tiles at most) SMs idle and every chunk of K waits for its loads: 21.5
+// us a launch, now 7.3.  More tiles reuse their operands better as 64 x 64 (720
+// right-hand sides, lines at 152 / 304 / 1000 tiles: 102.9 / 102.5 / 103.3 ms a solve,
+// 256: 57.6 / 56.7 / 56.6).  Each sum in the same order.
+static const int kFewTiles = 304;
+__global__ void __launch_bounds__(256) k_cgemm_sub_few(const c32 *A, int lda, const c32 *Bm, c32 *C, int ldb, int M,
+                                                       int NC, int K, const int *done) {
+    __shared__ c32 As[64][16 + 1];
+    __shared__ c32 Bs[64][64];
+    const int m0 = blockIdx.y * 16, n0 = blockIdx.x * 64;
+    const int qc = n0 + (threadIdx.x & 63);
+    if (__syncthreads_and(qc >= NC || done[qc])) return;
+    const int tr = threadIdx.x >> 4, tc = threadIdx.x & 15;  // 16 x 16 threads, 1 x 4 outputs
+    const int kr = (K + 15) & ~15;  // K <= 64
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+        const int t = threadIdx.x + 256 * u, r = t >> 6, k = t & 63;
+        As[k][r] = (m0 + r < M && k < K) ? A[(size_t)(m0 + r) * lda + k] : c32{0.0f, 0.0f};
+    }
+#pragma unroll
+    for (int u = 0; u < 16; ++u) {
+        const int t = threadIdx.x + 256 * u, k = t >> 6, c = t & 63;
+        Bs[k][c] = (k < K && n0 + c < NC) ? Bm[(size_t)k * ldb + n0 + c] : c32{0.0f, 0.0f};
+    }
+    __syncthreads();
+    c32 acc[4];
+#pragma unroll
+    for (int y = 0; y < 4; ++y) acc[y] = c32{0.0f, 0.0f};
+#pragma unroll 8
+    for (int k = 0; k < kr; ++k) {
+        const c32 a = As[k][tr];
+#pragma unroll
+        for (int y = 0; y < 4; ++y) {
+            const c32 b = Bs[k][tc + 16 * y];
+            acc[y].re = fmaf(a.re, b.re, acc[y].re);
+            acc[y].re = fmaf(-a.im, b.im, acc[y].re);
+            acc[y].im = fmaf(a.re, b.im, acc[y].im);
+            acc[y].im = fmaf(a.im, b.re, acc[y].im);
+        }
+    }
+    const int i = m0 + tr;
+    if (i >= M) return;
+#pragma unroll
+    for (int y = 0; y < 4; ++y) {
+        const int q = n0 + tc + 16 * y;
+        if (q >= NC) continue;
+        c32 &c = C[(size_t)i * ldb + q];
+        c.re -= acc[y].re;
+        c.im -= acc[y].im;
+    }
+}
+
+static void cgemm_sub(const c32 *A, int lda, const c32 *Bm, c32 *C, int ldb, int M, int NC, int K, const int *done) {
+    const unsigned nc = (NC + 63) / 64, nm = (M + 63) / 64;
+    if (nc * nm <= (unsigned)kFewTiles)
+        PEEC_LAUNCH(k_cgemm_sub_few, dim3(nc, (M + 15) / 16), 256, 0, A, lda, Bm, C, ldb, M, NC, K, done);
+    else
+        PEEC_LAUNCH(k_cgemm_sub, dim3(nc, nm), 256, 0, A, lda, Bm, C, ldb, M, NC, K, done);
+}
+
 // ---- real FP64: the inverse of an LU-factored matrix (transient system) ----
 
 // The real diagonal block solved for every right-hand side: 32 right-hand sides
@@ -602,15 +664,14 @@ bool mrhs_sweep(const void *Zs, const void *lu, const int *perm, const double *r
         const int r0 = blk * kDB, nrow = min(kDB, n - r0), r1 = r0 + nrow;
         PEEC_LAUNCH(k_trsm_diag<true>, dgrid, 256, 0, F, n, r0, nrow, Yt, nrhs, (const int *)done);
         if (r1 < n)
-            PEEC_LAUNCH(k_cgemm_sub, dim3((nrhs + 63) / 64, (n - r1 + 63) / 64), 256, 0, F + (size_t)r1 * n + r0, n,
-                        Yt + (size_t)r0 * nrhs, Yt + (size_t)r1 * nrhs, nrhs, n - r1, nrhs, nrow, (const int *)done);
+            cgemm_sub(F + (size_t)r1 * n + r0, n, Yt + (size_t)r0 * nrhs, Yt + (size_t)r1 * nrhs, nrhs, n - r1, nrhs,
+                      nrow, (const int *)done);
     }
     for (int blk = nb - 1; blk >= 0; --blk) {  // backward: upper
         const int r0 = blk * kDB, nrow = min(kDB, n - r0);
         PEEC_LAUNCH(k_trsm_diag<false>, dgrid, 256, 0, F, n, r0, nrow, Yt, nrhs, (const int *)done);
         if (r0 > 0)
-            PEEC_LAUNCH(k_cgemm_sub, dim3((nrhs + 63) / 64, (r0 + 63) / 64), 256, 0, F + r0, n,
-                        Yt + (size_t)r0 * nrhs, Yt, nrhs, r0, nrhs, nrow, (const int *)done);
+            cgemm_sub(F + r0, n, Yt + (size_t)r0 * nrhs, Yt, nrhs, r0, nrhs, nrow, (const int *)done);
     }
     PEEC_LAUNCH(k_update_out, tgrid, 256, 0, (c64 *)x, Yt, cs, n, nrhs, (float4 *)xs, (const int *)done);
     PEEC_LAUNCH(k_residual_gemm_df, dim3((nrhs + 31) / 32, (n + 63) / 64), 256, sizeof(RTile), (const float4 *)Zs,
