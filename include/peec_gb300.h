@@ -105,6 +105,17 @@ int peec_gb300_complex_lu_factor_device(Complex *d_a, size_t n, double pivot_tol
                                         long long *d_piv, int *d_perm,
                                         double *d_row_scale, double *d_column_scale,
                                         double *matrix_scale, int *failed_column);
+/* The same with the form of the updates given: 0 FP64 FMAs in pivot order, 1
+ * integer digits, 2 integer digits with the check for near ties (and FP64 FMAs
+ * from the start where it stops).  1 and 2 take FP64 FMAs after a singular pivot
+ * and without the memory for a copy of the matrix; *used (may be NULL): 0 if the
+ * factor comes from FP64 FMAs, 1 from digits.  Row and column scales: complex only. */
+int peec_gb300_lu_factor_device_form(int cplx, void *d_a, size_t n, double pivot_tolerance,
+                                     long long *d_piv, int *d_perm, double *d_row_scale,
+                                     double *d_column_scale, int form, int *used);
+/* The inverse (n x n, row-major) of the matrix whose factor and permutation
+ * peec_gb300_lu_factor_device left.  0, or -1 on errors. */
+int peec_gb300_inverse_device(const double *d_lu, const int *d_perm, size_t n, double *d_inverse);
 /* Same as peec_gb300_lu_factor_device, but allocates no device memory (no
  * cudaMalloc, cudaFree or allocating library call), for callers that own all
  * device memory through their own pool or hard budget, or that must not let
@@ -168,6 +179,14 @@ int peec_gb300_tc_gemm(const void *d_a, const void *d_b0, const void *d_b1, floa
  * persistent kernel (TMEM double-buffered accumulators, TMA epilogue). */
 int peec_gb300_tc_gemm_cplx(const void *d_a, const void *d_br, const void *d_bi, float *d_c, int m,
                             int n, int k, int row0, int col0, long long ldc);
+
+/* C (m x n, FP64, row-major, leading dimension ldc) -= A (m x k) B (k x n) in FP64
+ * accuracy on tcgen05, as sums of products of integer digits; complex entries
+ * (cplx != 0) are interleaved {re, im} and leading dimensions count entries.  C
+ * must not overlap A or B.  k <= 256, complex 192.  The update of the
+ * factorisations.  0, or -1 on invalid arguments or errors. */
+int peec_gb300_digit_gemm_sub(int cplx, const void *d_a, size_t lda, const void *d_b, size_t ldb, void *d_c,
+                              size_t ldc, int m, int n, int k);
 
 /* ---- RCS radiation vectors (rcs.c:701-1000, dual-patch quadrature) ----
  * For every direction d (directions: host [n_dir][3], unit vectors) and

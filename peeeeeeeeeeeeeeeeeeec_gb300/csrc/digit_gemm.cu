@@ -39,6 +39,7 @@
 #include <algorithm>
 #include <type_traits>
 
+#include "../../include/peec_gb300.h"
 #include "common.cuh"
 #include "tc_gemm.cuh"
 
@@ -981,3 +982,24 @@ bool digit_gemm_sub(bool cplx, const void *A, size_t lda, const void *B, size_t 
 }
 
 }  // namespace peec
+
+extern "C" int peec_gb300_digit_gemm_sub(int cplx, const void *d_a, size_t lda, const void *d_b, size_t ldb, void *d_c,
+                                         size_t ldc, int m, int n, int k) {
+    using namespace peec;
+    if (!d_a || !d_b || !d_c || m < 1 || n < 1 || k < 1 || lda < (size_t)k || ldb < (size_t)n || ldc < (size_t)n ||
+        k > (cplx ? kDigitMaxKCplx : kDigitMaxKReal))
+        return -1;
+    DigitScratch s;
+    DBuf<int> code(1);
+    if (!s.alloc(cplx != 0, m, n, k) || !code.p) return -1;
+    cudaMemsetAsync(code.p, 0, sizeof(int), stream());
+    if (!digit_gemm_sub(cplx != 0, d_a, lda, d_b, ldb, d_c, ldc, m, n, k, s, code.p)) return -1;
+    int h = 0;
+    cudaMemcpyAsync(&h, code.p, sizeof(int), cudaMemcpyDeviceToHost, stream());
+    if (!sync("digit GEMM")) return -1;
+    if (h != 0) {
+        set_error("digit GEMM: a wait ran out");
+        return -1;
+    }
+    return 0;
+}

@@ -2848,10 +2848,11 @@ namespace peec {
 // again(): puts the original matrix back into d_a; with it, large systems are
 // factored by digit GEMMs in a checked run, and by chains of FP64 FMAs from the
 // start again if that met a near tie of two pivot candidates or a singular
-// pivot: pivots and status are those of the chains in every case.
+// pivot: pivots and status are those of the chains in every case.  mode: the one
+// that the factor comes from on return.
 template <class T, class Again>
 static int factor_inplace(T *d_a, int n, double pivot_tolerance, bool cx, long long *d_piv, int *d_perm,
-                          double *d_row, double *d_col, double *scale, Status *hs, LuMode mode, Again again) {
+                          double *d_row, double *d_col, double *scale, Status *hs, LuMode &mode, Again again) {
     size_t nn = (size_t)n * n;
     DBuf<Status> st(1);
     DBuf<unsigned long long> mx(1);
@@ -2906,8 +2907,9 @@ static void report_status(const Status &hs, bool cx) {
 int lu_factor_again(double *d_a, int n, double pivot_tolerance, long long *d_piv, int *d_perm, double *scale,
                     int *failed_column, const std::function<bool()> &again) {
     Status hs;
-    if (factor_inplace<double>(d_a, n, pivot_tolerance, false, d_piv, d_perm, nullptr, nullptr, scale, &hs,
-                               n >= kDigitsFromReal ? LuMode::digits : LuMode::chain, again) != 0)
+    LuMode mode = n >= kDigitsFromReal ? LuMode::digits : LuMode::chain;
+    if (factor_inplace<double>(d_a, n, pivot_tolerance, false, d_piv, d_perm, nullptr, nullptr, scale, &hs, mode,
+                               again) != 0)
         return -1;
     *failed_column = hs.code ? hs.column : -1;
     if (!isfinite(*scale) || *scale <= 0.0) return -2;
@@ -2918,22 +2920,27 @@ int complex_lu_factor_again(Complex *d_a, int n, double pivot_tolerance, long lo
                             double *d_col, const std::function<bool()> &again) {
     Status hs;
     double scale = 0.0;
-    if (factor_inplace<cplx>((cplx *)d_a, n, pivot_tolerance, true, d_piv, d_perm, d_row, d_col, &scale, &hs,
-                             n >= kDigitsFromCplx ? LuMode::checked : LuMode::chain, again) != 0)
+    LuMode mode = n >= kDigitsFromCplx ? LuMode::checked : LuMode::chain;
+    if (factor_inplace<cplx>((cplx *)d_a, n, pivot_tolerance, true, d_piv, d_perm, d_row, d_col, &scale, &hs, mode,
+                             again) != 0)
         return -1;
     if (hs.code == 4 || hs.code == 5 || !isfinite(scale) || scale <= 0.0) return -2;
     if (hs.code) report_status(hs, true);
     return hs.code ? -2 : 0;
 }
 
+static LuMode checked_mode(int n, bool cx) {
+    return n >= (cx ? kDigitsFromCplx : kCheckedFromReal) ? LuMode::checked : LuMode::chain;
+}
+
 // The device-resident forms keep a copy of the matrix for a second run; where
 // there is no memory for it, chains it is.
 template <class T>
 static int factor_inplace_copy(T *d_a, int n, double pivot_tolerance, bool cx, long long *d_piv, int *d_perm,
-                               double *d_row, double *d_col, double *scale, Status *hs) {
+                               double *d_row, double *d_col, double *scale, Status *hs, LuMode &mode) {
     const size_t bytes = (size_t)n * n * sizeof(T);
     void *copy = nullptr;
-    if (n >= (cx ? kDigitsFromCplx : kCheckedFromReal) && cudaMallocAsync(&copy, bytes, stream()) != cudaSuccess) {
+    if (mode != LuMode::chain && cudaMallocAsync(&copy, bytes, stream()) != cudaSuccess) {
         (void)cudaGetLastError();
         copy = nullptr;
     }
@@ -2941,12 +2948,10 @@ static int factor_inplace_copy(T *d_a, int n, double pivot_tolerance, bool cx, l
         dfree(copy);
         return -1;
     }
-    const int s = factor_inplace<T>(d_a, n, pivot_tolerance, cx, d_piv, d_perm, d_row, d_col, scale, hs,
-                                    copy ? LuMode::checked : LuMode::chain, [&] {
-                                        return cuda_ok(cudaMemcpyAsync(d_a, copy, bytes, cudaMemcpyDeviceToDevice,
-                                                                       stream()),
-                                                       "LU copy");
-                                    });
+    if (!copy) mode = LuMode::chain;
+    const int s = factor_inplace<T>(d_a, n, pivot_tolerance, cx, d_piv, d_perm, d_row, d_col, scale, hs, mode, [&] {
+        return cuda_ok(cudaMemcpyAsync(d_a, copy, bytes, cudaMemcpyDeviceToDevice, stream()), "LU copy");
+    });
     dfree(copy);
     return s;
 }
@@ -2981,7 +2986,7 @@ static int factorize_common(const T *input, size_t n, double pivot_tolerance, bo
     }
     Status hs;
     double scale = 0.0;
-    const LuMode mode = ni >= (cx ? kDigitsFromCplx : kCheckedFromReal) ? LuMode::checked : LuMode::chain;
+    LuMode mode = checked_mode(ni, cx);
     if (factor_inplace<T>(d_a, ni, pivot_tolerance, cx, r.d_piv, r.d_perm, r.d_row, r.d_col, &scale, &hs, mode, [&] {
             return cuda_ok(cudaMemcpyAsync(d_a, input, nn * sizeof(T), cudaMemcpyHostToDevice, stream()), "LU upload");
         }) != 0) {
@@ -3272,7 +3277,9 @@ int peec_gb300_lu_factor_device(double *d_a, size_t n, double pivot_tolerance, l
     if (!d_a || !d_piv || !d_perm || n == 0 || n > (size_t)0x7fffffff) return -1;
     Status hs;
     double scale = 0.0;
-    if (factor_inplace_copy<double>(d_a, (int)n, pivot_tolerance, false, d_piv, d_perm, nullptr, nullptr, &scale, &hs) != 0)
+    LuMode mode = checked_mode((int)n, false);
+    if (factor_inplace_copy<double>(d_a, (int)n, pivot_tolerance, false, d_piv, d_perm, nullptr, nullptr, &scale, &hs,
+                                    mode) != 0)
         return -1;
     if (matrix_scale) *matrix_scale = scale;
     if (failed_column) *failed_column = hs.code ? hs.column : -1;
@@ -3290,8 +3297,9 @@ int peec_gb300_complex_lu_factor_device(Complex *d_a, size_t n, double pivot_tol
     if (!d_a || !d_piv || !d_perm || !d_row_scale || !d_column_scale || n == 0 || n > (size_t)0x7fffffff) return -1;
     Status hs;
     double scale = 0.0;
+    LuMode mode = checked_mode((int)n, true);
     if (factor_inplace_copy<cplx>((cplx *)d_a, (int)n, pivot_tolerance, true, d_piv, d_perm, d_row_scale, d_column_scale,
-                             &scale, &hs) != 0)
+                                  &scale, &hs, mode) != 0)
         return -1;
     if (matrix_scale) *matrix_scale = scale;
     if (failed_column) *failed_column = hs.code ? hs.column : -1;
@@ -3301,6 +3309,25 @@ int peec_gb300_complex_lu_factor_device(Complex *d_a, size_t n, double pivot_tol
         return -2;
     }
     return 0;
+}
+
+int peec_gb300_lu_factor_device_form(int cplx_, void *d_a, size_t n, double pivot_tolerance, long long *d_piv,
+                                     int *d_perm, double *d_row_scale, double *d_column_scale, int form, int *used) {
+    if (!d_a || !d_piv || !d_perm || (cplx_ && (!d_row_scale || !d_column_scale)) || n == 0 ||
+        n > (size_t)0x7fffffff || form < 0 || form > 2)
+        return -1;
+    Status hs;
+    double scale = 0.0;
+    LuMode mode = form == 0 ? LuMode::chain : form == 1 ? LuMode::digits : LuMode::checked;
+    const int s = cplx_ ? factor_inplace_copy<cplx>((cplx *)d_a, (int)n, pivot_tolerance, true, d_piv, d_perm,
+                                                    d_row_scale, d_column_scale, &scale, &hs, mode)
+                        : factor_inplace_copy<double>((double *)d_a, (int)n, pivot_tolerance, false, d_piv, d_perm,
+                                                      nullptr, nullptr, &scale, &hs, mode);
+    if (s != 0) return -1;
+    if (used) *used = mode == LuMode::chain ? 0 : 1;
+    if (hs.code == 4 || hs.code == 5 || !isfinite(scale) || scale <= 0.0) return -2;
+    if (hs.code) report_status(hs, cplx_ != 0);
+    return hs.code ? -2 : 0;
 }
 
 int peec_gb300_lu_solve_device(const double *d_lu, const int *d_perm, size_t n, const double *d_b, double *d_x,

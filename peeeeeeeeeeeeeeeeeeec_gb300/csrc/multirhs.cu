@@ -16,6 +16,7 @@
 // value per thread in the diagonal-block solves.
 #include <math.h>
 
+#include "../../include/peec_gb300.h"
 #include "common.cuh"
 #include "digit_gemm.cuh"
 
@@ -681,3 +682,8 @@ bool mrhs_sweep(const void *Zs, const void *lu, const int *perm, const double *r
 }
 
 }  // namespace peec
+
+extern "C" int peec_gb300_inverse_device(const double *d_lu, const int *d_perm, size_t n, double *d_inverse) {
+    if (!d_lu || !d_perm || !d_inverse || n == 0 || n > (size_t)0x7fffffff) return -1;
+    return peec::inverse_from_lu_real(d_lu, d_perm, (int)n, d_inverse) && peec::sync("inverse") ? 0 : -1;
+}
