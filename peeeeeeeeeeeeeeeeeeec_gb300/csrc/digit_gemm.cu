@@ -20,8 +20,11 @@
 // update.  Its error is about 2^-78 |row of A| |column of B| (what is dropped).
 // A chain of K FP64 FMAs rounds at 2^-53 of its running sum, so entries whose C
 // and update are both below 2^-kExactBelow |row| |column| are left out and done
-// in FP64 (matrices of weakly coupled parts, systems at kHz): no entry is
-// less accurate than on the FP64 pipe.  (Eleven digits, 66 pairs, with the line
+// in FP64 (matrices of weakly coupled parts, systems at kHz).  Complex entries are
+// looked at by their real and imaginary parts, as a chain rounds each for itself
+// (small resistances beside j omega L); parts that are exactly zero, because no
+// product has both factors (lossless systems), are told by bit masks of the
+// operands' nonzero parts and cost nothing.  (Eleven digits, 66 pairs, with the line
 // at 2^-18: 5% faster on random matrices, but 341 against 294 ms for the solve of
 // the 8402-unknown box, where more entries take the FP64 way.)
 //
@@ -35,6 +38,8 @@
 #include "digit_gemm.cuh"
 
 #include <cuda_bf16.h>
+
+#include <limits.h>
 
 #include <algorithm>
 #include <type_traits>
@@ -146,8 +151,10 @@ __device__ __forceinline__ Fixed fixed_point(double x, int shift, int emax) {
 // ef[r]: exponent of the largest |entry| of row r of B (0 for a zero row): B's
 // rows are divided by 2^ef, A's columns multiplied.  One block per row.
 template <bool CX>
-__global__ void __launch_bounds__(256) k_row_exponents(const double *B, size_t ldb, int n, int *ef, const int *code) {
+__global__ void __launch_bounds__(256) k_row_exponents(const double *B, size_t ldb, int n, int *ef, unsigned *exact,
+                                                       const int *code) {
     if (*code != 0) return;
+    if (blockIdx.x == 0 && threadIdx.x == 0) *exact = 0;
     __shared__ int s_max[8];
     const double *row = B + (size_t)blockIdx.x * ldb * (CX ? 2 : 1);
     int e = 0;
@@ -162,6 +169,23 @@ __global__ void __launch_bounds__(256) k_row_exponents(const double *B, size_t l
         for (int w = 1; w < 8; ++w) e = max(e, s_max[w]);
         ef[blockIdx.x] = e == 0 ? 0 : e - 1022;
     }
+}
+
+// Bit masks of a complex row of A or column of B: which of its (up to kMaskWords 32)
+// real and imaginary parts are not zero.
+static const int kMaskWords = 6;
+struct Mask {
+    unsigned re[8], im[8];
+};
+__device__ __forceinline__ void store_mask(Mask *masks, int i, int o, const double (*x)[2]) {
+    unsigned re = 0, im = 0;
+#pragma unroll
+    for (int t = 0; t < 8; ++t) {
+        re |= (__double_as_longlong(x[t][0]) << 1) != 0 ? 1u << t : 0u;
+        im |= (__double_as_longlong(x[t][1]) << 1) != 0 ? 1u << t : 0u;
+    }
+    reinterpret_cast<unsigned char *>(masks[i].re)[o] = (unsigned char)re;
+    reinterpret_cast<unsigned char *>(masks[i].im)[o] = (unsigned char)im;
 }
 
 // The lowest balanced digit (-64 .. 63) of X; X <- (X - digit) / 128.  s: its
@@ -221,7 +245,8 @@ __device__ __forceinline__ int swizzled(int r, int o) { return r * 32 + ((o ^ ((
 // entries.
 template <bool CX, int TPR>
 __global__ void __launch_bounds__(256) k_digits_rows(const double *A, size_t lda, int m, int k, int kc_count,
-                                                     unsigned char *out, int *ea, const int *ef, const int *code) {
+                                                     unsigned char *out, int *ea, Mask *masks, const int *ef,
+                                                     const int *code) {
     if (*code != 0) return;
     constexpr int P = CX ? 2 : 1;
     const int row = blockIdx.x * (256 / TPR) + threadIdx.x / TPR, o = threadIdx.x % TPR;
@@ -264,6 +289,7 @@ __global__ void __launch_bounds__(256) k_digits_rows(const double *A, size_t lda
     for (int s = TPR / 2; s > 0; s >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, s);
     emax += norm_shift(sq);
     if (o == 0) ea[row] = bad ? kNotFinite : emax < kZero / 2 ? kZero : emax - 1022;
+    if constexpr (CX) store_mask(masks, row, o, x);
     if (o >= 2 * kc_count) return;
     const int tile = row / kBM, r = row % kBM;
     unsigned char *base = out + (size_t)(tile * kc_count + (o >> 1)) * kDigits * Shape<CX>::kABytes + swizzled(r, o & 1);
@@ -302,7 +328,8 @@ __device__ __forceinline__ void load_rows(const double *B, size_t ldb, int n, in
 
 template <bool CX>
 __global__ void __launch_bounds__(512) k_digits_cols(const double *B, size_t ldb, int n, int k, int kc_count,
-                                                     unsigned char *out, int *eb, const int *ef, const int *code) {
+                                                     unsigned char *out, int *eb, Mask *masks, const int *ef,
+                                                     const int *code) {
     if (*code != 0) return;
     constexpr int P = CX ? 2 : 1;
     __shared__ int s_max[8][64];
@@ -353,8 +380,10 @@ __global__ void __launch_bounds__(512) k_digits_cols(const double *B, size_t ldb
     const int tile = col / Shape<CX>::BN, r = col % Shape<CX>::BN;
     if (tile >= (n + Shape<CX>::BN - 1) / Shape<CX>::BN) return;
     if (ty == 0) eb[col] = bad ? kNotFinite : emax < kZero / 2 ? kZero : emax - 1022;
-    for (int o = ty; o < 2 * kc_count; o += 8) {
+    for (int o = ty; o < (2 * kc_count + 3) / 4 * 4; o += 8) {
         load_rows<CX>(B, ldb, n, k, col, 8 * o, ef, x, f);
+        if constexpr (CX) store_mask(masks, col, o, x);
+        if (o >= 2 * kc_count) break;
         unsigned char *base =
             out + (size_t)(tile * kc_count + (o >> 1)) * kDigits * Shape<CX>::kBBytes + swizzled(r, o & 1);
         Fixed X[8];
@@ -453,11 +482,14 @@ __device__ __forceinline__ void tmem_wait_ld(int *v, int *w) {
 struct Args {
     const unsigned char *a, *b;
     const int *ea, *eb;
+    const Mask *ma, *mb;
     double *c;
     size_t ldc;
     const double *a64, *b64;  // the operands, for entries done in FP64
     size_t lda, ldb;
     int m, n, k, kc_count;
+    unsigned *exact;       // entries done in FP64 so far
+    unsigned exact_limit;  // beyond it *code becomes 7
     int *code;
 };
 
@@ -469,6 +501,34 @@ __device__ __forceinline__ bool below(long long v) {
 // |z| below 2^(E - kExactBelow)
 __device__ __forceinline__ bool below(double z, int E) {
     return (int)((__double_as_longlong(z) >> 52) & 0x7ff) < E + 1023 - kExactBelow;
+}
+
+// Parts of this lane's row (i) in columns j0 .. + 15 that are sums of zeros: bit c
+// for the real part of column j0 + c, bit 16 + c for the imaginary one.  (An
+// infinity or NaN times zero is none.)
+__device__ __forceinline__ unsigned zero_parts(const Args &A, int i, int j0) {
+    const int lane = threadIdx.x & 31, words = (2 * A.kc_count + 3) / 4;
+    const bool bad = A.ea[i] >= kNotFinite;
+    const unsigned bad_columns = __ballot_sync(0xffffffffu, A.eb[j0 + (lane & 15)] >= kNotFinite);
+    unsigned re[kMaskWords], im[kMaskWords], zero = 0;
+#pragma unroll
+    for (int w = 0; w < kMaskWords; ++w) {
+        re[w] = w < words ? A.ma[i].re[w] : 0u;
+        im[w] = w < words ? A.ma[i].im[w] : 0u;
+    }
+#pragma unroll 2
+    for (int c = 0; c < 16; ++c) {
+        unsigned r = 0, s = 0;
+#pragma unroll
+        for (int w = 0; w < kMaskWords; ++w)
+            if (w < words) {
+                const unsigned br = A.mb[j0 + c].re[w], bi = A.mb[j0 + c].im[w];
+                r |= (re[w] & br) | (im[w] & bi);
+                s |= (re[w] & bi) | (im[w] & br);
+            }
+        zero |= (r == 0 ? 1u : 0u) << c | (s == 0 ? 0x10000u : 0u) << c;
+    }
+    return bad ? 0u : zero & ~bad_columns;
 }
 
 // One entry of C -= A B in FP64: K products from k0 on, `step` apart.
@@ -764,6 +824,7 @@ __global__ void __launch_bounds__(32 * (2 + kEpiWarps), 1) k_digit_gemm(Args A) 
         constexpr int RPI = 32 / S::kCols, kSteps = S::kCols;  // rows per warp access, accesses per chunk
         const int rr = lane / S::kCols, cc = lane % S::kCols;
         int tile = 0;
+        unsigned fp64 = 0;  // this lane's entries done in FP64
         bool ok = true;
         for (int t = blockIdx.x; t < ntiles; t += gridDim.x, ++tile) {
             int tm, tn;
@@ -785,6 +846,8 @@ __global__ void __launch_bounds__(32 * (2 + kEpiWarps), 1) k_digit_gemm(Args A) 
             };
             fetch(0);
             fetch(1);
+            unsigned zero = 0;  // (while the first sums are formed)
+            if constexpr (CX) zero = zero_parts(A, row0 + lane, col0);
             // Sums of i + j >= 10 in units of 2^-kUnit; their bits below 2^-61 go to
             // TMEM, the rest is summed in units of 2^-61 with the others.
             long long run[32];
@@ -840,18 +903,17 @@ __global__ void __launch_bounds__(32 * (2 + kEpiWarps), 1) k_digit_gemm(Args A) 
                 tmem_wait_ld(low, low + 4);
                 Scalar *p = reinterpret_cast<Scalar *>(buf + lane * S::kRowStride);
                 double w[8];            // re, im of four columns, or eight columns
-                unsigned small = 0u;    // columns whose update is below the limit
+                unsigned small = 0u;    // columns whose update (complex: bits 0.. real, 16.. imaginary part) is below the limit
 #pragma unroll
                 for (int c = 0; c < S::kCols; ++c) {
                     const int col = ch * S::kCols + c;  // 0..15 (complex), 0..31 (real)
                     const int E = er + __shfl_sync(0xffffffffu, ec, col) - 61;
-                    bool sm = below(run[col]);
+                    small |= below(run[col]) ? 1u << c : 0u;
                     w[c] = __longlong_as_double(compose(run[col], (unsigned)low[c], E));
                     if constexpr (CX) {
-                        sm = sm && below(run[16 + col]);
+                        small |= below(run[16 + col]) ? 0x10000u << c : 0u;
                         w[4 + c] = __longlong_as_double(compose(run[16 + col], (unsigned)low[4 + c], E));
                     }
-                    small |= sm ? 1u << c : 0u;
                 }
 #pragma unroll
                 for (int c = 0; c < S::kCols; ++c) {
@@ -859,7 +921,8 @@ __global__ void __launch_bounds__(32 * (2 + kEpiWarps), 1) k_digit_gemm(Args A) 
                     const Scalar z = p[c];
                     const int E = er + __shfl_sync(0xffffffffu, ec, col);
                     if constexpr (CX) {
-                        const bool left = (small >> c & 1u) && below(z.x, E) && below(z.y, E);
+                        const unsigned part = small >> c & ~(zero >> col);
+                        const bool left = ((part & 1u) && below(z.x, E)) || ((part >> 16 & 1u) && below(z.y, E));
                         p[c] = make_double2(z.x - (left ? 0.0 : w[c]), z.y - (left ? 0.0 : w[4 + c]));
                         exact |= left ? 1u << col : 0u;
                     } else {
@@ -884,7 +947,14 @@ __global__ void __launch_bounds__(32 * (2 + kEpiWarps), 1) k_digit_gemm(Args A) 
             }
             if (row0 + lane >= A.m) exact = 0;
             exact &= col0 + S::kWarpCols <= A.n ? 0xffffffffu : A.n > col0 ? (1u << (A.n - col0)) - 1u : 0u;
-            if (__any_sync(0xffffffffu, exact != 0)) exact_entries<CX>(A, row0, col0, exact);
+            if (__any_sync(0xffffffffu, exact != 0)) {
+                fp64 += __popc(exact);
+                exact_entries<CX>(A, row0, col0, exact);
+            }
+        }
+        if constexpr (CX) {
+            fp64 = __reduce_add_sync(0xffffffffu, fp64);
+            if (lane == 0 && fp64 != 0 && atomicAdd(A.exact, fp64) + fp64 > A.exact_limit) atomicCAS(A.code, 0, 7);
         }
     leave:
         if (!ok) s_abort = 1;
@@ -901,26 +971,32 @@ __global__ void __launch_bounds__(32 * (2 + kEpiWarps), 1) k_digit_gemm(Args A) 
     if (warp == 0) tc::tmem_dealloc(tmem, 512);
 }
 
+static size_t round_up(size_t v, size_t to) { return (v + to - 1) / to * to; }
+
 template <bool CX>
 static bool run(const void *A, size_t lda, const void *B, size_t ldb, void *C, size_t ldc, int m, int n, int k,
-                DigitScratch &s, int *code) {
+                DigitScratch &s, int *code, size_t exact_limit) {
     typedef Shape<CX> S;
     const int kc = (k + kKC - 1) / kKC;
     const int mt = (m + kBM - 1) / kBM, nt = (n + S::BN - 1) / S::BN;
     static const cudaError_t attr =
         cudaFuncSetAttribute(k_digit_gemm<CX>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::kSmem);
     if (!cuda_ok(attr, "digit GEMM shared memory")) return false;
-    PEEC_LAUNCH(k_row_exponents<CX>, k, 256, 0, (const double *)B, ldb, n, s.ef, (const int *)code);
+    PEEC_LAUNCH(k_row_exponents<CX>, k, 256, 0, (const double *)B, ldb, n, s.ef, s.exact,
+                (const int *)code);
+    Mask *ma = static_cast<Mask *>(s.mask), *mb = ma ? ma + round_up(s.m, kBM) : nullptr;
     auto rows = k <= 64 ? k_digits_rows<CX, 8> : k <= 128 ? k_digits_rows<CX, 16> : k_digits_rows<CX, 32>;
     PEEC_LAUNCH(rows, mt * kBM * (k <= 64 ? 8 : k <= 128 ? 16 : 32) / 256, 256, 0, (const double *)A, lda, m, k, kc,
-                (unsigned char *)s.a, s.ea, (const int *)s.ef, (const int *)code);
+                (unsigned char *)s.a, s.ea, ma, (const int *)s.ef, (const int *)code);
     PEEC_LAUNCH(k_digits_cols<CX>, (nt * S::BN + 63) / 64, 512, 0, (const double *)B, ldb, n, k, kc, (unsigned char *)s.b,
-                s.eb, (const int *)s.ef, (const int *)code);
+                s.eb, mb, (const int *)s.ef, (const int *)code);
     Args a;
     a.a = (const unsigned char *)s.a;
     a.b = (const unsigned char *)s.b;
     a.ea = s.ea;
     a.eb = s.eb;
+    a.ma = ma;
+    a.mb = mb;
     a.c = (double *)C;
     a.ldc = ldc;
     a.a64 = (const double *)A;
@@ -931,6 +1007,8 @@ static bool run(const void *A, size_t lda, const void *B, size_t ldb, void *C, s
     a.n = n;
     a.k = k;
     a.kc_count = kc;
+    a.exact = s.exact;
+    a.exact_limit = (unsigned)std::min(exact_limit, (size_t)UINT_MAX);
     a.code = code;
     int dev = 0, sms = 0;
     cudaGetDevice(&dev);
@@ -939,13 +1017,12 @@ static bool run(const void *A, size_t lda, const void *B, size_t ldb, void *C, s
     return launch_ok("digit GEMM");
 }
 
-static size_t round_up(size_t v, size_t to) { return (v + to - 1) / to * to; }
-
 }  // namespace dg
 
 size_t digit_scratch_bytes(bool cplx, size_t m, size_t n, size_t k) {
     const size_t kp = dg::round_up(k, dg::kKC), mp = dg::round_up(m, dg::kBM), np = dg::round_up(n, 96);
-    return mp * kp * dg::kDigits * 2 * (cplx ? 2 : 1) + np * kp * dg::kDigits * 2 * (cplx ? 3 : 1) + 4 * (mp + np + kp);
+    return mp * kp * dg::kDigits * 2 * (cplx ? 2 : 1) + np * kp * dg::kDigits * 2 * (cplx ? 3 : 1) + 4 * (mp + np + kp) +
+           (cplx ? (mp + np) * sizeof(dg::Mask) : 0);
 }
 
 bool DigitScratch::alloc(bool cplx_, int m_, int n_, int k_) {
@@ -959,7 +1036,9 @@ bool DigitScratch::alloc(bool cplx_, int m_, int n_, int k_) {
     ea = static_cast<int *>(dalloc(4 * mp));
     eb = static_cast<int *>(dalloc(4 * np));
     ef = static_cast<int *>(dalloc(4 * kp));
-    return a && b && ea && eb && ef;
+    exact = static_cast<unsigned *>(dalloc(sizeof(unsigned)));
+    if (cplx) mask = dalloc((mp + np) * sizeof(dg::Mask));
+    return a && b && ea && eb && ef && exact && (mask || !cplx);
 }
 
 DigitScratch::~DigitScratch() {
@@ -968,17 +1047,19 @@ DigitScratch::~DigitScratch() {
     dfree(ea);
     dfree(eb);
     dfree(ef);
+    dfree(exact);
+    dfree(mask);
 }
 
 bool digit_gemm_sub(bool cplx, const void *A, size_t lda, const void *B, size_t ldb, void *C, size_t ldc, int m, int n,
-                    int k, DigitScratch &s, int *code) {
+                    int k, DigitScratch &s, int *code, size_t exact_limit) {
     if (m <= 0 || n <= 0 || k <= 0) return true;
     if (s.cplx != cplx || m > s.m || n > s.n || k > s.k || k > (cplx ? kDigitMaxKCplx : kDigitMaxKReal)) {
         set_error("digit GEMM: size beyond its scratch");
         return false;
     }
-    return cplx ? dg::run<true>(A, lda, B, ldb, C, ldc, m, n, k, s, code)
-                : dg::run<false>(A, lda, B, ldb, C, ldc, m, n, k, s, code);
+    return cplx ? dg::run<true>(A, lda, B, ldb, C, ldc, m, n, k, s, code, exact_limit)
+                : dg::run<false>(A, lda, B, ldb, C, ldc, m, n, k, s, code, exact_limit);
 }
 
 }  // namespace peec

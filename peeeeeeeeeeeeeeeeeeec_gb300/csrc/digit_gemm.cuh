@@ -17,6 +17,8 @@ static const int kDigitMaxKCplx = 192;
 struct DigitScratch {
     void *a = nullptr, *b = nullptr;
     int *ea = nullptr, *eb = nullptr, *ef = nullptr;
+    unsigned *exact = nullptr;  // entries of the last update done in FP64
+    void *mask = nullptr;  // complex: the nonzero parts of rows and columns
     int m = 0, n = 0, k = 0;
     bool cplx = false;
     DigitScratch() = default;
@@ -31,8 +33,10 @@ size_t digit_scratch_bytes(bool cplx, size_t m, size_t n, size_t k);
 // ldb); complex entries are interleaved {re, im} and the leading dimensions
 // count entries.  C must not overlap A or B.  m, n, k within the scratch's
 // sizes.  *code (device): nothing is done when it is not 0; it is set to 6
-// when a bounded wait inside the kernel runs out.
+// when a bounded wait inside the kernel runs out, and to 7 when more than exact_limit
+// entries were so small beside their rows and columns that FP64 FMAs did them
+// (complex only; the update is complete all the same).
 bool digit_gemm_sub(bool cplx, const void *A, size_t lda, const void *B, size_t ldb, void *C, size_t ldc, int m, int n,
-                    int k, DigitScratch &s, int *code);
+                    int k, DigitScratch &s, int *code, size_t exact_limit = ~(size_t)0);
 
 }  // namespace peec

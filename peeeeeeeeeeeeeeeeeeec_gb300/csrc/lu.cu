@@ -117,7 +117,7 @@ __device__ __forceinline__ cplx addv(cplx a, cplx b) { return cplx{a.re + b.re, 
 __device__ __forceinline__ cplxf addv(cplxf a, cplxf b) { return cplxf{a.re + b.re, a.im + b.im}; }
 
 struct Status {
-    int code;    // 0 ok, 2 singular / invalid pivot, 7 near tie of two pivot candidates (checked runs)
+    int code;    // 0 ok, 2 singular / invalid pivot, 7 near tie of two pivot candidates, or mostly FP64 work (checked runs)
     int column;  // failing column
     double value;
 };
@@ -2583,7 +2583,8 @@ static thread_local LuTiming g_lu_timing;  // per host thread, like the stream
 enum class LuMode {
     chain,    // chains of FP64 FMAs in pivot order: the reference's arithmetic up to FMA rounding
     digits,   // digit GEMMs
-    checked,  // digit GEMMs, stopping with status 7 at a near tie of two pivot candidates
+    checked,  // digit GEMMs, stopping with status 7 at a near tie of two pivot candidates or where
+              // most entries are left to FP64 FMAs
 };
 // Unknowns from which digit GEMMs are used (LU of random matrices on GB300,
 // chains / digits in ms: complex 1000: 17.6 / 16.7, 1200: 22.2 / 20.2, 1400: 27.7 /
@@ -2594,6 +2595,14 @@ enum class LuMode {
 static const int kDigitsFromCplx = 1300;
 static const int kDigitsFromReal = 2000;
 static const int kCheckedFromReal = 5000;
+static const int kLookAt = 192;  // the column where a checked run looks whether it was stopped
+// Share of the entries of the first updates (up to kLookAt) that may be left to FP64
+// FMAs: these cost the digit GEMM about 1.5 times what they cost k_gemm_rect, and
+// the share hardly changes with the column.  Boxes with resistances of 1e-3 / 1e-4 /
+// 1e-5 / 1e-6 of |Z| beside lossless couplings at 30 MHz, 8402 unknowns: 0.2 / 5 / 28 / 67 %
+// of the entries (parts that small) and 343 / 517 / 1040 / 1393 ms, FP64 alone 1366;
+// 2102 unknowns: 0.1 / 1 / 16 / 60 % and 22 / 29 / 43 / 51 ms, FP64 alone 35.
+static double most_in_fp64(int n) { return std::min(0.4, 5e-5 * n); }
 static const int kLuWideFrom = 3000;  // unknowns from which wide outer blocks pay (2102 complex: 45 ms with, 43 without, before the rows of U were solved in one kernel)
 
 // How close two pivot candidates of column k must be to count as a near tie.
@@ -2719,14 +2728,18 @@ static bool factor_device(T *d_a, int n, double limit, long long *d_piv, Status 
         // C -= L U on rows r0 .. r1-1, columns c0 .. c1-1 with the columns / rows k0 .. k1-1
         auto update = [&](int k0, int k1, int r0, int r1, int c0, int c1) {
             if (tm.enabled) tm.flops_update += (cx ? 8.0 : 2.0) * (double)(r1 - r0) * (c1 - c0) * (k1 - k0);
+            const bool first = mode == LuMode::checked && k0 < kLookAt && r0 == k1 && c1 == n;
+            const double entries = (double)(r1 - r0) * (c1 - c0);
             return digit_gemm_sub(cx, d_a + (size_t)r0 * n + k0, n, d_a + (size_t)k0 * n + c0, n,
-                                  d_a + (size_t)r0 * n + c0, n, r1 - r0, c1 - c0, k1 - k0, digits, &d_st->code);
+                                  d_a + (size_t)r0 * n + c0, n, r1 - r0, c1 - c0, k1 - k0, digits, &d_st->code,
+                                  first ? (size_t)(most_in_fp64(n) * entries) : ~(size_t)0);
         };
         bool looked = mode != LuMode::checked;
         for (int K0 = 0; K0 < n; K0 += W) {
             const int K1 = std::min(n, K0 + W);
-            if (!looked && K0 >= 192) {
-                // matrices that tie do so early: look once before the bulk of the work
+            if (!looked && K0 >= kLookAt) {
+                // matrices that tie, or whose entries are mostly left to FP64, do
+                // so early: look once before the bulk of the work
                 looked = true;
                 int code = 0;
                 cudaMemcpyAsync(&code, &d_st->code, sizeof(int), cudaMemcpyDeviceToHost, stream());

@@ -15,6 +15,7 @@ import pytest
 
 pytestmark = pytest.mark.gpu
 U = 2.0 ** -53
+TURNS = np.array([1, 1j, -1, -1j])
 
 
 class Device:
@@ -302,3 +303,57 @@ def test_transient_system_with_digits(gpu_lib, oracle, nx, ny):
             assert werr(I, Io) < I_TOL and werr(V, Vo) < V_TOL
         finally:
             t.close()
+
+
+@pytest.mark.parametrize("eps", [1e-7, 1e-10, 1e-13])
+@pytest.mark.parametrize("turned", [False, True])
+def test_each_part_of_complex_entries_keeps_its_own_accuracy(gpu_lib, eps, turned):
+    """Imaginary parts eps of the real ones (a small resistance beside j omega L
+    and the other way round: rows, inner index and columns turned by j at random):
+    each part is as accurate as an FMA chain of its own products."""
+    m, n, k = 150, 110, 192
+    rng = np.random.default_rng(11)
+    a, b, c = (rng.standard_normal(s) + 1j * eps * rng.standard_normal(s) for s in ((m, k), (k, n), (m, n)))
+    if turned:
+        r, s, t = (TURNS[rng.integers(0, 4, x)] for x in (m, n, k))
+        a, b, c = a * r[:, None] * t[None].conj(), b * t[:, None] * s[None], c * r[:, None] * s[None]
+    check(a, b, c, digit_sub(gpu_lib, a, b, c), some(m), floor=False)
+
+
+@pytest.mark.parametrize("k", [1, 17, 64, 130, 192])
+def test_parts_that_are_sums_of_zeros(gpu_lib, k):
+    """Without the small parts (a lossless system) the other part is exactly what it was,
+    and a single nonzero factor far below the rest (1e-30 or 1e-200) is not overlooked."""
+    m, n = 150, 110
+    rng = np.random.default_rng(12)
+    r, s, t = (TURNS[rng.integers(0, 4, x)] for x in (m, n, k))
+    a, b, c = (rng.standard_normal(x).astype(complex) for x in ((m, k), (k, n), (m, n)))
+    a, b, c = a * r[:, None] * t[None].conj(), b * t[:, None] * s[None], c * r[:, None] * s[None]
+    i = k - 1
+    a[5, i] += 1e-30 * 1j * r[5] * np.conj(t[i])
+    b[i, 7] += 1e-30 * 1j * t[i] * s[7]
+    a[6, i] += 1e-200 * 1j * r[6] * np.conj(t[i])
+    out = digit_sub(gpu_lib, a, b, c)
+    check(a, b, c, out, some(m) + [5, 6], floor=False)
+    small = out / r[:, None] / s[None]
+    whole = np.ones((m, n), dtype=bool)
+    whole[[5, 6]] = whole[:, 7] = False
+    assert np.all(small.imag[whole] == 0)
+    assert np.all(small.imag[[5, 6]] != 0) and np.all(small.imag[:, 7] != 0)
+
+
+@pytest.mark.parametrize("eps,digits", [(0.0, 1), (1e-2, 1), (1e-9, 0)])
+def test_systems_of_small_second_parts(gpu_lib, eps, digits):
+    """A checked run in which FP64 FMAs would do most entries takes them from the start;
+    without second parts, or with ones of the usual size, it keeps the digits."""
+    n = 700
+    rng = np.random.default_rng(13)
+    a = rng.standard_normal((n, n)) + 1j * eps * rng.standard_normal((n, n))
+    s, lu, piv, rs, cs, used = factor(gpu_lib, a, CHECKED)
+    assert s == 0 and used == digits
+    _, lu0, piv0, _, _, _ = factor(gpu_lib, a, FMA)
+    assert np.array_equal(piv, piv0)
+    if eps == 0.0:
+        assert np.all(lu.imag == 0)
+    if not digits:
+        assert np.array_equal(lu, lu0)
