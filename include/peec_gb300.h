@@ -94,8 +94,8 @@ int peec_gb300_set_near_reuse(int on);
  * int32) the combined row permutation the solves use.  failed_column is the
  * column of a singular pivot, or -1.  Large systems (complex from 1300, real
  * from 5000 unknowns) are updated on the tensor cores from integer digits; for
- * that the call holds a copy of the matrix while it runs (without the memory
- * for it, FP64 FMAs do the updates): where two pivot candidates are so close
+ * that the call holds a copy of the matrix and the digits while it runs (without
+ * the memory for them, FP64 FMAs do the updates): where two pivot candidates are so close
  * that rounding could decide between them it starts again with FP64 FMAs, so
  * pivots and status do not depend on the form of the updates. */
 int peec_gb300_lu_factor_device(double *d_a, size_t n, double pivot_tolerance,
@@ -187,6 +187,11 @@ int peec_gb300_tc_gemm_cplx(const void *d_a, const void *d_br, const void *d_bi,
  * factorisations.  0, or -1 on invalid arguments or errors. */
 int peec_gb300_digit_gemm_sub(int cplx, const void *d_a, size_t lda, const void *d_b, size_t ldb, void *d_c,
                               size_t ldc, int m, int n, int k);
+
+/* Bytes that the digits of one factorisation or inverse called from this host
+ * thread may take (at first without limit): beyond it, and where there is no memory for
+ * them, FP64 FMAs do the updates.  Returns the previous limit. */
+size_t peec_gb300_set_digit_scratch_limit(size_t bytes);
 
 /* ---- RCS radiation vectors (rcs.c:701-1000, dual-patch quadrature) ----
  * For every direction d (directions: host [n_dir][3], unit vectors) and

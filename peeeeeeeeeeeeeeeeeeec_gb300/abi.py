@@ -244,6 +244,7 @@ EXT_SYMBOLS = [
     ("peec_gb300_lu_factor_device_form", C.c_int,
      [C.c_int, C.c_void_p, C.c_size_t, C.c_double, C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_int, c_int_p]),
     ("peec_gb300_inverse_device", C.c_int, [C.c_void_p, C.c_void_p, C.c_size_t, C.c_void_p]),
+    ("peec_gb300_set_digit_scratch_limit", C.c_size_t, [C.c_size_t]),
     ("peec_gb300_digit_gemm_sub", C.c_int,
      [C.c_int, C.c_void_p, C.c_size_t, C.c_void_p, C.c_size_t, C.c_void_p, C.c_size_t, C.c_int, C.c_int, C.c_int]),
     ("peec_gb300_lu_factor_device_noalloc", C.c_int,

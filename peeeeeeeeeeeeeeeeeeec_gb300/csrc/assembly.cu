@@ -2047,24 +2047,10 @@ static bool assemble_entries(const TileArgs &T, int nrec, bool reuse) {
     const size_t words = ((size_t)n * n + 31) / 32;
     unsigned long long cap = 1;
     while (cap < 4ull * (unsigned long long)n) cap <<= 1;
-    bool room = reuse;
-    if (room && cudaMallocAsync((void **)&U.tab, slots * sizeof(EntrySlot), stream()) != cudaSuccess) {
-        cudaGetLastError();
-        U.tab = nullptr;
-        room = false;
-    }
-    struct Freer {
-        void *p;
-        ~Freer() {
-            if (p) cudaFreeAsync(p, stream());
-        }
-    } freer{U.tab};
-    if (room && (!hash.alloc(n) || !ok.alloc(n) || !slot_of.alloc(n) || !cls.alloc(n) || !ctab.alloc(cap) ||
-                 !near_bits.alloc(words) || !mass.alloc(n))) {
-        cudaGetLastError();
-        U.tab = nullptr;
-    }
-    if (U.tab) {
+    DBuf<EntrySlot> tab;
+    if (reuse && tab.alloc_if_room(slots) && hash.alloc_if_room(n) && ok.alloc_if_room(n) && slot_of.alloc_if_room(n) &&
+        cls.alloc_if_room(n) && ctab.alloc_if_room(cap) && near_bits.alloc_if_room(words) && mass.alloc_if_room(n)) {
+        U.tab = tab.p;
         U.cls = cls.p;
         U.mask = slots - 1;
         U.near_bits = near_bits.p;
@@ -2090,11 +2076,8 @@ static bool assemble_entries(const TileArgs &T, int nrec, bool reuse) {
     // in bands of tile rows whose list has at most 2^22 entries (or one tile row)
     int rows = std::max(1, std::min(nt, (1 << 22) / (kTile * kTile * nt)));
     DBuf<unsigned long long> list;
-    while (!list.alloc((size_t)rows * nt * kTile * kTile)) {
-        if (rows == 1) return false;
-        cudaGetLastError();
-        rows /= 2;
-    }
+    while (rows > 1 && !list.alloc_if_room((size_t)rows * nt * kTile * kTile)) rows /= 2;
+    if (!list.p && !list.alloc((size_t)rows * nt * kTile * kTile)) return false;
     for (int ta0 = 0; ta0 < nt; ta0 += rows) {
         cudaMemsetAsync(count.p, 0, sizeof(unsigned), stream());
         PEEC_LAUNCH(k_entry_list, dim3(nt, std::min(rows, nt - ta0)), 256, 0, T, U, ta0, list.p, count.p);

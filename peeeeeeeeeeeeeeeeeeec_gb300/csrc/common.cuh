@@ -38,6 +38,8 @@ bool launch_ok(const char *what);
 // Stream-ordered device allocation on the library stream.
 void *dalloc(size_t bytes);
 void dfree(void *p);
+// The same where the caller can do without: no error is recorded or printed.
+void *dalloc_if_room(size_t bytes);
 
 template <class T> struct DBuf {
     T *p = nullptr;
@@ -48,6 +50,12 @@ template <class T> struct DBuf {
         release();
         n = count;
         p = count ? static_cast<T *>(dalloc(count * sizeof(T))) : nullptr;
+        return count == 0 || p != nullptr;
+    }
+    bool alloc_if_room(size_t count) {
+        release();
+        n = count;
+        p = static_cast<T *>(dalloc_if_room(count * sizeof(T)));
         return count == 0 || p != nullptr;
     }
     void release() {

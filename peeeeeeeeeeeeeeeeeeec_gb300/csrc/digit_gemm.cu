@@ -1025,23 +1025,32 @@ size_t digit_scratch_bytes(bool cplx, size_t m, size_t n, size_t k) {
            (cplx ? (mp + np) * sizeof(dg::Mask) : 0);
 }
 
+size_t &digit_scratch_limit() {
+    static thread_local size_t limit = ~(size_t)0;
+    return limit;
+}
+
 bool DigitScratch::alloc(bool cplx_, int m_, int n_, int k_) {
+    release();
+    if (digit_scratch_bytes(cplx_, m_, n_, k_) > digit_scratch_limit()) return false;
     cplx = cplx_;
     m = m_;
     n = n_;
     k = k_;
     const size_t kp = dg::round_up(k, dg::kKC), mp = dg::round_up(m, dg::kBM), np = dg::round_up(n, 96);
-    a = dalloc(mp * kp * dg::kDigits * 2 * (cplx ? 2 : 1));
-    b = dalloc(np * kp * dg::kDigits * 2 * (cplx ? 3 : 1));
-    ea = static_cast<int *>(dalloc(4 * mp));
-    eb = static_cast<int *>(dalloc(4 * np));
-    ef = static_cast<int *>(dalloc(4 * kp));
-    exact = static_cast<unsigned *>(dalloc(sizeof(unsigned)));
-    if (cplx) mask = dalloc((mp + np) * sizeof(dg::Mask));
-    return a && b && ea && eb && ef && exact && (mask || !cplx);
+    a = dalloc_if_room(mp * kp * dg::kDigits * 2 * (cplx ? 2 : 1));
+    b = dalloc_if_room(np * kp * dg::kDigits * 2 * (cplx ? 3 : 1));
+    ea = static_cast<int *>(dalloc_if_room(4 * mp));
+    eb = static_cast<int *>(dalloc_if_room(4 * np));
+    ef = static_cast<int *>(dalloc_if_room(4 * kp));
+    exact = static_cast<unsigned *>(dalloc_if_room(sizeof(unsigned)));
+    if (cplx) mask = dalloc_if_room((mp + np) * sizeof(dg::Mask));
+    if (a && b && ea && eb && ef && exact && (mask || !cplx)) return true;
+    release();
+    return false;
 }
 
-DigitScratch::~DigitScratch() {
+void DigitScratch::release() {
     dfree(a);
     dfree(b);
     dfree(ea);
@@ -1049,6 +1058,10 @@ DigitScratch::~DigitScratch() {
     dfree(ef);
     dfree(exact);
     dfree(mask);
+    a = b = mask = nullptr;
+    ea = eb = ef = nullptr;
+    exact = nullptr;
+    m = n = k = 0;
 }
 
 bool digit_gemm_sub(bool cplx, const void *A, size_t lda, const void *B, size_t ldb, void *C, size_t ldc, int m, int n,
@@ -1064,6 +1077,12 @@ bool digit_gemm_sub(bool cplx, const void *A, size_t lda, const void *B, size_t 
 
 }  // namespace peec
 
+extern "C" size_t peec_gb300_set_digit_scratch_limit(size_t bytes) {
+    const size_t before = peec::digit_scratch_limit();
+    peec::digit_scratch_limit() = bytes;
+    return before;
+}
+
 extern "C" int peec_gb300_digit_gemm_sub(int cplx, const void *d_a, size_t lda, const void *d_b, size_t ldb, void *d_c,
                                          size_t ldc, int m, int n, int k) {
     using namespace peec;
@@ -1072,7 +1091,10 @@ extern "C" int peec_gb300_digit_gemm_sub(int cplx, const void *d_a, size_t lda, 
         return -1;
     DigitScratch s;
     DBuf<int> code(1);
-    if (!s.alloc(cplx != 0, m, n, k) || !code.p) return -1;
+    if (!s.alloc(cplx != 0, m, n, k) || !code.p) {
+        set_error("digit GEMM: no memory for the digits");
+        return -1;
+    }
     cudaMemsetAsync(code.p, 0, sizeof(int), stream());
     if (!digit_gemm_sub(cplx != 0, d_a, lda, d_b, ldb, d_c, ldc, m, n, k, s, code.p)) return -1;
     int h = 0;

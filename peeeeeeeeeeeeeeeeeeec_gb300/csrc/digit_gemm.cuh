@@ -22,12 +22,18 @@ struct DigitScratch {
     int m = 0, n = 0, k = 0;
     bool cplx = false;
     DigitScratch() = default;
+    // false, with nothing allocated and no error recorded, where there is no memory
+    // for it or it is beyond digit_scratch_limit()
     bool alloc(bool cplx_, int m_, int n_, int k_);
-    ~DigitScratch();
+    void release();
+    ~DigitScratch() { release(); }
     DigitScratch(const DigitScratch &) = delete;
     DigitScratch &operator=(const DigitScratch &) = delete;
 };
 size_t digit_scratch_bytes(bool cplx, size_t m, size_t n, size_t k);
+// Bytes that a DigitScratch of the calling thread may take (no limit at first): the
+// server keeps jobs within their share of its budget.
+size_t &digit_scratch_limit();
 
 // C (m x n, row-major, leading dimension ldc) -= A (m x k, lda) B (k x n,
 // ldb); complex entries are interleaved {re, im} and the leading dimensions

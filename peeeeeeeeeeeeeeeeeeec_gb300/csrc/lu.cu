@@ -2614,7 +2614,7 @@ static const int kLuWideFrom = 3000;  // unknowns from which wide outer blocks p
 static double near_tie_fraction(int k) { return 0x1p-45 + (double)k * k * 0x1p-63; }
 
 template <class T>
-static bool factor_device(T *d_a, int n, double limit, long long *d_piv, Status *d_st, LuMode mode) {
+static bool factor_device(T *d_a, int n, double limit, long long *d_piv, Status *d_st, LuMode &mode) {
     LuTiming &tm = g_lu_timing;
     if (tm.enabled) tm.reset();
     DBuf<unsigned char> scratch;
@@ -2646,6 +2646,18 @@ static bool factor_device(T *d_a, int n, double limit, long long *d_piv, Status 
         sc.krow = b + off + 2 * G * NB * sizeof(T);
     }
     constexpr bool cx = sizeof(T) == sizeof(cplx);
+    // Outer blocks of W columns, inner blocks of two panels.  Everything
+    // wider than a panel is a digit GEMM: per inner block, the block's
+    // columns below its first row get what the outer block's earlier
+    // columns did (before the panels), then its rows to the right (after
+    // them: the panels' swaps bring rows from below that lack it too); per
+    // outer block, the trailing update with K = W.  A digit GEMM's tile
+    // costs an integer epilogue per entry whatever K is (m = n = 4000
+    // complex: 764 us with K = 64, 1730 us with 192), so W is its largest K;
+    // small systems, where launches count, take one inner block.
+    const int W = n < kLuWideFrom ? 2 * NB : cx ? kDigitMaxKCplx : kDigitMaxKReal;
+    DigitScratch digits;
+    if (mode != LuMode::chain && n > 2 * NB && !digits.alloc(cx, n - 2 * NB, n - 2 * NB, W)) mode = LuMode::chain;
     auto swaps = [&](int k0, int kb) {
         PEEC_LAUNCH(k_laswp<T>, (n + kLaswpCols - 1) / kLaswpCols, 256, 2 * NB * kLaswpCols * sizeof(T), d_a, n, k0, kb,
                     d_piv, d_st);
@@ -2713,18 +2725,6 @@ static bool factor_device(T *d_a, int n, double limit, long long *d_piv, Status 
             }
         }
     } else {
-        // Outer blocks of W columns, inner blocks of two panels.  Everything
-        // wider than a panel is a digit GEMM: per inner block, the block's
-        // columns below its first row get what the outer block's earlier
-        // columns did (before the panels), then its rows to the right (after
-        // them: the panels' swaps bring rows from below that lack it too); per
-        // outer block, the trailing update with K = W.  A digit GEMM's tile
-        // costs an integer epilogue per entry whatever K is (m = n = 4000
-        // complex: 764 us with K = 64, 1730 us with 192), so W is its largest K;
-        // small systems, where launches count, take one inner block.
-        const int W = n < kLuWideFrom ? 2 * NB : cx ? kDigitMaxKCplx : kDigitMaxKReal;
-        DigitScratch digits;
-        if (n > 2 * NB && !digits.alloc(cx, n - 2 * NB, n - 2 * NB, W)) return false;
         // C -= L U on rows r0 .. r1-1, columns c0 .. c1-1 with the columns / rows k0 .. k1-1
         auto update = [&](int k0, int k1, int r0, int r1, int c0, int c1) {
             if (tm.enabled) tm.flops_update += (cx ? 8.0 : 2.0) * (double)(r1 - r0) * (c1 - c0) * (k1 - k0);
@@ -2947,15 +2947,22 @@ static LuMode checked_mode(int n, bool cx) {
 }
 
 // The device-resident forms keep a copy of the matrix for a second run; where
-// there is no memory for it, chains it is.
+// there is no memory for it and what the factorisation takes beside it (the digits,
+// and a few vectors and panels' worth), chains it is.
 template <class T>
 static int factor_inplace_copy(T *d_a, int n, double pivot_tolerance, bool cx, long long *d_piv, int *d_perm,
                                double *d_row, double *d_col, double *scale, Status *hs, LuMode &mode) {
     const size_t bytes = (size_t)n * n * sizeof(T);
     void *copy = nullptr;
-    if (mode != LuMode::chain && cudaMallocAsync(&copy, bytes, stream()) != cudaSuccess) {
-        (void)cudaGetLastError();
-        copy = nullptr;
+    if (mode != LuMode::chain) {
+        copy = dalloc_if_room(bytes);
+        const int k = cx ? kDigitMaxKCplx : kDigitMaxKReal;
+        void *rest = copy ? dalloc_if_room(digit_scratch_bytes(cx, n, n, k) + 4096 * (size_t)n + (16 << 20)) : nullptr;
+        if (!rest) {
+            dfree(copy);
+            copy = nullptr;
+        }
+        dfree(rest);
     }
     if (copy && !cuda_ok(cudaMemcpyAsync(copy, d_a, bytes, cudaMemcpyDeviceToDevice, stream()), "LU copy")) {
         dfree(copy);

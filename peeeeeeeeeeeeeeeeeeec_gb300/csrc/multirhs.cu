@@ -570,7 +570,12 @@ bool inverse_from_lu_real(const double *lu, const int *perm, int n, double *Minv
         else
             PEEC_LAUNCH(k_trsm_diag_d<false>, dgrid, 256, 0, lu, n, r0, nrow, Minv, n);
     };
-    if (n < kDigitsFrom) {
+    // Digit GEMMs: outer blocks of their largest K, inside them each diagonal
+    // block's rows first get what the block's solved rows contribute.
+    const int W = kDigitMaxKReal;
+    DigitScratch digits;
+    DBuf<int> code;
+    if (n < kDigitsFrom || !digits.alloc(false, n, n, W) || !code.alloc_if_room(1)) {
         const int nb = (n + kDB - 1) / kDB;
         for (int blk = 0; blk < nb; ++blk) {
             const int r0 = blk * kDB, nrow = min(kDB, n - r0), r1 = r0 + nrow;
@@ -588,12 +593,6 @@ bool inverse_from_lu_real(const double *lu, const int *perm, int n, double *Minv
         }
         return launch_ok("inverse from the LU factor");
     }
-    // Digit GEMMs: outer blocks of their largest K, inside them each diagonal
-    // block's rows first get what the block's solved rows contribute.
-    const int W = kDigitMaxKReal;
-    DigitScratch digits;
-    DBuf<int> code(1);
-    if (!digits.alloc(false, n, n, W) || !code.p) return false;
     cudaMemsetAsync(code.p, 0, sizeof(int), stream());
     // rows r0 .. r1-1 of Minv -= (rows r0 .., columns k0 .. k1-1 of the factor) rows k0 .. k1-1 of Minv
     auto update = [&](int r0, int r1, int k0, int k1) {

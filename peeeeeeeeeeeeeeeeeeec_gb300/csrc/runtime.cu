@@ -71,6 +71,14 @@ void *dalloc(size_t bytes) {
     return p;
 }
 
+void *dalloc_if_room(size_t bytes) {
+    void *p = nullptr;
+    if (bytes == 0) return nullptr;
+    if (cudaMallocAsync(&p, bytes, stream()) == cudaSuccess) return p;
+    (void)cudaGetLastError();
+    return nullptr;
+}
+
 void dfree(void *p) {
     if (p) cudaFreeAsync(p, stream());
 }

@@ -357,3 +357,49 @@ def test_systems_of_small_second_parts(gpu_lib, eps, digits):
         assert np.all(lu.imag == 0)
     if not digits:
         assert np.array_equal(lu, lu0)
+
+
+@pytest.fixture
+def no_digits(gpu_lib):
+    """No memory for digits: their scratch is refused to this thread."""
+    before = gpu_lib.peec_gb300_set_digit_scratch_limit(0)
+    yield gpu_lib
+    gpu_lib.peec_gb300_set_digit_scratch_limit(before)
+
+
+@pytest.mark.parametrize("cplx", [False, True])
+def test_factorisation_without_memory_for_digits(no_digits, cplx):
+    a = normal(np.random.default_rng(14), cplx, 1400, 1400)
+    want = factor(no_digits, a, FMA)
+    for form in (DIGITS, CHECKED):
+        got = factor(no_digits, a, form)
+        assert got[0] == 0 and got[5] == 0
+        assert all(np.array_equal(x, y) for x, y in zip(got[1:5], want[1:5]))
+
+
+def test_host_factorisation_without_memory_for_digits(no_digits):
+    from helpers import ComplexLU
+    a = normal(np.random.default_rng(15), True, 1310, 1310)
+    f = ComplexLU(no_digits, a)
+    assert f.status == 0
+    lu, piv, rs, cs = f.factors()
+    f.free()
+    _, lu0, piv0, rs0, cs0, _ = factor(no_digits, a, FMA)
+    assert np.array_equal(lu, lu0) and np.array_equal(piv, piv0) and np.array_equal(rs, rs0) and np.array_equal(cs, cs0)
+
+
+@pytest.mark.parametrize("n", [1025])
+def test_inverse_without_memory_for_digits(no_digits, n):
+    test_inverse(no_digits, n)
+
+
+@pytest.mark.parametrize("nx,ny", [(28, 25)])
+def test_transient_system_without_memory_for_digits(no_digits, oracle, nx, ny):
+    test_transient_system_with_digits(no_digits, oracle, nx, ny)
+
+
+def test_no_error_is_left_where_digits_are_refused(no_digits, capfd):
+    capfd.readouterr()
+    a = normal(np.random.default_rng(16), True, 1310, 1310)
+    assert factor(no_digits, a, CHECKED)[0] == 0
+    assert "ERROR" not in capfd.readouterr().err
