@@ -95,9 +95,12 @@ int peec_gb300_set_near_reuse(int on);
  * column of a singular pivot, or -1.  Large systems (complex from 1300, real
  * from 5000 unknowns) are updated on the tensor cores from integer digits; for
  * that the call holds a copy of the matrix and the digits while it runs (without
- * the memory for them, FP64 FMAs do the updates): where two pivot candidates are so close
- * that rounding could decide between them it starts again with FP64 FMAs, so
- * pivots and status do not depend on the form of the updates. */
+ * the memory for them, FP64 FMAs do the updates).  Where two pivot candidates come
+ * closer than 2^-44 + k^1.5 2^-53 of the pivot in column k, it starts again with
+ * FP64 FMAs, whose pivots these then are.  That line is empirical, well above the
+ * differences measured between candidates by digits and by FP64 FMAs (2^-38 at
+ * most in PEEC systems), and no bound: an ill-conditioned matrix may get another
+ * order of nearly equal pivots than FP64 FMAs give it. */
 int peec_gb300_lu_factor_device(double *d_a, size_t n, double pivot_tolerance,
                                 long long *d_piv, int *d_perm, double *matrix_scale,
                                 int *failed_column);

@@ -1267,7 +1267,8 @@ __global__ void __launch_bounds__(kClMaxThreads) k_panel_cl(T *a, int n, int k0,
         if constexpr (!f32)
             if (tie_ulps && lead && u && i != p) {
                 const Key top = exact ? col_key(wr[kk], true) : wu;
-                const Key margin = tie_ulps + __umul64hi((top - 1) << 12, tie_ulps) + kCloseUlps;
+                Key margin = tie_ulps + __umul64hi((top - 1) << 12, tie_ulps) + kCloseUlps;
+                if ((u - 1) >> 52 != (top - 1) >> 52) margin *= 2;  // ulps of the binade below
                 if (u + margin >= top) atomicCAS(&st->code, 0, 7);
             }
         T *pcur = s_prow[par];
@@ -2605,13 +2606,22 @@ static const int kLookAt = 192;  // the column where a checked run looks whether
 static double most_in_fp64(int n) { return std::min(0.4, 5e-5 * n); }
 static const int kLuWideFrom = 3000;  // unknowns from which wide outer blocks pay (2102 complex: 45 ms with, 43 without, before the rows of U were solved in one kernel)
 
-// How close two pivot candidates of column k must be to count as a near tie.
-// Candidates by FP64 chains and by digits differ by at most 2^-48 of the pivot in
-// column 64, 2^-46 in 512, 2^-43 in 1024 and 2^-40 in 2048 (PEEC boxes and plates of
-// 2102 to 3668 unknowns from 1 Hz to 100 MHz; random matrices 2^-39 in 3000), and
-// the closest candidates there are at least 100 times that apart but on meshes
-// whose symmetry makes them tie.
-static double near_tie_fraction(int k) { return 0x1p-45 + (double)k * k * 0x1p-63; }
+// How close two pivot candidates of column k must be to count as a near tie.  An
+// empirical line: the largest differences found between a candidate by FP64 chains
+// and by digits, relative to the pivot, by columns from
+//             64     128    256    512    1024   2048   4096   8192
+//   PEEC      2^-48  2^-47  2^-46  2^-46  2^-43  2^-40  2^-39  2^-38   (boxes and plates of 2102 to
+//             8402 unknowns from 1 Hz to 100 MHz, with and without resistances)
+//   random    2^-47  2^-45  2^-43  2^-41  2^-40  2^-39  2^-38  2^-37   (300 to 12000; normal, decaying,
+//             graded)
+// Two candidates can differ by twice that: the line is 16 times above it for PEEC
+// systems and about 4 times for random ones.  It is no bound: an ill-conditioned
+// leading block raises every later difference (positive random entries: 2^-35 in
+// column 700).  Of 32 box systems (1316 .. 8714 unknowns, 3 to 97 MHz) 30 have no
+// candidates within 2^-31 of each other in late columns, one (a cube) 2^-34.7 in
+// column 3897, one 2^-51 in 508; where symmetry or a low frequency brings candidates closer, as on
+// nearly every plate, the run by digits is given up, mostly in the first 200 columns.
+static double near_tie_fraction(int k) { return 0x1p-44 + k * sqrt((double)k) * 0x1p-53; }
 
 template <class T>
 static bool factor_device(T *d_a, int n, double limit, long long *d_piv, Status *d_st, LuMode &mode) {

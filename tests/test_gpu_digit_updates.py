@@ -403,3 +403,24 @@ def test_no_error_is_left_where_digits_are_refused(no_digits, capfd):
     a = normal(np.random.default_rng(16), True, 1310, 1310)
     assert factor(no_digits, a, CHECKED)[0] == 0
     assert "ERROR" not in capfd.readouterr().err
+
+
+@pytest.mark.parametrize("cplx,pivot", [(False, 1.0), (False, 1.9), (False, 0.75), (True, 1.0)])
+def test_near_ties_in_late_columns(gpu_lib, cplx, pivot):
+    """Two candidates of column 2112 whose rows have met no update (zeros before): a
+    checked run gives the digits up where they are closer than 2^-44 + k^1.5 2^-53
+    of the pivot (k = 2176, the end of the block), and twice the difference of
+    2^-39 found between candidates of the two forms there is well inside."""
+    first, n = 2112, 2180
+    rng = np.random.default_rng(17)
+    t = np.eye(n - first) + 0.1 * rng.uniform(-1, 1, (n - first,) * 2) * (1 - np.eye(n - first))
+    t[1:, 0] *= 0.1
+    a = np.zeros((n, n), dtype=complex if cplx else float)
+    a[:first, :first] = normal(rng, cplx, first, first)
+    line = 2.0 ** -44 + 2176.0 ** 1.5 * 2.0 ** -53
+    for apart, digits in ((2.0 ** -38, 0), (0.8 * line, 0), (4 * line, 1)):
+        t[0, 0], t[1, 0] = pivot, pivot * (1 - apart)
+        a[first:, first:] = t
+        s, _, piv, rs, cs, used = factor(gpu_lib, a, CHECKED)
+        assert s == 0 and piv[first] == first and used == digits
+        assert not cplx or (np.all(rs[first:] == 1) and np.all(cs[first:] == 1))
