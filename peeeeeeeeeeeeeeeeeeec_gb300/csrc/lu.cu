@@ -2618,13 +2618,16 @@ static const int kLuWideFrom = 3000;  // unknowns from which wide outer blocks p
 // systems and about 4 times for random ones.  It is no bound: an ill-conditioned
 // leading block raises every later difference (positive random entries: 2^-35 in
 // column 700).  Of 32 box systems (1316 .. 8714 unknowns, 3 to 97 MHz) 30 have no
-// candidates within 2^-31 of each other in late columns, one (a cube) 2^-34.7 in
-// column 3897, one 2^-51 in 508; where symmetry or a low frequency brings candidates closer, as on
+// candidates closer than 2^-44 + k^2 2^-58, one (a cube) 2^-34.7 in column 3897,
+// one 2^-51 in 508; where symmetry or a low frequency brings candidates closer, as on
 // nearly every plate, the run by digits is given up, mostly in the first 200 columns.
+// A pivot that is no further than that share of the matrix's scale above the limit
+// of a singular one is left to the chains as well: where the two forms round to
+// either side of it, theirs counts.
 static double near_tie_fraction(int k) { return 0x1p-44 + k * sqrt((double)k) * 0x1p-53; }
 
 template <class T>
-static bool factor_device(T *d_a, int n, double limit, long long *d_piv, Status *d_st, LuMode &mode) {
+static bool factor_device(T *d_a, int n, double limit, double scale, long long *d_piv, Status *d_st, LuMode &mode) {
     LuTiming &tm = g_lu_timing;
     if (tm.enabled) tm.reset();
     DBuf<unsigned char> scratch;
@@ -2685,7 +2688,7 @@ static bool factor_device(T *d_a, int n, double limit, long long *d_piv, Status 
             PEEC_LAUNCH((k_rows_of_u<T, 32>), grid, 32 * kRowsWarps, (rows_of_u_smem<T, 32>()), d_a, n, k0, kb, c0, c1,
                         d_st);
     };
-    auto panel = [&](int k0, int kb, double tie) -> bool {
+    auto panel = [&](int k0, int kb, double tie, double limit) -> bool {
         bool done = false;
         if (cl64_enabled() && !launch_cl_panel<T>(d_a, n, k0, kb, limit, d_piv, d_st, tie, done)) return false;
         if (done) return true;
@@ -2722,7 +2725,7 @@ static bool factor_device(T *d_a, int n, double limit, long long *d_piv, Status 
         for (int k0 = 0; k0 < n; k0 += NB) {
             const int kb = std::min(NB, n - k0), r1 = k0 + kb, rest = n - r1;
             tm.mark(2);
-            if (!panel(k0, kb, 0.0)) return false;
+            if (!panel(k0, kb, 0.0, limit)) return false;
             tm.mark(0);
             swaps(k0, kb);
             if (rest > 0) rows_of_u(k0, kb, r1, n);
@@ -2759,13 +2762,14 @@ static bool factor_device(T *d_a, int n, double limit, long long *d_piv, Status 
             for (int b0 = K0; b0 < K1; b0 += 2 * NB) {
                 const int b1 = std::min(K1, b0 + 2 * NB);
                 // the first block's entries have seen chains only: the same in every mode
-                const double tie = mode == LuMode::checked && b0 > 0 ? near_tie_fraction(b1) : 0.0;
+                const double share = b0 > 0 ? near_tie_fraction(b1) : 0.0;
+                const double tie = mode == LuMode::checked ? share : 0.0;
                 tm.mark(2);
                 if (b0 > K0 && !update(K0, b0, b0, n, b0, b1)) return false;
                 for (int k0 = b0; k0 < b1; k0 += NB) {
                     const int kb = std::min(NB, n - k0), r1 = k0 + kb;
                     tm.mark(2);
-                    if (!panel(k0, kb, tie)) return false;
+                    if (!panel(k0, kb, tie, limit + share * scale)) return false;
                     tm.mark(0);
                     swaps(k0, kb);
                     if (r1 < b1) {  // the block's second panel
@@ -2898,7 +2902,7 @@ static int factor_inplace(T *d_a, int n, double pivot_tolerance, bool cx, long l
         memcpy(scale, &bits, sizeof(double));
         if (hs->code != 0 || !isfinite(*scale) || *scale <= 0.0) return 0;
         double limit = pivot_tolerance * *scale;
-        if (!factor_device<T>(d_a, n, limit, d_piv, st.p, mode)) return -1;
+        if (!factor_device<T>(d_a, n, limit, *scale, d_piv, st.p, mode)) return -1;
         size_t perm_smem = (size_t)n * sizeof(int);
         if (perm_smem > 48 * 1024)
             cudaFuncSetAttribute(k_perm, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)perm_smem);

@@ -424,3 +424,21 @@ def test_near_ties_in_late_columns(gpu_lib, cplx, pivot):
         s, _, piv, rs, cs, used = factor(gpu_lib, a, CHECKED)
         assert s == 0 and piv[first] == first and used == digits
         assert not cplx or (np.all(rs[first:] == 1) and np.all(cs[first:] == 1))
+
+
+@pytest.mark.parametrize("cplx", [False, True])
+@pytest.mark.parametrize("form", [DIGITS, CHECKED])
+def test_status_of_systems_that_are_singular_to_rounding(gpu_lib, cplx, form):
+    """The last column a combination of others: the last pivot is rounding, another
+    one by digits than by FP64 FMAs, and for every tolerance around it FP64 FMAs
+    say whether the matrix is refused."""
+    n, refused = 200, 0
+    for seed in range(4):
+        rng = np.random.default_rng(seed)
+        a = normal(rng, cplx, n, n)
+        a[:, -1] = a[:, :-1] @ (rng.integers(-3, 4, n - 1) / 16.0)
+        for tol in 2.0 ** np.arange(-62.0, -46.0, 0.5):
+            want = factor(gpu_lib, a, FMA, tol)[0]
+            refused += want != 0
+            assert factor(gpu_lib, a, form, tol)[0] == want
+    assert 0 < refused < 4 * 32
