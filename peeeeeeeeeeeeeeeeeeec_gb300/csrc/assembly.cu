@@ -375,8 +375,12 @@ enum : int { MARG_THRESHOLD = 1, MARG_TIE = 2, MARG_TRACE_FULL = 4 };
 static const int kTraceCap = 256;       // decisions recorded per job
 static const unsigned char kAccept = 0xFF;
 // A refined node's entry is its bisected edge, plus kClose if another edge is within
-// 1e-6 of its length: at other nodes no copy can find another edge longest.
+// 1e-6 of its length or within kCloseUlps ulps of the largest coordinate: at other
+// nodes no copy can find another edge longest.  (Corners of copies differ by at most
+// 8 such ulps a coordinate, midpoints round by half of one; two edges then
+// differ by less than 4 sqrt(3) 9 ulps from one copy to another.)
 static const unsigned char kClose = 4;
+static const double kCloseUlps = 64.0;
 
 __device__ double warp_adaptive(const double *outer, NearWarpSmem &sm, int order, double abs_tol,
                                 unsigned long long &evals, int &mflags, unsigned char *trace, int &trace_len) {
@@ -504,6 +508,7 @@ struct NearEvalArgs {
     int *marginal;  // [nrec] MARG_* flags of the record's jobs (null: not recorded)
     unsigned char *trace;  // [jobs * kTraceCap] decision traces (null: not recorded)
     int *trace_len;        // [jobs]
+    double cmax;           // largest |coordinate|
 };
 
 // One warp per job (record, triangle pair t = s*2+u, direction d); warps
@@ -661,6 +666,7 @@ struct LevelArgs {
     int *count;            // [kLevels + 1] nodes of every level
     int *overflow;
     unsigned long long *evals;
+    double close_abs;      // edges this close in length: kClose
 };
 
 // One thread per job: zero-area and identical-triangle jobs are finished
@@ -820,7 +826,8 @@ __global__ void __launch_bounds__(kTreeThreads, 3) k_level_tree(LevelArgs A, int
                         const unsigned tied =
                             __ballot_sync(0xffffffffu, lane < 3 && lane != e && len >= longest * (1.0 - 1e-10));
                         if (tied) mflags |= MARG_TIE;
-                        if (__any_sync(0xffffffffu, lane < 3 && lane != e && len >= longest * (1.0 - 1e-6))) close = kClose;
+                        const double close_len = fmin(longest * (1.0 - 1e-6), longest - A.close_abs);
+                        if (__any_sync(0xffffffffu, lane < 3 && lane != e && len >= close_len)) close = kClose;
                         int at = 0;
                         if (lane == 0) at = atomicAdd(&A.count[lv + 1], 2);
                         at = __shfl_sync(0xffffffffu, at, 0);
@@ -951,6 +958,7 @@ static bool near_eval_levels(const NearEvalArgs &E, int nrec) {
     L.count = cnt.p;
     L.overflow = cnt.p + kLevels + 1;
     L.evals = E.evals;
+    L.close_abs = kCloseUlps * 2.220446049250313e-16 * E.cmax;
     for (long long job0 = 0; job0 < total;) {
         const long long nj = std::min(chunk, total - job0);
         L.job0 = job0;
@@ -2330,6 +2338,7 @@ static int run_assembly(DeviceRegions &D, int kind, const AssemblyOptions &o, do
             cudaMemsetAsync(trace_len.p, 0, (size_t)njobrec * 8 * sizeof(int), stream());
         }
         NearEvalArgs A;
+        A.cmax = R.cmax;
         A.corner = R.corner;
         A.rec = rec.p;
         A.job_rec = job_rec;
