@@ -84,6 +84,7 @@ struct RegionsDev {
     float4 *boxf = nullptr;    // [np*2]  box rounded to FP32: (lo, size), (hi, 0) -- the scan's far filter
     int *axis = nullptr;       // [n]     0/1/2 when dir is exactly +-e_axis, else -1 (inductance)
     double cmax = 0.0;         // largest |corner coordinate| (scale of the rounding noise)
+    double extent = 0.0;       // longest side of the bounding box
     double mid[3] = {};        // middle of the bounding box
 };
 
@@ -1608,8 +1609,11 @@ __device__ __forceinline__ bool near_lookup(const TileArgs &T, int i, int j, dou
 // key (class, class, displacement), with the two regions in a fixed order.
 // Entries with a near patch pair keep their own evaluation (their adaptive
 // decisions are compared one by one above), and so does whatever differs by
-// more than kReuseUlps ulps of the largest coordinate: the points of the
-// double-float rule are held to the same 8 ulps (two floats, 2^-49).
+// more than kReuseUlps ulps of the mesh's extent (or of its largest coordinate, if
+// that is smaller): the points of the double-float rule, taken from the mesh's middle,
+// are held to as much (two floats, 2^-49).  Far from the origin coordinates are rounded
+// more coarsely than that, and copies are no longer taken for such: what they
+// differ by, 1e-9 of a cell 1e6 cells away, is no rounding of the integral.
 //
 // Groups are formed by a hash over coordinates in cells of 4096 times that
 // tolerance (a cluster of equal coordinates is rarely split by a cell's edge);
@@ -2063,7 +2067,8 @@ static bool assemble_entries(const TileArgs &T, int nrec, bool reuse) {
         U.mask = slots - 1;
         U.near_bits = near_bits.p;
         U.mass = mass.p;
-        U.tol = kReuseUlps * 2.220446049250313e-16 * (R.cmax > 0.0 ? R.cmax : 1.0);
+        const double size = fmin(R.cmax, R.extent);
+        U.tol = kReuseUlps * 2.220446049250313e-16 * (size > 0.0 ? size : 1.0);
         U.inv_cell = 1.0 / (kReuseCell * U.tol);
         cudaMemsetAsync(U.tab, 0xff, slots * sizeof(EntrySlot), stream());
         cudaMemsetAsync(near_bits.p, 0, words * sizeof(unsigned), stream());
@@ -2199,7 +2204,11 @@ struct DeviceRegions {
             lo[t % 3] = t < 3 ? v : fmin(lo[t % 3], v);
             hi[t % 3] = t < 3 ? v : fmax(hi[t % 3], v);
         }
-        for (int k = 0; k < 3; ++k) view.mid[k] = 0.5 * (lo[k] + hi[k]);
+        view.extent = 0.0;
+        for (int k = 0; k < 3; ++k) {
+            view.mid[k] = 0.5 * (lo[k] + hi[k]);
+            view.extent = fmax(view.extent, hi[k] - lo[k]);
+        }
         if (ok && np) {
             PEEC_LAUNCH(k_patch_prep, (np + 127) / 128, 128, 0, view);
             ok = launch_ok("patch preparation");

@@ -7,6 +7,9 @@ import sys
 import numpy as np
 import pytest
 
+from helpers import inductance, potential
+from peeeeeeeeeeeeeeeeeeec_gb300.mesh import SynthMesh
+
 pytestmark = pytest.mark.gpu
 HERE = os.path.dirname(os.path.abspath(__file__))
 
@@ -52,3 +55,36 @@ def test_copies_whose_longest_edge_differs():
         res[mode] = r.stdout.split()
     assert res["0"] == ["4", "2"]
     assert res["1"] == res["0"]
+
+
+@pytest.mark.parametrize("offset", [0.0, 2.0 ** 10, 2.0 ** 20])
+def test_shared_entries_far_from_the_origin(gpu_lib, offset):
+    """A plate of 12 x 11 cells whose node coordinates are off by up to two ulps of
+    the largest one: entries of regions at least five cells apart with and without reuse.
+    Points are held as float pairs of distances from the mesh's middle, 2^-49 of its
+    half extent, four of them in a difference of two points and of two results; the
+    corrected sharing of copies within 8 ulps of the extent adds 16 2^-52 of it."""
+    nx, ny, h = 12, 11, 0.05
+    rng = np.random.default_rng(21)
+    i, j = np.meshgrid(np.arange(nx + 1), np.arange(ny + 1))
+    xyz = np.zeros((i.size, 3))
+    xyz[:, 0], xyz[:, 1] = offset + h * i.ravel(), offset + h * j.ravel()
+    xyz[:, :2] += rng.integers(-2, 3, (i.size, 2)) * np.spacing(np.abs(xyz).max())
+    a, b = np.meshgrid(np.arange(nx), np.arange(ny))
+    p = (b * (nx + 1) + a).ravel()
+    got = {}
+    with SynthMesh.from_arrays(xyz, np.stack([p, p + 1, p + nx + 2, p + nx + 1], 1)) as m:
+        ends = xyz[m.edges()].mean(axis=1)
+        before = gpu_lib.peec_gb300_set_near_reuse(0)
+        try:
+            for on in (0, 1):
+                gpu_lib.peec_gb300_set_near_reuse(on)
+                got[on] = [f(gpu_lib, m) for f in (inductance, potential)]
+        finally:
+            gpu_lib.peec_gb300_set_near_reuse(before)
+    for (s0, own), (s1, shared), at in zip(got[0], got[1], (ends, xyz)):
+        assert s0 == 0 and s1 == 0
+        apart = np.linalg.norm(at[:, None] - at[None], axis=-1)
+        far = (apart > 5.5 * h) & (own != 0)
+        bound = (8 * 2.0 ** -49 * 0.5 * nx * h + 16 * 2.0 ** -52 * nx * h) / (4 * h) + 64 * 2.0 ** -48
+        assert np.max(abs(shared - own)[far] / abs(own)[far]) < bound
