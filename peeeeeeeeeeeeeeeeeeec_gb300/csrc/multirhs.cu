@@ -273,7 +273,10 @@ static void cgemm_sub(const c32 *A, int lda, const c32 *Bm, c32 *C, int ldb, int
 // (One warp a right-hand side with the rows in its lanes spent two FMAs of 32 lanes
 // on every row, and the quotient in all of them: 3552 right-hand sides, upper 133
 // us, lower 30; now 31 and 25.)  A quotient is y r, r the row's reciprocal,
-// corrected by its remainder.
+// corrected by its remainder, where nothing under- or overflows.
+__device__ __forceinline__ bool in_mid_range(double v) {  // 2^-500 <= |v| < 2^500
+    return ((unsigned)(__double_as_longlong(v) >> 52 & 0x7ff) - 523u) < 1000u;
+}
 template <bool LOWER>
 __global__ void __launch_bounds__(256) k_trsm_diag_d(const double *lu, int n, int r0, int nrow, double *Y,
                                                      int nrhs) {
@@ -305,8 +308,11 @@ __global__ void __launch_bounds__(256) k_trsm_diag_d(const double *lu, int n, in
             double *x = xs[m & 1];
             if (warp == w) {
                 if (!LOWER) {
-                    const double y = v[rm], c = rcp[m], z = y * c;
-                    v[rm] = fma(fma(-z, B[m][m], y), c, z);
+                    const double y = v[rm], b = B[m][m], c = rcp[m], z = y * c;
+                    if (in_mid_range(b) && (in_mid_range(y) || (__double_as_longlong(y) << 1) == 0))
+                        v[rm] = fma(fma(-z, b, y), c, z);
+                    else
+                        v[rm] = y / b;
                 }
                 x[lane] = v[rm];
             }

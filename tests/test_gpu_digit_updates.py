@@ -442,3 +442,15 @@ def test_status_of_systems_that_are_singular_to_rounding(gpu_lib, cplx, form):
             refused += want != 0
             assert factor(gpu_lib, a, form, tol)[0] == want
     assert 0 < refused < 4 * 32
+
+
+def test_inverse_outside_the_middle_of_the_range(gpu_lib):
+    """Quotients whose divisor's reciprocal overflows, or whose dividend is infinite,
+    are those of a division."""
+    for u, want in ((np.array([[1e-310, 1e-10], [0.0, 1.0]]), [[np.inf, -1e-10 / 1e-310], [0.0, 1.0]]),
+                    (np.array([[2.0, np.inf], [0.0, 1.0]]), [[np.nan, -np.inf], [0.0, 1.0]]),  # 1 - inf 0
+                    (np.array([[1e300, 1e-20], [0.0, 1e-5]]), [[1e-300, -1e-20 * 1e5 / 1e300], [0.0, 1e5]])):
+        with Device(gpu_lib) as d:
+            p = [d.put(u), d.put(np.arange(2, dtype=np.int32)), d.put(np.zeros((2, 2)))]
+            assert gpu_lib.peec_gb300_inverse_device(p[0], p[1], 2, p[2]) == 0
+            assert np.allclose(d.get(p[2], u), want, rtol=4 * U, atol=5e-324, equal_nan=True)
