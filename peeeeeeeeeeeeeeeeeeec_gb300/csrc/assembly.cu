@@ -2206,7 +2206,8 @@ struct DeviceRegions {
         }
         view.extent = 0.0;
         for (int k = 0; k < 3; ++k) {
-            view.mid[k] = 0.5 * (lo[k] + hi[k]);
+            view.mid[k] = 0.5 * lo[k] + 0.5 * hi[k];
+            if (!isfinite(view.mid[k])) view.mid[k] = 0.0;  // (an infinite corner spoils its own patch only)
             view.extent = fmax(view.extent, hi[k] - lo[k]);
         }
         if (ok && np) {

@@ -88,3 +88,22 @@ def test_shared_entries_far_from_the_origin(gpu_lib, offset):
         far = (apart > 5.5 * h) & (own != 0)
         bound = (8 * 2.0 ** -49 * 0.5 * nx * h + 16 * 2.0 ** -52 * nx * h) / (4 * h) + 64 * 2.0 ** -48
         assert np.max(abs(shared - own)[far] / abs(own)[far]) < bound
+
+
+@pytest.mark.parametrize("value", [np.inf, -np.inf, np.nan])
+def test_a_non_finite_corner_names_its_own_entry(gpu_lib, capfd, value):
+    """Points are taken from the mesh's middle: an infinite corner must not spoil the
+    other patches' points.  The entry that is named is the one of the FP64 rule."""
+    named = []
+    before = gpu_lib.peec_gb300_set_far_precision(1)
+    try:
+        for mode in (0, 1):
+            gpu_lib.peec_gb300_set_far_precision(mode)
+            with SynthMesh.plate(2.0, 1.0, 8, 4) as m:
+                m.dual.node_patches[30].patches[0].points[0] = value
+                capfd.readouterr()
+                assert potential(gpu_lib, m)[0] != 0
+                named.append([x for x in capfd.readouterr().err.splitlines() if "failed" in x])
+    finally:
+        gpu_lib.peec_gb300_set_far_precision(before)
+    assert named[0] and named[0] == named[1]
