@@ -2588,11 +2588,13 @@ enum class LuMode {
               // most entries are left to FP64 FMAs
 };
 // Unknowns from which digit GEMMs are used (LU of random matrices on GB300,
-// chains / digits in ms: complex 1000: 17.6 / 16.7, 1200: 22.2 / 20.2, 1400: 27.7 /
-// 23.6, 2102: 52.6 / 36.0, 4000: 199 / 86, 8402: 1436 / 248; real 1500: 14.2 / 12.9,
-// 2102: 22.4 / 19.4, 4000: 66.0 / 44.3, 8402: 386 / 111).  A checked run may have to
-// be done again by chains, so the lines lie somewhat above the crossings (and
-// well above for real systems: those of regular meshes nearly always tie).
+// chains / digits in ms: complex 800: 6.9 / 6.6, 1300: 14.7 / 11.7, 2102: 36.9 / 21.2,
+// 4000: 174.7 / 58.3, 8402: 1384 / 252; real 1000: 4.7 / 4.7, 2000: 12.8 / 10.1, 4000:
+// 52.7 / 26.8, 8402: 366 / 102).  A checked run that is given up costs the columns up to there
+// (plates of 1541 / 4256 / 7701 unknowns: 20.9 / 209 / 1080 ms, chains alone 19.3 / 203 / 1065), so
+// its lines lie above the crossings, and well above for real systems: MNA matrices of
+// regular meshes tie exactly, and the run by digits buys them nothing (box of 8402: 369 ms,
+// chains 366).
 static const int kDigitsFromCplx = 1300;
 static const int kDigitsFromReal = 2000;
 static const int kCheckedFromReal = 5000;
@@ -2604,7 +2606,12 @@ static const int kLookAt = 192;  // the column where a checked run looks whether
 // of the entries (parts that small) and 343 / 517 / 1040 / 1393 ms, FP64 alone 1366;
 // 2102 unknowns: 0.1 / 1 / 16 / 60 % and 22 / 29 / 43 / 51 ms, FP64 alone 35.
 static double most_in_fp64(int n) { return std::min(0.4, 5e-5 * n); }
-static const int kLuWideFrom = 3000;  // unknowns from which wide outer blocks pay (2102 complex: 45 ms with, 43 without, before the rows of U were solved in one kernel)
+// Unknowns from which wide outer blocks pay, where the trailing digit GEMM's
+// epilogue weighs more than the second form of its inner ones (64 columns / wide,
+// ms: complex 5000 90.8 / 92.4, 6000 128.9 / 127.5, 8402 266.6 / 251.1; real 5500
+// 47.2 / 48.9, 6500 65.7 / 64.5, 8402 114.0 / 101.9).
+static const int kLuWideFromCplx = 5500;
+static const int kLuWideFromReal = 6200;
 
 // How close two pivot candidates of column k must be to count as a near tie.  An
 // empirical line: the largest differences found between a candidate by FP64 chains
@@ -2668,7 +2675,7 @@ static bool factor_device(T *d_a, int n, double limit, double scale, long long *
     // costs an integer epilogue per entry whatever K is (m = n = 4000
     // complex: 764 us with K = 64, 1730 us with 192), so W is its largest K;
     // small systems, where launches count, take one inner block.
-    const int W = n < kLuWideFrom ? 2 * NB : cx ? kDigitMaxKCplx : kDigitMaxKReal;
+    const int W = n < (cx ? kLuWideFromCplx : kLuWideFromReal) ? 2 * NB : cx ? kDigitMaxKCplx : kDigitMaxKReal;
     DigitScratch digits;
     if (mode != LuMode::chain && n > 2 * NB && !digits.alloc(cx, n - 2 * NB, n - 2 * NB, W)) mode = LuMode::chain;
     auto swaps = [&](int k0, int kb) {

@@ -246,13 +246,23 @@ def test_lu_by_digits_at_block_edges(gpu_lib, n, cplx, form):
         assert np.array_equal(piv, factor(gpu_lib, a, FMA)[2])
 
 
-def test_real_lu_by_digits_in_wide_blocks(gpu_lib):
-    """From 3000 unknowns on outer blocks of 256 columns: the real update at its largest K."""
-    n = 3137
-    a = normal(np.random.default_rng(1), False, n, n)
+@pytest.mark.parametrize("cplx,n", [(False, 6273), (True, 5601)])
+def test_lu_by_digits_in_wide_blocks(gpu_lib, cplx, n):
+    """Outer blocks of 256 real (from 6200 unknowns) and 192 complex columns (from 5500),
+    the last one ragged: P A x = L U x for signs x, each side within gamma_n |L| |U| |x|
+    of the exact one, twice that for L U x and once for the factor."""
+    a = normal(np.random.default_rng(1), cplx, n, n)
     s, lu, piv, rs, cs, used = factor(gpu_lib, a, CHECKED)
     assert s == 0 and used == 1
-    assert residual(a, lu, piv, rs, cs) <= n * U / (1 - n * U)
+    a = (a / rs[:, None]) / cs[None]
+    order = np.arange(n)
+    for k, p in enumerate(piv):
+        order[[k, p]] = order[[p, k]]
+    l, u = np.tril(lu, -1), np.triu(lu)
+    x = np.random.default_rng(2).choice([-1.0, 1.0], (n, 4))
+    y, z = u @ x, np.abs(u) @ np.abs(x)
+    gamma = (2 * np.sqrt(2) if cplx else 1.0) * n * U / (1 - n * U)
+    assert np.all(abs(l @ y + y - (a @ x)[order]) <= 4 * gamma * (np.abs(l) @ z + z))
 
 
 def test_complex_sizes_that_take_digits_by_themselves(gpu_lib):
