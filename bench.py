@@ -1005,6 +1005,36 @@ def run_reference(args, rank, world):
     print(json.dumps(line))
 
 
+LINE_BYTES = 12000  # of the printed line: who keeps the end of a long output gets a cut line, which does not parse
+
+
+def printed(record):
+    """The record as it is printed: floats to six digits; from the legs and rooflines,
+    lists of per-request figures and long descriptions are left to --details."""
+    def short(x, leg):
+        if isinstance(x, float):
+            return float("%.6g" % x)
+        if isinstance(x, str):
+            return x if not leg or len(x) <= 60 else x[:57] + "..."
+        if isinstance(x, dict):
+            return {k: short(v, leg) for k, v in x.items() if not (leg and isinstance(v, list) and len(v) > 4)}
+        if isinstance(x, list):
+            return [short(v, leg) for v in x]
+        return x
+
+    legs = {"serving", "batched", "transient", "retarded", "rcs", "incidence", "far_precision", "mixed", "cpu_baseline",
+            "roofline"}
+    out = {k: short(v, k in legs) for k, v in record.items()}
+    out["rooflines"] = [{k: short(r[k], True) for k in ("kernel", "bound", "achieved", "peak", "unit", "frac", "ms")}
+                        for r in record.get("rooflines") or []]
+    # should it still be too long, the legs give way to the contract's keys
+    for k in ("far_precision", "incidence", "batched", "serving", "retarded", "rooflines", "rcs", "transient", "mixed"):
+        if len(json.dumps(out)) <= LINE_BYTES:
+            break
+        out[k] = "see --details"
+    return out
+
+
 def main():
     ap = argparse.ArgumentParser()
     ap.add_argument("--gpus", type=int, default=1)
@@ -1016,6 +1046,7 @@ def main():
     ap.add_argument("--no-mixed", action="store_true")
     ap.add_argument("--box", default=None, help="lx,ly,lz,nx,ny,nz (default: the 5 cm box)")
     ap.add_argument("--transient-steps", type=int, default=4096)
+    ap.add_argument("--details", metavar="FILE", help="write the whole record there (the printed line is cut to %d bytes)" % LINE_BYTES)
     ap.add_argument("--no-retarded", action="store_true")
     ap.add_argument("--serve-window", type=float, default=0.2, help="seconds of Poisson arrivals (0: skip)")
     ap.add_argument("--serve-workers", type=int, default=8)
@@ -1274,7 +1305,10 @@ def main():
                 "pipe_peaks_tflops": {"fp64": p64.value, "fp32": p32.value,
                                       "how": "FMA loops on this GPU (the pool's measured peaks cover HBM and BF16)"},
                 "rooflines": roofs, "roofline": max(roofs, key=lambda r: r["ms"]) if roofs else None}
-        print(json.dumps(line))
+        if args.details:
+            with open(args.details, "w") as f:
+                json.dump(line, f)
+        print(json.dumps(printed(line)))
     if dist:
         dist.barrier()
         dist.destroy_process_group()
