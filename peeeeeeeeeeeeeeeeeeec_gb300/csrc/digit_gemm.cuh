@@ -31,8 +31,7 @@ struct DigitScratch {
     DigitScratch &operator=(const DigitScratch &) = delete;
 };
 size_t digit_scratch_bytes(bool cplx, size_t m, size_t n, size_t k);
-// Bytes that a DigitScratch of the calling thread may take (no limit at first): the
-// server keeps jobs within their share of its budget.
+// Bytes that a DigitScratch of the calling thread may take (no limit at first).
 size_t &digit_scratch_limit();
 
 // C (m x n, row-major, leading dimension ldc) -= A (m x k, lda) B (k x n,

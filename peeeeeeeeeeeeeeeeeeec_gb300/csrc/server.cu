@@ -60,13 +60,6 @@ struct MeshEntry {
 
 static const size_t kSpareBytes = 64 << 20;  // of a job's estimate: scratch
 
-// The calling thread's digit scratch limit while it lives.
-struct DigitLimit {
-    size_t before = digit_scratch_limit();
-    explicit DigitLimit(size_t bytes) { digit_scratch_limit() = bytes; }
-    ~DigitLimit() { digit_scratch_limit() = before; }
-};
-
 struct Job {
     long long ticket = 0;
     int kind = 0;  // 0 harmonic, 1 transient lightning
@@ -80,7 +73,6 @@ struct Job {
     size_t bytes = 0;       // per-request device estimate (caches excluded)
     size_t mesh_bytes = 0;  // Lp / P / geometry of the mesh
     size_t sys_bytes = 0;   // transient system of (scheme, dt)
-    size_t digit_limit = kSpareBytes;  // what the FP64 factorisation's digits may take
     PeecRequestResult res{};
     bool done = false;
 };
@@ -137,13 +129,11 @@ class Server {
         // also keeps Z as float pairs for its residual
         j->bytes = 32 * n * n + (r->mixed ? 9216 * n : 0) + (r->mixed && r->nrhs >= 32 ? 16 * n * n : 0) +
                    112 * n * r->nrhs + kSpareBytes;
-        // the FP64 factorisation's digits, beyond those 64 MiB (where the budget
-        // does not hold them, it does without)
+        // the FP64 factorisation's digits, beyond those 64 MiB.  A budget that does
+        // not hold them changes no result: they are taken all the same, and only where
+        // the device has no memory for them FP64 FMAs do the updates.
         const size_t digits = digit_scratch_bytes(true, n, n, kDigitMaxKCplx);
-        if (digits > kSpareBytes && j->bytes + j->mesh_bytes + digits <= budget_) {
-            j->bytes += digits;
-            j->digit_limit = digits;
-        }
+        if (digits > kSpareBytes && j->bytes + j->mesh_bytes + digits <= budget_) j->bytes += digits;
         return enqueue(j);
     }
 
@@ -169,10 +159,7 @@ class Server {
         j->sys_bytes = transient_system_bytes(ne, nv);
         j->bytes = 8 * r->n_steps * np + 64 * nt + 4 * np + kSpareBytes;
         const size_t digits = digit_scratch_bytes(false, nt, nt, kDigitMaxKReal);
-        if (digits > kSpareBytes && j->bytes + j->mesh_bytes + j->sys_bytes + digits <= budget_) {
-            j->sys_bytes += digits;
-            j->digit_limit = digits;
-        }
+        if (digits > kSpareBytes && j->bytes + j->mesh_bytes + j->sys_bytes + digits <= budget_) j->sys_bytes += digits;
         return enqueue(j);
     }
 
@@ -332,7 +319,6 @@ class Server {
             if (status == 0 && j->kind == 1) {
                 if (build_sys) {
                     void *sys = nullptr;
-                    const DigitLimit limit(j->digit_limit);
                     int s = peec_gb300_transient_create(me->L, me->P, me->edges, nullptr, me->ne, me->nv,
                                                         j->treq.scheme, j->treq.dt, &sys);
                     std::lock_guard<std::mutex> g(mu_);
@@ -420,7 +406,6 @@ class Server {
             DBuf<double> rs(n), cs(n);
             if (!W.alloc(n * n) || !piv.p || !perm.p || !rs.p || !cs.p) return -1;
             if (peec_gb300_copy_device(W.p, Z.p, n * n * sizeof(Complex)) != 0) return -1;
-            const DigitLimit limit(j.digit_limit);
             status = complex_lu_factor_again(W.p, (int)n, 1e-14, piv.p, perm.p, rs.p, cs.p, [&] {
                 return peec_gb300_copy_device(W.p, Z.p, n * n * sizeof(Complex)) == 0;
             });
