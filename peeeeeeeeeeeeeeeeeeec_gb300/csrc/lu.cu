@@ -117,7 +117,7 @@ __device__ __forceinline__ cplx addv(cplx a, cplx b) { return cplx{a.re + b.re, 
 __device__ __forceinline__ cplxf addv(cplxf a, cplxf b) { return cplxf{a.re + b.re, a.im + b.im}; }
 
 struct Status {
-    int code;    // 0 ok, 2 singular / invalid pivot, 7 near tie of two pivot candidates, or mostly FP64 work (checked runs)
+    int code;    // 0 ok, 2 singular / invalid pivot, 7 near tie of two pivot candidates (checked runs), or mostly FP64 work
     int column;  // failing column
     double value;
 };
@@ -2583,9 +2583,8 @@ static thread_local LuTiming g_lu_timing;  // per host thread, like the stream
 // How a factorisation does its trailing updates.
 enum class LuMode {
     chain,    // chains of FP64 FMAs in pivot order: the reference's arithmetic up to FMA rounding
-    digits,   // digit GEMMs
-    checked,  // digit GEMMs, stopping with status 7 at a near tie of two pivot candidates or where
-              // most entries are left to FP64 FMAs
+    digits,   // digit GEMMs, stopping with status 7 where most entries are left to FP64 FMAs
+    checked,  // the same, stopping at a near tie of two pivot candidates as well
 };
 // Unknowns from which digit GEMMs are used (LU of random matrices on GB300,
 // chains / digits in ms: complex 800: 6.9 / 6.6, 1300: 14.7 / 11.7, 2102: 36.9 / 21.2,
@@ -2748,13 +2747,13 @@ static bool factor_device(T *d_a, int n, double limit, double scale, long long *
         // C -= L U on rows r0 .. r1-1, columns c0 .. c1-1 with the columns / rows k0 .. k1-1
         auto update = [&](int k0, int k1, int r0, int r1, int c0, int c1) {
             if (tm.enabled) tm.flops_update += (cx ? 8.0 : 2.0) * (double)(r1 - r0) * (c1 - c0) * (k1 - k0);
-            const bool first = mode == LuMode::checked && k0 < kLookAt && r0 == k1 && c1 == n;
+            const bool first = k0 < kLookAt && r0 == k1 && c1 == n;
             const double entries = (double)(r1 - r0) * (c1 - c0);
             return digit_gemm_sub(cx, d_a + (size_t)r0 * n + k0, n, d_a + (size_t)k0 * n + c0, n,
                                   d_a + (size_t)r0 * n + c0, n, r1 - r0, c1 - c0, k1 - k0, digits, &d_st->code,
                                   first ? (size_t)(most_in_fp64(n) * entries) : ~(size_t)0);
         };
-        bool looked = mode != LuMode::checked;
+        bool looked = mode != LuMode::checked && !cx;
         for (int K0 = 0; K0 < n; K0 += W) {
             const int K1 = std::min(n, K0 + W);
             if (!looked && K0 >= kLookAt) {
@@ -2880,9 +2879,8 @@ namespace peec {
 // before any factorisation.
 //
 // again(): puts the original matrix back into d_a; with it, large systems are
-// factored by digit GEMMs in a checked run, and by chains of FP64 FMAs from the
-// start again if that met a near tie of two pivot candidates or a singular
-// pivot: pivots and status are those of the chains in every case.  mode: the one
+// factored by digit GEMMs, and by chains of FP64 FMAs from the start again if that
+// stopped (LuMode) or met a singular pivot.  mode: the one
 // that the factor comes from on return.
 template <class T, class Again>
 static int factor_inplace(T *d_a, int n, double pivot_tolerance, bool cx, long long *d_piv, int *d_perm,
@@ -2936,8 +2934,11 @@ static void report_status(const Status &hs, bool cx) {
                 hs.column, hs.column, hs.value);
 }
 
-// For callers inside the library that can make the matrix again.  Real: the
-// pivots stay inside (the transient system), so near ties need no second run.
+// For callers inside the library that can make the matrix again.  Their pivots stay
+// inside (transient systems, the server's and the sweep's FP64 solves), so near ties
+// need no second run: either candidate is as good a pivot.  (A plate of 12109 unknowns
+// has one in a late column at some frequencies: served at 51 and 73 MHz beside other
+// requests, 12 and 17 s instead of 2.)
 int lu_factor_again(double *d_a, int n, double pivot_tolerance, long long *d_piv, int *d_perm, double *scale,
                     int *failed_column, const std::function<bool()> &again) {
     Status hs;
@@ -2954,7 +2955,7 @@ int complex_lu_factor_again(Complex *d_a, int n, double pivot_tolerance, long lo
                             double *d_col, const std::function<bool()> &again) {
     Status hs;
     double scale = 0.0;
-    LuMode mode = n >= kDigitsFromCplx ? LuMode::checked : LuMode::chain;
+    LuMode mode = n >= kDigitsFromCplx ? LuMode::digits : LuMode::chain;
     if (factor_inplace<cplx>((cplx *)d_a, n, pivot_tolerance, true, d_piv, d_perm, d_row, d_col, &scale, &hs, mode,
                              again) != 0)
         return -1;
