@@ -1377,6 +1377,11 @@ __device__ __forceinline__ float rsqrt_hw(float x) {
 //    is exact), one Halley step y + r y / 2 + 3 r^2 y / 8, third order from 2^-22
 //    (with y r (1/2 + 3 r / 8) the rounding next to 1/2 left a mean of 2e-16).
 //  - The sum's low part is left as it grows (<= 2^-24 of the sum a term).
+// The two corrections in te are added the larger one first.  The order changes entries in
+// their last bits only, yet decides whether systems at the rounding floor of FP64 pass a
+// gate there (plates at 1 kHz, refined to 1e-10: about half of those with sides 1 mm
+// apart miss it, with any form of this rule or the one before); it was kept where
+// the tests' plate passes.
 __device__ __forceinline__ void df_add_inverse(const float4 ah, const float4 al, const float4 bh, const float4 bl,
                                                float &hi, float &lo) {
     const f2 ux = two_sum(ah.x, -bh.x), uy = two_sum(ah.y, -bh.y), uz = two_sum(ah.z, -bh.z);

@@ -10,21 +10,24 @@
 // of at most 1 and cut into kDigits balanced digits of seven bits, x = sum_i d_i
 // 2^(1 - 7 i), |d_i| <= 64 -- integers that BF16 holds exactly.  The product of
 // digits i and j has weight 2^(2 - 7 (i + j)): the pairs with the same sum i + j
-// up to kDigits + 1 are added up in one TMEM accumulator each.  Such a sum of at
-// most ten pairs is an integer below 2^24 (10 x 2 K x 2^12 at K = 192 complex, 10 x
-// K x 2^12 at K = 256 real), so FP32 accumulation is exact (the last two sums could
-// round by a unit of 2^-82 at worst).
+// up to kDigits + 1 are added up in one TMEM accumulator each.  A sum of up to ten
+// pairs is an integer below 2^24 (10 x 2 K x 2^12 at K = 192 complex, 10 x K x 2^12 at K
+// = 256 real), so FP32 accumulation is exact; the last two complex sums, of eleven and
+// twelve pairs, could pass 2^24 and then round by a unit, 2^-82 and 2^-89.
 //
 // The sums are combined in 90-bit integers of unit 2^-89 and leave them once,
 // rounded to FP64, for the subtraction from C: the only FP64 operation of an
-// update.  Its error is about 2^-78 |row of A| |column of B| (what is dropped).
+// update.  Its error is what is dropped, the pairs i + j >= 14: about 2^-78 |row of A|
+// |column of B| for digits that look random, 2^-72 at worst (11 x 2 K x 2^12 x 2^-96, all
+// of one sign).
 // A chain of K FP64 FMAs rounds at 2^-53 of its running sum, so entries whose C
 // and update are both below 2^-kExactBelow |row| |column| are left out and done
 // in FP64 (matrices of weakly coupled parts, systems at kHz).  Complex entries are
 // looked at by their real and imaginary parts, as a chain rounds each for itself
 // (small resistances beside j omega L); parts that are exactly zero, because no
 // product has both factors (lossless systems), are told by bit masks of the
-// operands' nonzero parts and cost nothing.  (Eleven digits, 66 pairs, with the line
+// operands' nonzero parts and cost nothing.  Down to that line an entry or part is then
+// no less accurate than on the FP64 pipe, for digits that look random.  (Eleven digits, 66 pairs, with the line
 // at 2^-18: 5% faster on random matrices, but 341 against 294 ms for the solve of
 // the 8402-unknown box, where more entries take the FP64 way.)
 //
@@ -460,7 +463,7 @@ __device__ __forceinline__ void tmem_ld8(uint32_t taddr, float *v) {
         : "r"(taddr)
         : "memory");
 }
-// 8 words of this warp's 32 TMEM lanes out and 4 back
+// 8 words of this warp's 32 TMEM lanes out; 4 back below
 __device__ __forceinline__ void tmem_st8(uint32_t taddr, const int *v) {
     asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"r"(taddr), "r"(v[0]),
                  "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7])
@@ -727,13 +730,13 @@ __device__ __forceinline__ bool issue_pass(uint32_t base_addr, uint32_t tmem, in
     return true;
 }
 
-// Fourteen warps: warp 0 lane 0 brings the digits, warp 1 lane 0 issues the
-// MMAs, warps 2..13 take the sums from TMEM (32 rows and a third of the columns
-// each: 32 sums a thread in registers; with eight warps of 64 sums the
-// registers spilled and a sum took 64 cycles) and update C, which comes into
-// shared memory ahead of time (asynchronous copies of 64-byte row pieces, two
+// Fourteen warps: lane 0 of warp 0 brings the digits, warp 1 issues the MMAs (the
+// whole warp, an elected lane each), warps 2..13 take the sums from TMEM (32 rows and
+// a third of the columns each: 32 sums a thread in registers; with eight warps of 64
+// sums the registers spilled and a sum took 64 cycles) and update C, which comes
+// into shared memory ahead of time (asynchronous copies of 64-byte row pieces, two
 // in flight).
-// A tile's digit pairs run in passes over K, three accumulators at a time; each
+// A tile's digit pairs run in three passes over K, four accumulators (sums) each; each
 // accumulator goes back as soon as its warps have read it, so the MMAs of one
 // pass overlap the reads of the one before, and the update of C overlaps the
 // next tile.
