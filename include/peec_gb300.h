@@ -110,8 +110,10 @@ int peec_gb300_complex_lu_factor_device(Complex *d_a, size_t n, double pivot_tol
                                         double *matrix_scale, int *failed_column);
 /* The same with the form of the updates given: 0 FP64 FMAs in pivot order, 1
  * integer digits, 2 integer digits with the check for near ties (and FP64 FMAs
- * from the start where it stops).  1 and 2 take FP64 FMAs after a singular pivot
- * and without the memory for a copy of the matrix; *used (may be NULL): 0 if the
+ * from the start where it stops).  1 and 2 take FP64 FMAs after a pivot at or near
+ * the limit of a singular one, where most entries of a complex matrix are too small
+ * beside their rows and columns for the digits, and without the memory for the digits
+ * and a copy of the matrix; *used (may be NULL): 0 if the
  * factor comes from FP64 FMAs, 1 from digits.  Row and column scales: complex only. */
 int peec_gb300_lu_factor_device_form(int cplx, void *d_a, size_t n, double pivot_tolerance,
                                      long long *d_piv, int *d_perm, double *d_row_scale,
