@@ -25,7 +25,8 @@ Legs beside the headline: the mixed-precision solve, serving (config 5:
 Poisson harmonic and lightning requests), the config-4 sweep on 12 of its
 48 meshes (--batch), transient, retarded, RCS, incidence and far-rule
 precision;
---config3 and --config4 run those configurations alone.
+--config3 and --config4 run those configurations alone.  The printed line is
+kept short; --details FILE writes the whole record.
 Multi-GPU: the path does not shard; --gpus N runs N independent replicas
 (one process per GPU) and reports the aggregate.
 """

@@ -85,7 +85,8 @@ int peec_gb300_set_far_precision(int mode);
 /* Reuse of translated copies (default on): near patch pairs whose
  * corners are translated copies of each other (to a few ulps of the largest
  * coordinate) share one adaptive evaluation, and so do matrix entries without
- * near pairs one double-float far sum.  Returns the previous setting. */
+ * near pairs one double-float far sum (copies to a few ulps of the mesh's extent).
+ * Returns the previous setting. */
 int peec_gb300_set_near_reuse(int on);
 
 /* ---- dense factorisations of device-resident matrices (in place) ----
